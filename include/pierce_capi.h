@@ -161,7 +161,10 @@ typedef struct pierce_tuning {
 enum pierce_edge_source {
     PIERCE_EDGES_AUTO = 0,       /* per side: the kept triangles' edges where the join builds grouped
                                     per-join hierarchies and the side keeps fewer than half of its
-                                    triangles, else the dataset's edges (triangles when it has none) */
+                                    triangles, else the dataset's edges (triangles when it has none; a
+                                    dataset the library expanded itself may take either: they are the
+                                    same segments).  Where both sides take their triangles' edges, an
+                                    exact two-way join into a pair table tests the triangles pairwise */
     PIERCE_EDGES_DATASET = 1,    /* the dataset's edge list (the `.pre` edges) */
     PIERCE_EDGES_TRIANGLES = 2   /* the edges of the triangles kept for the join's per-join hierarchies, each
                                     segment of a leaf group once (needs active_bvh) */
@@ -212,10 +215,12 @@ typedef struct pierce_join_opts {
 
 typedef struct pierce_stats {
     double ms_total;              /* GPU time of the whole join (CUDA events) */
-    double ms_edge_rays[2];       /* A->B, B->A edge-ray kernels (all passes) */
+    double ms_edge_rays[2];       /* A->B, B->A edge-ray kernels (all passes); a join by triangle pairs
+                                     tests both directions at once: [0] alone */
     double ms_parity[2];          /* A->B, B->A parity kernels */
     double ms_dedup;              /* scan, sort/unique or compaction */
-    uint64_t rays;                /* edge rays traced (per pass) */
+    uint64_t rays;                /* edge rays traced (per pass); a join by triangle pairs: the segments of
+                                     the groups it tests, each group's once (the rays of its triangles) */
     uint64_t node_visits;         /* BVH nodes fetched */
     uint64_t tri_tests;           /* ray-triangle tests */
     uint64_t raw_hits;            /* pair emissions before deduplication */

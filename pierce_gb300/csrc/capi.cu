@@ -108,6 +108,8 @@ enum : int {
     SLOT_NODES4_OBJ_A = 32,  // ... of the object hierarchies (culling)
     SLOT_NODES4_OBJ_B = 33,
     SLOT_CONT_PARITY = 35,    // containment: parity table of B's first vertices in A
+    SLOT_LISTED_A = 36,       // joins by triangle pairs: A's listed groups
+    SLOT_SPILL = 37,          // ... their work words and entries left for the next round
     SLOT_ENTRY_AB = 38,       // rays from triangles: entry nodes of the listed groups, A->B
     SLOT_ENTRY_BA = 39,
 };
@@ -980,6 +982,32 @@ struct Join {
         const int64_t kept = (d ? vb : va).num_tris;
         return 2 * kept < (int64_t)ds->nt;
     }
+    // Joins by triangle pairs (pairs.cu) take the place of the edge rays of
+    // both directions where the pair set is that of both sides' kept
+    // triangles' edges: exact predicates into a pair table, both directions,
+    // unsplit, the default walk, each side's rays from its kept triangles (or
+    // from an edge list the library made from the same triangles), and A's
+    // hierarchy four-wide with at most 2^27 groups (27-bit node ids on the
+    // walk's stack).  One walk per group of B triangles instead of one per
+    // edge of both sides, and B needs no hierarchy: whole joins 72.4 -> 15.9
+    // ms (dense, 12,007 x 9,001 meshes), 3.28 -> 2.20 ms (2 x 50,000
+    // ellipsoids, intersection), 0.68 -> 0.49 ms (2 x 60 spheres).  The other
+    // forms keep the rays: float32 hits and one-way joins depend on the
+    // segments themselves, two-pass sizing counts hits per ray, and shards
+    // are defined by rays.
+    bool pairs_route = false;
+    PairJoin pj;
+    bool triangle_pairs_wanted() const {
+        const bool both = o.predicate == PIERCE_CONTAINMENT || (ab && ba);
+        return both && o.precision == PIERCE_EXACT && o.sizing != PIERCE_SIZING_TWO_PASS && o.traversal == 0 &&
+               shard_n() == 1 && o.edge_source != PIERCE_EDGES_DATASET;
+    }
+    // every edge the side would trace is an edge of its kept triangles
+    bool triangle_edges(int d, int64_t kept) const {
+        const pierce_dataset* ds = d ? B : A;
+        return o.edge_source == PIERCE_EDGES_TRIANGLES || ds->ne == 0 || ds->edges_of_tris ||
+               2 * kept < (int64_t)ds->nt;
+    }
     // Ray lists of the sides that trace their kept triangles' edges: the
     // edges of the side's per-join soup, G triangles per group, listed group
     // by group; a side's groups are filtered against the other side's
@@ -1045,8 +1073,8 @@ struct Join {
 
     // LEARNED sizing of an overlap join, once its hierarchies exist: the
     // network's prediction is capped by 4 x the sampled incidence bound
-    // (k_group_incidences: 1/64 of A's kept groups against B's kept
-    // triangles) + 4096.  Objects far longer than their neighbours (tubes)
+    // (k_unit_incidences: 1/64 of B's kept groups against A's kept triangles;
+    // k_group_incidences, A's against B's, where the join traces rays) + 4096.  Objects far longer than their neighbours (tubes)
     // have boxes that meet nearly everything, which the network's features
     // cannot see; their kept groups are small.  A cap below the true count
     // costs only the two-pass rerun.
@@ -1055,7 +1083,11 @@ struct Join {
         if (int s = scratch(ctx, SLOT_AUX, 64, &pc)) return s;
         unsigned long long* d_count = static_cast<unsigned long long*>(pc) + 2;
         constexpr int kStep = 64;
-        if (int s = launch_group_incidences(ctx, va.soup, va.num_tris, groups_a_, kStep, vb, d_count)) return s;
+        if (pairs_route) {
+            if (int s = launch_unit_incidences(ctx, va, pj, kStep, d_count)) return s;
+        } else if (int s = launch_group_incidences(ctx, va.soup, va.num_tris, groups_a_, kStep, vb, d_count)) {
+            return s;
+        }
         int64_t n = 0;
         if (int s = host_value(ctx, d_count, 8, &n, "sampled incidences")) return s;
         const uint64_t cap = 4 * (uint64_t)n * kStep + 4096;
@@ -1430,27 +1462,15 @@ struct Join {
             if (int s = launch_chunk_cull(ctx, false, A->d_vertices, A->d_indices, A->d_tri_to_object, va, act_a, objB,
                                           tchunk_a, (uint32_t*)ta, words + 5, nullptr, chunk_list, words + 8))
                 return s;
-            bool filtered[2] = {false, false};
-            if (int s = grouped_side(0, tchunk_a, (uint32_t*)ta, leaf_a, &objB_, &filtered[0])) return s;
+            bool filtered = false;
+            if (int s = grouped_side(0, tchunk_a, (uint32_t*)ta, leaf_a, &objB_, &filtered)) return s;
             groups_a_ = group_size(leaf_a);
             if (int s = launch_chunk_cull(ctx, false, B->d_vertices, B->d_indices, B->d_tri_to_object, vb, act_b, va,
                                           tchunk_b, (uint32_t*)tb, words + 6, nullptr, chunk_list, words + 8))
                 return s;
-            if (int s = grouped_side(1, tchunk_b, (uint32_t*)tb, leaf_b, &va, &filtered[1])) return s;
-            const bool use[2] = {triangle_rays(0, true), triangle_rays(1, true)};
-            const int G[2] = {group_size(leaf_a), group_size(leaf_b)};
-            // rays: A's groups against B's kept triangles; B's groups met A's already
-            const bool pre[2] = {false, filtered[1]};
-            if (int s = soup_ray_lists(use, G, pre)) return s;
-            if (!use[0])
-                if (int s = launch_chunk_cull(ctx, true, nullptr, nullptr, nullptr, va, act_a, vb, echunk_a, list[0],
-                                              words + 0, nullptr, chunk_list, words + 8))
-                    return s;
-            if (!use[1])
-                if (int s = launch_chunk_cull(ctx, true, nullptr, nullptr, nullptr, vb, act_b, va, echunk_b, list[1],
-                                              words + 1, nullptr, chunk_list, words + 8))
-                    return s;
-            listed[0] = listed[1] = true;
+            if (int s = pair_side(tchunk_b, (uint32_t*)tb)) return s;
+            if (!pairs_route)
+                if (int s = ray_side()) return s;
             timer.span(b0, timer.record(), &st.ms_build);
             return PIERCE_OK;
         }
@@ -1540,6 +1560,81 @@ struct Join {
         st.active_triangles[0] = (uint64_t)na;
         st.active_triangles[1] = (uint64_t)nb;
         timer.span(b0, timer.record(), &st.ms_build);
+        return PIERCE_OK;
+    }
+
+    // B's side of a join by triangle pairs, where it applies (pairs_route):
+    // its kept groups of the flagged chunks, met by A's kept triangles.
+    int pair_side(const uint8_t* flags, uint32_t* ids) {
+        pairs_route = false;
+        const int G = group_size(join_leaf(o, A));
+        if (!triangle_pairs_wanted() || G != group_size(join_leaf(o, B)) || G > 16 || va.root_is_leaf || !va.nodes4 ||
+            va.num_tris / G >= (int64_t(1) << 27) || !triangle_edges(0, va.num_tris))
+            return PIERCE_OK;
+        const int64_t chunks = (int64_t)((B->nt + 31) / 32);
+        if (int s = launch_flag_list(ctx, flags, chunks, ids, words + 10)) return s;
+        int64_t nc = 0;
+        if (int s = host_value(ctx, words + 10, 8, &nc, "active chunks")) return s;
+        const int64_t ng = nc * (32 / G);
+        if (ng * G >= (int64_t(1) << 30)) return PIERCE_OK;
+        void *sp = nullptr, *gp = nullptr, *fp = nullptr;
+        if (int s = scratch(ctx, SLOT_RED_SOUP_B, 48 * 32 * (size_t)std::max<int64_t>(nc, 1), &sp)) return s;
+        if (int s = scratch(ctx, SLOT_GROUPS, 96 * (size_t)std::max<int64_t>(ng, 1) + 512, &gp)) return s;
+        if (int s = scratch(ctx, SLOT_LISTED_A, (size_t)(va.num_tris / G) + 64, &fp)) return s;
+        if (int s = build_group_units(ctx, B->d_vertices, B->d_indices, B->d_tri_to_object, (int64_t)B->nt, ids, nc, G,
+                                      gp, (float4*)sp, va, words + 12, B->num_parts ? B->d_obj_part : nullptr,
+                                      &pj.units))
+            return s;
+        pj.bsoup = (const float4*)sp;
+        pj.b_count = words + 12;
+        pj.b_part = B->d_obj_part;
+        pj.G = G;
+        pj.a_listed = (uint8_t*)fp;
+        // entries left for the next round: up to 512 of each resident warp's
+        pj.spill_cap = std::min<uint64_t>((uint64_t)std::max<int64_t>(ng, 32) * 512, 1ull << 22);
+        void* wp = nullptr;
+        if (int s = scratch(ctx, SLOT_SPILL, 64 + 2 * 8 * pj.spill_cap, &wp)) return s;
+        pj.work = static_cast<unsigned long long*>(wp);
+        pj.spill = reinterpret_cast<uint2*>(pj.work + 8);
+        pj.amb_queue = amb_queue;
+        pj.amb_cap = amb_cap;
+        int64_t kept = nc * 32;  // at most; the exact count only where it decides
+        if (!triangle_edges(1, kept)) {
+            if (int s = host_value(ctx, words + 12, 8, &kept, "kept groups")) return s;
+            kept *= G;
+            if (!triangle_edges(1, kept)) return PIERCE_OK;
+        }
+        pairs_route = true;
+        return PIERCE_OK;
+    }
+
+    // B's per-join hierarchy over the groups that meet A's kept triangles,
+    // and the ray lists of both sides.
+    int ray_side() {
+        uint8_t* act_a = active;
+        uint8_t* act_b = active + std::max(A->num_objects, 1);
+        uint8_t* tchunk_b = chunk_flags + (A->nt + 31) / 32 + 1;
+        uint8_t* echunk_a = tchunk_b + (B->nt + 31) / 32 + 1;
+        uint8_t* echunk_b = echunk_a + (A->ne + 31) / 32 + 1;
+        const int leaf_a = join_leaf(o, A), leaf_b = join_leaf(o, B);
+        void* tb = nullptr;
+        if (int s = scratch(ctx, SLOT_TRIS_B, 4 * (B->nt + 64), &tb)) return s;
+        bool filtered = false;
+        if (int s = grouped_side(1, tchunk_b, (uint32_t*)tb, leaf_b, &va, &filtered)) return s;
+        const bool use[2] = {triangle_rays(0, true), triangle_rays(1, true)};
+        const int G[2] = {group_size(leaf_a), group_size(leaf_b)};
+        // rays: A's groups against B's kept triangles; B's groups met A's already
+        const bool pre[2] = {false, filtered};
+        if (int s = soup_ray_lists(use, G, pre)) return s;
+        if (!use[0])
+            if (int s = launch_chunk_cull(ctx, true, nullptr, nullptr, nullptr, va, act_a, vb, echunk_a, list[0],
+                                          words + 0, nullptr, chunk_list, words + 8))
+                return s;
+        if (!use[1])
+            if (int s = launch_chunk_cull(ctx, true, nullptr, nullptr, nullptr, vb, act_b, va, echunk_b, list[1],
+                                          words + 1, nullptr, chunk_list, words + 8))
+                return s;
+        listed[0] = listed[1] = true;
         return PIERCE_OK;
     }
 
@@ -1693,7 +1788,14 @@ struct Join {
             if (int s = scratch(ctx, SLOT_TABLE, slots * 8, &p)) return s;
             uint64_t* table = static_cast<uint64_t*>(p);
             cudaMemsetAsync(table, 0xFF, slots * 8, ctx->stream);
-            if (int s = edge_rays(2, nullptr, nullptr, nullptr, nullptr, nullptr, table, slots)) return s;
+            if (pairs_route) {
+                const int b = timer.record();
+                pj.defer = defer;
+                if (int s = launch_tri_pairs(ctx, va, pj, table, slots)) return s;
+                timer.span(b, timer.record(), &st.ms_edge_rays[0]);
+            } else if (int s = edge_rays(2, nullptr, nullptr, nullptr, nullptr, nullptr, table, slots)) {
+                return s;
+            }
             uint32_t bits = 0;
             if (int s = read_device_error(ctx, &bits)) return s;
             if (bits & ERR_STACK_OVERFLOW) return set_error(PIERCE_ERR_STACK_OVERFLOW, "BVH traversal stack overflow");
@@ -1988,7 +2090,12 @@ struct Join {
         }
         s = prepare();
         if (s) return s;
-        if (strict_capacity && o.predicate == PIERCE_OVERLAP && groups_a_ > 0 && A->num_parts == 0)
+        // A prediction up to 2^22 pairs stands: its table (64 MB at the default
+        // load) takes about 30 us to clear and compact, the sampled bound 30
+        // us and more and a host round trip (0.04 ms on 128 tubes x 6,400
+        // ellipsoids, 1.4 ms on the dense join of 21,008 meshes).
+        if (strict_capacity && o.predicate == PIERCE_OVERLAP && groups_a_ > 0 && A->num_parts == 0 &&
+            o.expected_pairs > (1ull << 22))
             if ((s = cap_learned_size())) return s;
         s = run_predicate(out);
         if (strict_capacity && (s == PIERCE_ERR_HASH_FULL || s == PIERCE_ERR_OUTPUT_OVERFLOW)) {
@@ -1999,6 +2106,11 @@ struct Join {
             cudaMemsetAsync(ctx->d_err, 0, sizeof(uint32_t), ctx->stream);
             // the traversal counters describe the join that produced the pairs
             cudaMemsetAsync(ctx->d_counters, 0, sizeof(DevCounters), ctx->stream);
+            // which traces rays: B's hierarchy and the ray lists are still to come
+            if (pairs_route) {
+                pairs_route = false;
+                if ((s = ray_side())) return s;
+            }
             s = run_predicate(out);
         }
         const int t1 = timer.record();
@@ -2018,6 +2130,7 @@ struct Join {
         st.hash_accesses = c.hash_accesses;
         st.hash_contentions = c.hash_contentions;
         st.num_pairs = (*out)->count;
+        if (pairs_route) st.active_triangles[1] = c.kept_b * (uint64_t)pj.G;
         return PIERCE_OK;
     }
 

@@ -37,7 +37,7 @@ struct DevCounters {
     unsigned long long parity_rays;
     unsigned long long hash_accesses;
     unsigned long long hash_contentions;
-    unsigned long long pad;
+    unsigned long long kept_b;  // joins by triangle pairs: B's kept groups
 };
 
 // Binary BVH node holding the boxes of its two children (64 bytes, four
@@ -135,6 +135,30 @@ struct ColumnGrid {
 
 constexpr int kSizingScratchSlot = 21;  // 21 and 22: learned sizing (sizing.cu)
 
+// The walking side of a join by triangle pairs (pairs.cu): B's kept groups of
+// triangles without a hierarchy.
+struct GroupUnits {
+    int64_t bound = 0;                // candidate groups; the kept count is on the device
+    const float* gbox = nullptr;      // boxes of the candidates
+    const uint32_t* glist = nullptr;  // the kept candidates
+};
+
+// A join by triangle pairs: B's kept groups against A's per-join hierarchy.
+struct PairJoin {
+    GroupUnits units;
+    const float4* bsoup = nullptr;               // the kept groups' triangles, G each
+    const unsigned long long* b_count = nullptr; // kept groups
+    const int32_t* b_part = nullptr;             // partition per B object (partitioned joins)
+    int G = 4;                                   // triangles per group, both sides
+    uint8_t* a_listed = nullptr;                 // a byte per A leaf group
+    unsigned long long* work = nullptr;          // 8 words: deferred-test count, cursors, left-over counts
+    uint2* spill = nullptr;                      // two buffers of entries left for the next round
+    uint64_t spill_cap = 0;
+    unsigned long long* amb_queue = nullptr;
+    uint64_t amb_cap = 0;
+    bool defer = true;                           // queue undecided pairs (else exact inline)
+};
+
 struct BvhShape {
     int leaf_size = 1;
     int root_is_leaf = 1;
@@ -229,6 +253,7 @@ struct pierce_dataset {
     float* d_tri_chunk_box = nullptr;
     float* d_edge_chunk_box = nullptr;
     int edges_grouped = 0;  // edge sources non-decreasing (edges grouped by object)
+    int edges_of_tris = 0;  // the library made the edges itself: exactly the triangles' edges
     // hierarchy over the object boxes (with its four-wide copy), which the
     // per-join path culls against: built by the first join that needs it
     // and kept, since it depends only on the objects and their partitions
@@ -330,11 +355,23 @@ int build_grouped_lbvh(pierce_ctx* ctx, const float* verts, const uint32_t* idx,
                        Node* nodes, BvhShape* shape, const DevDataset* filter = nullptr,
                        unsigned long long* d_count = nullptr, int64_t* kept = nullptr,
                        const int32_t* obj_part = nullptr, int32_t num_parts = 0, int2* part_roots = nullptr);
+int build_group_units(pierce_ctx* ctx, const float* verts, const uint32_t* idx, const int32_t* t2o, int64_t nt,
+                      const uint32_t* chunk_list, int64_t n_chunks, int G, void* group_scratch, float4* soup,
+                      const DevDataset& filter, unsigned long long* d_count, const int32_t* obj_part,
+                      GroupUnits* out);
 int launch_group_filter(pierce_ctx* ctx, const float* gbox, int64_t ng, const DevDataset& other,
                         const int32_t* gt2o, const int32_t* obj_part, uint8_t* flags);
 // partitioned datasets: *mixed |= some group of a flagged chunk spans two partitions
 int launch_group_mixed(pierce_ctx* ctx, const uint8_t* chunk_flags, int64_t n_chunks, const int32_t* t2o,
                        const int32_t* obj_part, int64_t nt, int G, int32_t* mixed);
+
+// join.cu, pairs.cu: the pair tests of a join by triangle pairs into a pair
+// hash set, and its ray count
+int launch_pair_rays(pierce_ctx* ctx, const float4* asoup, int64_t na, const uint8_t* a_listed, const float4* bsoup,
+                     const unsigned long long* b_count, int64_t b_bound, int G);
+int launch_unit_incidences(pierce_ctx* ctx, const DevDataset& a, const PairJoin& j, int step,
+                           unsigned long long* count);
+int launch_tri_pairs(pierce_ctx* ctx, const DevDataset& a, const PairJoin& j, uint64_t* table, uint64_t slots);
 
 // sortscan.cu (CUB library calls)
 int sort_u32_pairs(pierce_ctx* ctx, uint32_t* keys_in, uint32_t* keys_out, uint32_t* vals_in, uint32_t* vals_out,

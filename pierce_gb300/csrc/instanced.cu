@@ -165,6 +165,7 @@ extern "C" int pierce_dataset_create_instanced(pierce_ctx* ctx, const pierce_mes
     ds->nt = nt;
     ds->ne = (tuning && tuning->skip_edges) ? 0 : ne;  // skip_edges: rays come from the triangles
     ds->num_objects = num_meshes;
+    ds->edges_of_tris = 1;  // the template's edges, over the same vertices
     void *d_blob = nullptr, *d_inst = nullptr, *d_off = nullptr;
     int s = PIERCE_OK;
     do {

@@ -952,6 +952,28 @@ __global__ void __launch_bounds__(256) k_group_soup(const float4* __restrict__ g
     }
 }
 
+// The kept groups' triangles in list order (no hierarchy: the walking side of
+// a join by triangle pairs), G per group; the kept count stays on the device.
+__global__ void __launch_bounds__(256) k_unit_soup(const uint32_t* __restrict__ glist,
+                                                   const unsigned long long* __restrict__ count, int G,
+                                                   const uint32_t* __restrict__ chunk_list,
+                                                   const float* __restrict__ verts, const uint32_t* __restrict__ idx,
+                                                   const int32_t* __restrict__ t2o, int64_t nt,
+                                                   float4* __restrict__ soup) {
+    const int per_chunk = 32 / G;
+    const int64_t n = (int64_t)*count * G;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t g = __ldg(glist + i / G);
+        const int64_t t = group_item(chunk_list[g / per_chunk], (int)(g % per_chunk), G, (int)(i % G), nt);
+        const float3 a = load_vertex(verts, __ldg(idx + 3 * t));
+        const float3 b = load_vertex(verts, __ldg(idx + 3 * t + 1));
+        const float3 c = load_vertex(verts, __ldg(idx + 3 * t + 2));
+        soup[3 * i + 0] = make_float4(a.x, a.y, a.z, __int_as_float(__ldg(t2o + t)));
+        soup[3 * i + 1] = make_float4(b.x, b.y, b.z, __int_as_float((int)t));
+        soup[3 * i + 2] = make_float4(c.x, c.y, c.z, 0.0f);
+    }
+}
+
 // Leaves of the group hierarchy (one group each) become soup ranges of G.
 __global__ void k_group_leaves(Node* nodes, int64_t num_nodes, int G) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < num_nodes; i += (int64_t)gridDim.x * blockDim.x) {
@@ -1164,6 +1186,39 @@ int build_grouped_lbvh(pierce_ctx* ctx, const float* verts, const uint32_t* idx,
         shape->num_nodes = gshape.num_nodes;
     }
     return check_cuda(cudaGetLastError(), "grouped bvh build");
+}
+
+// The walking side of a join by triangle pairs: the groups of G consecutive
+// triangles of the listed chunks whose box meets a leaf item of `filter`, as
+// a soup in list order with their boxes (gbox[6 g] of group g = glist[j]).
+// The number kept stays in *d_count; group_scratch as build_grouped_lbvh's.
+int build_group_units(pierce_ctx* ctx, const float* verts, const uint32_t* idx, const int32_t* t2o, int64_t nt,
+                      const uint32_t* chunk_list, int64_t n_chunks, int G, void* group_scratch, float4* soup,
+                      const DevDataset& filter, unsigned long long* d_count, const int32_t* obj_part,
+                      GroupUnits* out) {
+    cudaStream_t st = ctx->stream;
+    const int64_t ng = n_chunks * (32 / G);
+    *out = GroupUnits{};
+    out->bound = ng;
+    if (ng == 0) return check_cuda(cudaMemsetAsync(d_count, 0, 8, st), "group units");
+    char* q = static_cast<char*>(group_scratch);
+    float* gbox = reinterpret_cast<float*>(q + 48 * ng);
+    uint32_t* gidx = reinterpret_cast<uint32_t*>(q + 72 * ng);
+    int32_t* gt2o = reinterpret_cast<int32_t*>(q + 84 * ng);
+    k_group_boxes<<<(unsigned)std::max<int64_t>(1, std::min<int64_t>((n_chunks + 7) / 8, (int64_t)ctx->sm_count * 16)),
+                    256, 0, st>>>(verts, idx, t2o, nt, chunk_list, n_chunks, G, gbox, gidx, gt2o);
+    ctx->launches += 1;
+    uint8_t* flags = reinterpret_cast<uint8_t*>(q + 88 * ng);
+    char* lq = q + 88 * ng + ng;
+    lq += (256 - ((uintptr_t)lq & 255)) & 255;
+    uint32_t* glist = reinterpret_cast<uint32_t*>(lq);
+    if (int s = launch_group_filter(ctx, gbox, ng, filter, obj_part ? gt2o : nullptr, obj_part, flags)) return s;
+    if (int s = select_flagged(ctx, flags, ng, glist, d_count)) return s;
+    k_unit_soup<<<grid_for(ctx, ng * G, 256), 256, 0, st>>>(glist, d_count, G, chunk_list, verts, idx, t2o, nt, soup);
+    ctx->launches += 1;
+    out->gbox = gbox;
+    out->glist = glist;
+    return check_cuda(cudaGetLastError(), "group units");
 }
 
 int build_bvh(pierce_ctx* ctx, pierce_dataset* ds, int leaf_size) {

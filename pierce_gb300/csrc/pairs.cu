@@ -1,0 +1,621 @@
+// Overlap by triangle pairs: the kept triangle groups of B against A's
+// per-join hierarchy, every reached pair of triangles tested once.
+//
+// Two closed triangles meet exactly when an edge of one meets the other, so
+// with exact predicates the pairs of a two-way join are those of the edge
+// rays of both sides' kept triangles (join.cu, mesh_overlap_edges.cu:105-208)
+// -- but one walk per group of B triangles replaces a walk per edge of both
+// sides, only A needs a hierarchy, and a triangle pair is decided from its
+// plane sides and two orientations instead of six segment tests.
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <cstring>
+
+#include "common.cuh"
+#include "hash.cuh"
+#include "predicates.cuh"
+
+namespace pgpu {
+
+namespace {
+
+constexpr int kPairWarps = 4;        // warps per block
+constexpr int kPairUnits = 32;       // B groups a warp walks together
+constexpr int kPairStack = 512;      // walk entries per warp
+constexpr int kPairReserve = 144;    // of them left for a single entry's subtree (48 levels x 3)
+constexpr int kPairLeafQueue = 160;  // reached (group, leaf) pairs: < 32 left over + 32 x 4
+constexpr int kPairTriQueue = 64;    // triangle pairs: < 32 left over + 32
+
+struct WarpWork {
+    float box[6][kPairUnits];
+    uint32_t unit[kPairUnits];       // the groups in hand
+    uint32_t stack[kPairStack];      // node << 5 | unit
+    uint32_t leafq[kPairLeafQueue];  // leaf group << 5 | unit
+    uint2 triq[kPairTriQueue];       // (A soup triangle, B soup triangle)
+};
+
+}  // namespace
+
+struct PairParams {
+    DevDataset a;                         // soup, nodes4, part_roots of A's per-join hierarchy
+    const float4* bsoup;                  // B's kept groups, G triangles each
+    const unsigned long long* b_count;    // their number
+    const float* gbox;                    // boxes of B's candidate groups ...
+    const uint32_t* glist;                // ... and the kept ones among them
+    const int32_t* b_part;                // partition per B object (partitioned joins)
+    int G;                                // triangles per group, both sides
+    uint64_t* table;
+    uint64_t mask;
+    uint32_t* err;
+    DevCounters* ctr;
+    unsigned long long* cursor;
+    unsigned long long* amb_queue;        // undecided pairs: B triangle << 32 | A triangle
+    unsigned long long* amb_count;
+    uint64_t amb_cap;
+    uint8_t* a_listed;                    // per A leaf group: meets the box of a kept B triangle
+    // rounds: entries (group, node) left by the round before (null: every
+    // group from the root), and where a warp leaves what is still on its
+    // stack after `budget` steps (spill null: it carries on)
+    const uint2* entries;
+    const unsigned long long* n_entries;
+    uint2* spill;
+    unsigned long long* n_spill;
+    uint64_t spill_cap;
+    int budget;
+};
+
+// Closed triangle against closed triangle in float32.  Both plane-side tests
+// with the forward error bound of certain_sign first; when every side is
+// certain and both triangles straddle the other's plane, the two segments in
+// which they cut the planes' common line overlap exactly when two
+// orientations agree (Guigue and Devillers, "Fast and Robust
+// Triangle-Triangle Overlap Test Using Orientation Predicates", 2003).  A
+// vertex of one that is a vertex of the other (duplicated meshes, contacts)
+// is a common point when one of the two certainly has an area.
+// SEG_AMBIGUOUS: some sign is not certain.
+__device__ __forceinline__ int tri_tri_fp32_class(float3 a0, float3 a1, float3 a2, float3 b0, float3 b1, float3 b2) {
+    int s0, s1, s2, t0, t1, t2;
+    bool area;
+    {
+        const float3 u = f3sub(a1, a0), v = f3sub(a2, a0);
+        const float3 n = f3cross(u, v), np = f3cross_perm(u, v);
+        const float3 p = f3sub(b0, a0), q = f3sub(b1, a0), r = f3sub(b2, a0);
+        t0 = certain_sign(f3dot(p, n), f3dot_abs(p, np), 12.0f);
+        t1 = certain_sign(f3dot(q, n), f3dot_abs(q, np), 12.0f);
+        t2 = certain_sign(f3dot(r, n), f3dot_abs(r, np), 12.0f);
+        if (t0 && t0 == t1 && t0 == t2) return SEG_MISS;
+        area = certain_sign(n.x, np.x, 8.0f) || certain_sign(n.y, np.y, 8.0f) || certain_sign(n.z, np.z, 8.0f);
+    }
+    {
+        const float3 u = f3sub(b1, b0), v = f3sub(b2, b0);
+        const float3 n = f3cross(u, v), np = f3cross_perm(u, v);
+        const float3 p = f3sub(a0, b0), q = f3sub(a1, b0), r = f3sub(a2, b0);
+        s0 = certain_sign(f3dot(p, n), f3dot_abs(p, np), 12.0f);
+        s1 = certain_sign(f3dot(q, n), f3dot_abs(q, np), 12.0f);
+        s2 = certain_sign(f3dot(r, n), f3dot_abs(r, np), 12.0f);
+        if (s0 && s0 == s1 && s0 == s2) return SEG_MISS;
+        area = area || certain_sign(n.x, np.x, 8.0f) || certain_sign(n.y, np.y, 8.0f) || certain_sign(n.z, np.z, 8.0f);
+    }
+    if (!s0 || !s1 || !s2 || !t0 || !t1 || !t2) {
+        const bool shared = same_point(a0, b0) || same_point(a0, b1) || same_point(a0, b2) || same_point(a1, b0) ||
+                            same_point(a1, b1) || same_point(a1, b2) || same_point(a2, b0) || same_point(a2, b1) ||
+                            same_point(a2, b2);
+        return shared && area ? SEG_HIT : SEG_AMBIGUOUS;
+    }
+    // a0 and b0: the vertices alone on their side (rotations keep the planes' orientation)
+    if (s0 == s2) { const float3 x = a0; a0 = a1; a1 = a2; a2 = x; s0 = s1; }          // a1 alone
+    else if (s0 == s1) { const float3 x = a0; a0 = a2; a2 = a1; a1 = x; s0 = s2; }     // a2 alone
+    if (t0 == t2) { const float3 x = b0; b0 = b1; b1 = b2; b2 = x; t0 = t1; }
+    else if (t0 == t1) { const float3 x = b0; b0 = b2; b2 = b1; b1 = x; t0 = t2; }
+    // both lone vertices on the positive side of the other plane: a lone
+    // vertex below it turns round when that plane's triangle does
+    if (s0 < 0) { const float3 x = b1; b1 = b2; b2 = x; }
+    if (t0 < 0) { const float3 x = a1; a1 = a2; a2 = x; }
+    // apart when (b1 - a0) . ((a1 - a0) x (b0 - a0)) or (b2 - a0) . ((b0 -
+    // a0) x (a2 - a0)) is positive
+    const float3 p = f3sub(b0, a0), u = f3sub(a1, a0), v = f3sub(b1, a0), w = f3sub(a2, a0), x = f3sub(b2, a0);
+    const float3 c1 = f3cross(u, p), m1 = f3cross_perm(u, p);
+    const int o1 = certain_sign(f3dot(v, c1), f3dot_abs(v, m1), 12.0f);
+    const float3 c2 = f3cross(p, w), m2 = f3cross_perm(p, w);
+    const int o2 = certain_sign(f3dot(x, c2), f3dot_abs(x, m2), 12.0f);
+    if (o1 > 0 || o2 > 0) return SEG_MISS;
+    if (o1 == 0 || o2 == 0) return SEG_AMBIGUOUS;
+    return SEG_HIT;
+}
+
+
+// The edge definition, exact: an edge of one triangle meets the other.
+__device__ __noinline__ bool tri_tri_exact(float3 a0, float3 a1, float3 a2, float3 b0, float3 b1, float3 b2,
+                                           PredCounters& pc) {
+    bool hit = false;
+#pragma unroll 1
+    for (int side = 0; side < 2 && !hit; ++side) {
+#pragma unroll 1
+        for (int k = 0; k < 3 && !hit; ++k) {
+            hit = seg_tri_exact(b0, b1, a0, a1, a2, pc);
+            const float3 x = b0;
+            b0 = b1;
+            b1 = b2;
+            b2 = x;
+        }
+        const float3 x = a0, y = a1, z = a2;
+        a0 = b0; a1 = b1; a2 = b2;
+        b0 = x; b1 = y; b2 = z;
+    }
+    return hit;
+}
+
+// Each warp takes a few B groups (units) at a time and walks them over A's
+// four-wide nodes together: the (node, unit) entries still to visit lie on
+// one stack in shared memory, every lane visits one entry per step and the
+// children it meets go back on the stack, so the lanes stay busy however the
+// lengths of the units' walks differ.  Reached leaves are queued the same
+// way; a full warp of them finds the pairs of triangles whose boxes meet, and
+// a full warp of those runs the triangle test.  U: triangles of a group
+// tested against each other at a time (G when G <= 4); BIG: G > 4, in blocks
+// of 4 x 4.
+//
+// What it replaces, the edge rays of both sides, was bound by divergence
+// (7-11 of 32 lanes active: walks of different lengths in one warp) and by
+// the number of walks.  Measured against them on a GB300: dense join of
+// 12,007 x 9,001 meshes 64.2 -> 8.9 ms (67 M rays and 1.8 G node visits
+// become 3.2 M walks and 123 M visits), 2 x 50,000 ellipsoids 1.13 -> 0.35
+// ms, 400,000 x 100,000 ellipsoids 1.86 -> 0.54 ms, 64 batched joins 28.3 ->
+// 4.2 ms.  6 blocks of 128 per SM (80 registers): 8.86 ms on the dense join
+// against 9.42 with 8 blocks (64 registers, spills) and 9.37 with 5.
+template <int U, bool BIG, bool DEFER>
+__global__ void __launch_bounds__(32 * kPairWarps, DEFER ? 6 : 4) k_tri_pairs(PairParams P) {
+    __shared__ WarpWork work[kPairWarps];
+    const int lane = threadIdx.x & 31;
+    const unsigned below = (1u << lane) - 1u;
+    WarpWork& W = work[threadIdx.x >> 5];
+    const int64_t n = P.entries ? (int64_t)min(*P.n_entries, (unsigned long long)P.spill_cap) : (int64_t)*P.b_count;
+    if (!P.entries && blockIdx.x == 0 && threadIdx.x == 0) P.ctr->kept_b = (unsigned long long)n;
+    // units per fetch: few when there are few, so that all warps share them
+    const int64_t warps = (int64_t)gridDim.x * kPairWarps;
+    const int per = (int)min((int64_t)kPairUnits, max((int64_t)1, n / warps));
+    const int G = BIG ? P.G : U;
+    const int side = BIG ? G / U : 1;  // blocks per side of a leaf pair
+    PredCounters pc{0, 0};
+    uint32_t nodes = 0, tests = 0, hits = 0, probes = 0, ambiguous = 0;
+    int sp = 0, lq = 0, tq = 0, steps = 0;
+    bool more = true, finish = false;
+    // this lane's reached leaf, the block of it in hand and its pairs left:
+    // bit U j + i for A triangle ta + j, B triangle tb + i
+    int blk = side * side;
+    uint32_t leaf_a = 0, leaf_b = 0, mask = 0;
+    bool has_leaf = false;
+    float ga[6] = {0, 0, 0, 0, 0, 0};
+    for (;;) {
+        if (tq >= 32 || (tq > 0 && finish)) {
+            const int take = min(tq, 32);
+            tq -= take;
+            if (lane < take) {
+                const uint2 e = W.triq[tq + lane];
+                const float4 a0 = __ldg(P.a.soup + 3 * (size_t)e.x), a1 = __ldg(P.a.soup + 3 * (size_t)e.x + 1),
+                             a2 = __ldg(P.a.soup + 3 * (size_t)e.x + 2);
+                const float4 b0 = __ldg(P.bsoup + 3 * (size_t)e.y), b1 = __ldg(P.bsoup + 3 * (size_t)e.y + 1),
+                             b2 = __ldg(P.bsoup + 3 * (size_t)e.y + 2);
+                const float3 p0 = make_float3(a0.x, a0.y, a0.z), p1 = make_float3(a1.x, a1.y, a1.z),
+                             p2 = make_float3(a2.x, a2.y, a2.z);
+                const float3 q0 = make_float3(b0.x, b0.y, b0.z), q1 = make_float3(b1.x, b1.y, b1.z),
+                             q2 = make_float3(b2.x, b2.y, b2.z);
+                ++tests;
+                const int cls = tri_tri_fp32_class(p0, p1, p2, q0, q1, q2);
+                bool hit = cls == SEG_HIT;
+                if (cls == SEG_AMBIGUOUS) {
+                    ++ambiguous;
+                    if (DEFER) {
+                        const unsigned long long slot = atomicAdd(P.amb_count, 1ull);
+                        if (slot < P.amb_cap) P.amb_queue[slot] = ((unsigned long long)e.y << 32) | e.x;
+                        else atomicOr(P.err, ERR_AMBIGUOUS_OVERFLOW);
+                    } else {
+                        hit = tri_tri_exact(p0, p1, p2, q0, q1, q2, pc);
+                    }
+                }
+                if (hit) {
+                    ++hits;
+                    hash_insert(P.table, P.mask, pack_key(__float_as_int(a0.w), __float_as_int(b0.w)), P.err, probes);
+                }
+            }
+            __syncwarp();
+            continue;
+        }
+        // one pair of every lane that has some left goes on the queue
+        const unsigned left = __ballot_sync(0xFFFFFFFFu, mask != 0);
+        if (left) {
+            if (mask) {
+                const int bit = __ffs(mask) - 1;
+                mask &= mask - 1;
+                const int bi = BIG ? (blk - 1) % side : 0, bj = BIG ? (blk - 1) / side : 0;
+                W.triq[tq + __popc(left & below)] =
+                    make_uint2(leaf_a * G + (uint32_t)(bj * U + bit / U), leaf_b * G + (uint32_t)(bi * U + bit % U));
+            }
+            tq += __popc(left);
+            __syncwarp();
+            continue;
+        }
+        if (blk < side * side) {
+            // block (bj, bi) of the leaf pairs in hand: which boxes meet
+            const int bi = BIG ? blk % side : 0, bj = BIG ? blk / side : 0;
+            ++blk;
+            if (has_leaf) {
+                const float4* bs = P.bsoup + 3 * ((size_t)leaf_b * G + bi * U);
+                const float4* as = P.a.soup + 3 * ((size_t)leaf_a * G + bj * U);
+                float3 blo[U], bhi[U];
+#pragma unroll
+                for (int i = 0; i < U; ++i) {
+                    const float4 x = __ldg(bs + 3 * i), y = __ldg(bs + 3 * i + 1), z = __ldg(bs + 3 * i + 2);
+                    blo[i] = make_float3(fminf(x.x, fminf(y.x, z.x)), fminf(x.y, fminf(y.y, z.y)),
+                                         fminf(x.z, fminf(y.z, z.z)));
+                    bhi[i] = make_float3(fmaxf(x.x, fmaxf(y.x, z.x)), fmaxf(x.y, fmaxf(y.y, z.y)),
+                                         fmaxf(x.z, fmaxf(y.z, z.z)));
+                }
+                float3 ulo = make_float3(3.4e38f, 3.4e38f, 3.4e38f), uhi = make_float3(-3.4e38f, -3.4e38f, -3.4e38f);
+#pragma unroll
+                for (int j = 0; j < U; ++j) {
+                    const float4 x = __ldg(as + 3 * j), y = __ldg(as + 3 * j + 1), z = __ldg(as + 3 * j + 2);
+                    const float3 lo = make_float3(fminf(x.x, fminf(y.x, z.x)), fminf(x.y, fminf(y.y, z.y)),
+                                                  fminf(x.z, fminf(y.z, z.z)));
+                    const float3 hi = make_float3(fmaxf(x.x, fmaxf(y.x, z.x)), fmaxf(x.y, fmaxf(y.y, z.y)),
+                                                  fmaxf(x.z, fmaxf(y.z, z.z)));
+#pragma unroll
+                    for (int i = 0; i < U; ++i)
+                        if (box_overlap(lo.x, hi.x, lo.y, hi.y, lo.z, hi.z, blo[i], bhi[i])) mask |= 1u << (U * j + i);
+                    ulo = make_float3(fminf(ulo.x, lo.x), fminf(ulo.y, lo.y), fminf(ulo.z, lo.z));
+                    uhi = make_float3(fmaxf(uhi.x, hi.x), fmaxf(uhi.y, hi.y), fmaxf(uhi.z, hi.z));
+                }
+                if (BIG) {
+                    ulo = make_float3(ga[0], ga[1], ga[2]);
+                    uhi = make_float3(ga[3], ga[4], ga[5]);
+                }
+                // A's group is listed when its box meets a kept triangle's
+                bool listed = false;
+#pragma unroll
+                for (int i = 0; i < U; ++i)
+                    listed |= box_overlap(ulo.x, uhi.x, ulo.y, uhi.y, ulo.z, uhi.z, blo[i], bhi[i]);
+                if (listed) P.a_listed[leaf_a] = 1;
+            }
+            continue;
+        }
+        if (lq >= 32 || (lq > 0 && sp == 0)) {
+            const int take = min(lq, 32);
+            lq -= take;
+            has_leaf = lane < take;
+            if (has_leaf) {
+                const uint32_t e = W.leafq[lq + lane];
+                leaf_a = e >> 5;
+                leaf_b = W.unit[e & 31u];
+                if (BIG) {
+                    for (int k = 0; k < 3; ++k) {
+                        ga[k] = 3.4e38f;
+                        ga[3 + k] = -3.4e38f;
+                    }
+                    for (int t = 0; t < 3 * G; ++t) {
+                        const float4 v = __ldg(P.a.soup + 3 * (size_t)leaf_a * G + t);
+                        ga[0] = fminf(ga[0], v.x); ga[1] = fminf(ga[1], v.y); ga[2] = fminf(ga[2], v.z);
+                        ga[3] = fmaxf(ga[3], v.x); ga[4] = fmaxf(ga[4], v.y); ga[5] = fmaxf(ga[5], v.z);
+                    }
+                }
+            }
+            blk = 0;
+            __syncwarp();
+            continue;
+        }
+        if (sp > 0) {
+            if (P.spill && ++steps > P.budget) {
+                // a long walk: what is left of it goes to the next round
+                unsigned long long at = 0;
+                if (lane == 0) at = atomicAdd(P.n_spill, (unsigned long long)sp);
+                at = __shfl_sync(0xFFFFFFFFu, at, 0);
+                const int fit = (int)min((unsigned long long)sp, P.spill_cap - min(at, (unsigned long long)P.spill_cap));
+                for (int i = lane; i < fit; i += 32) {
+                    const uint32_t e = W.stack[sp - 1 - i];
+                    P.spill[at + i] = make_uint2(W.unit[e & 31u], e >> 5);
+                }
+                sp -= fit;
+                steps = 0;
+                __syncwarp();
+                if (fit) continue;
+            }
+            // the top entries, as many as leave room for their children; one
+            // entry's subtree alone needs at most kPairReserve
+            const int room = (kPairStack - kPairReserve - sp) / 3;
+            const int take = min(min(sp, 32), max(room, 1));
+            sp -= take;
+            const bool in = lane < take;
+            const uint32_t e = in ? W.stack[sp + lane] : 0u;
+            __syncwarp();
+            if (sp + 4 * take > kPairStack) {  // a hierarchy deeper than any this library builds
+                if (lane == 0) atomicOr(P.err, ERR_STACK_OVERFLOW);
+                sp = 0;
+                continue;
+            }
+            nodes += in ? 1u : 0u;
+            const uint32_t u = e & 31u;
+            const Node4* nd = P.a.nodes4 + (e >> 5);
+            const float4 lx = __ldg(&nd->lox), hx = __ldg(&nd->hix), ly = __ldg(&nd->loy), hy = __ldg(&nd->hiy);
+            const float4 lz = __ldg(&nd->loz), hz = __ldg(&nd->hiz);
+            const int4 ch = __ldg(&nd->ch);
+            const int cnt = __ldg(&nd->meta.x);
+            const float3 lo = make_float3(W.box[0][u], W.box[1][u], W.box[2][u]);
+            const float3 hi = make_float3(W.box[3][u], W.box[4][u], W.box[5][u]);
+            const bool h[4] = {box_overlap(lx.x, hx.x, ly.x, hy.x, lz.x, hz.x, lo, hi),
+                               box_overlap(lx.y, hx.y, ly.y, hy.y, lz.y, hz.y, lo, hi),
+                               box_overlap(lx.z, hx.z, ly.z, hy.z, lz.z, hz.z, lo, hi),
+                               box_overlap(lx.w, hx.w, ly.w, hy.w, lz.w, hz.w, lo, hi)};
+            const int c[4] = {ch.x, ch.y, ch.z, ch.w};
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const bool inner = in && h[j] && c[j] >= 0;
+                const bool leaf = in && h[j] && c[j] < 0 && ((cnt >> (8 * j)) & 0xFF);
+                const unsigned mi = __ballot_sync(0xFFFFFFFFu, inner), ml = __ballot_sync(0xFFFFFFFFu, leaf);
+                if (inner) W.stack[sp + __popc(mi & below)] = ((uint32_t)c[j] << 5) | u;
+                if (leaf) W.leafq[lq + __popc(ml & below)] = (((uint32_t)(~c[j]) / (uint32_t)G) << 5) | u;
+                sp += __popc(mi);
+                lq += __popc(ml);
+            }
+            __syncwarp();
+            continue;
+        }
+        if (more) {
+            unsigned long long b = 0;
+            if (lane == 0) b = atomicAdd(P.cursor, (unsigned long long)per);
+            const int64_t base = (int64_t)__shfl_sync(0xFFFFFFFFu, b, 0);
+            const bool item = lane < per && base + lane < n;
+            bool node = item, leaf = false;
+            uint32_t entry = (uint32_t)lane;  // node 0
+            if (item) {
+                uint2 e = make_uint2((uint32_t)(base + lane), 0);
+                if (P.entries) e = P.entries[base + lane];
+                W.unit[lane] = e.x;
+                const float* gb = P.gbox + 6 * (size_t)__ldg(P.glist + e.x);
+#pragma unroll
+                for (int k = 0; k < 6; ++k) W.box[k][lane] = __ldg(gb + k);
+                if (P.entries) {
+                    entry = (e.y << 5) | (uint32_t)lane;
+                } else if (P.a.part_roots) {
+                    const int32_t o = __float_as_int(__ldg(&P.bsoup[3 * (size_t)e.x * G].w));
+                    const int2 r = __ldg(P.a.part_roots + __ldg(P.b_part + o));
+                    node = r.x >= 0;
+                    leaf = r.x < 0 && r.y > 0;
+                    entry = ((node ? (uint32_t)r.x : (uint32_t)(~r.x) / (uint32_t)G) << 5) | (uint32_t)lane;
+                }
+            }
+            const unsigned mn = __ballot_sync(0xFFFFFFFFu, node), ml = __ballot_sync(0xFFFFFFFFu, leaf);
+            if (node) W.stack[__popc(mn & below)] = entry;
+            if (leaf) W.leafq[__popc(ml & below)] = entry;
+            sp = __popc(mn);
+            lq = __popc(ml);
+            steps = 0;
+            more = base + per < n;
+            __syncwarp();
+            continue;
+        }
+        if (tq == 0) break;
+        finish = true;  // the pairs left over
+    }
+    flush_counter(&P.ctr->node_visits, nodes);
+    flush_counter(&P.ctr->tri_tests, tests);
+    flush_counter(&P.ctr->raw_hits, hits);
+    flush_counter(&P.ctr->fp32_ambiguous, ambiguous);
+    flush_counter(&P.ctr->hash_accesses, probes);
+    flush_counter(&P.ctr->hash_contentions, probes - hits);
+    if (!DEFER) flush_counter(&P.ctr->fp64_ambiguous, pc.fp64_ambiguous);
+}
+
+// Exact answers of the queued triangle pairs.
+__global__ void __launch_bounds__(128) k_resolve_pairs(PairParams P) {
+    PredCounters pc{0, 0};
+    uint32_t probes = 0, hits = 0;
+    const unsigned long long n = min(*P.amb_count, (unsigned long long)P.amb_cap);
+    for (unsigned long long i = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; i < n;
+         i += (unsigned long long)gridDim.x * blockDim.x) {
+        const unsigned long long e = P.amb_queue[i];
+        const float4* a = P.a.soup + 3 * (size_t)(uint32_t)e;
+        const float4* b = P.bsoup + 3 * (size_t)(e >> 32);
+        const float4 a0 = __ldg(a), a1 = __ldg(a + 1), a2 = __ldg(a + 2);
+        const float4 b0 = __ldg(b), b1 = __ldg(b + 1), b2 = __ldg(b + 2);
+        if (!tri_tri_exact(make_float3(a0.x, a0.y, a0.z), make_float3(a1.x, a1.y, a1.z), make_float3(a2.x, a2.y, a2.z),
+                           make_float3(b0.x, b0.y, b0.z), make_float3(b1.x, b1.y, b1.z), make_float3(b2.x, b2.y, b2.z),
+                           pc))
+            continue;
+        ++hits;
+        hash_insert(P.table, P.mask, pack_key(__float_as_int(a0.w), __float_as_int(b0.w)), P.err, probes);
+    }
+    flush_counter(&P.ctr->fp64_ambiguous, pc.fp64_ambiguous);
+    flush_counter(&P.ctr->hash_accesses, probes);
+    flush_counter(&P.ctr->hash_contentions, probes - hits);
+}
+
+int launch_tri_pairs(pierce_ctx* ctx, const DevDataset& a, const PairJoin& j, uint64_t* table, uint64_t slots) {
+    cudaStream_t st = ctx->stream;
+    const int64_t na = a.num_tris / j.G;
+    // words of j.work: [0] deferred tests, then per round [1 + 2 r] cursor, [2 + 2 r] spilled entries
+    constexpr int kRounds = 3;
+    constexpr int kBudget = 192;
+    cudaMemsetAsync(j.work, 0, (1 + 2 * kRounds) * sizeof(unsigned long long), st);
+    cudaMemsetAsync(j.a_listed, 0, (size_t)na, st);
+    PairParams P;
+    std::memset(&P, 0, sizeof(P));
+    P.a = a;
+    P.bsoup = j.bsoup;
+    P.b_count = j.b_count;
+    P.gbox = j.units.gbox;
+    P.glist = j.units.glist;
+    P.b_part = j.b_part;
+    P.G = j.G;
+    P.table = table;
+    P.mask = slots - 1;
+    P.err = ctx->d_err;
+    P.ctr = ctx->d_counters;
+    P.amb_queue = j.amb_queue;
+    P.amb_count = j.work;
+    P.amb_cap = j.amb_cap;
+    P.a_listed = j.a_listed;
+    if (j.units.bound > 0) {
+        const int64_t blocks = std::min<int64_t>((j.units.bound + kPairWarps - 1) / kPairWarps, (int64_t)ctx->sm_count * 8);
+        const unsigned grid = (unsigned)std::max<int64_t>(blocks, 1), threads = 32 * kPairWarps;
+        // A group's walk is as long as what it meets (a coarse mesh's group
+        // meets thousands of leaves of a fine one): a warp leaves what a
+        // long walk still has on its stack to the next round, where it is
+        // spread over all warps (64 batched joins of levels 1 to 5: 12.2 ms
+        // in one round, 4.2 ms in three).
+        for (int r = 0; r < kRounds; ++r) {
+            P.cursor = j.work + 1 + 2 * r;
+            P.entries = r ? j.spill + (r - 1) * j.spill_cap : nullptr;
+            P.n_entries = r ? j.work + 2 * r : nullptr;
+            P.spill = r + 1 < kRounds ? j.spill + r * j.spill_cap : nullptr;
+            P.n_spill = j.work + 2 + 2 * r;
+            P.spill_cap = j.spill_cap;
+            P.budget = kBudget;
+#define PG_PAIRS(U, BIG)                                                                \
+    do {                                                                                \
+        if (j.defer) k_tri_pairs<U, BIG, true><<<grid, threads, 0, st>>>(P);            \
+        else k_tri_pairs<U, BIG, false><<<grid, threads, 0, st>>>(P);                   \
+    } while (0)
+            if (j.G == 1) PG_PAIRS(1, false);
+            else if (j.G == 2) PG_PAIRS(2, false);
+            else if (j.G == 4) PG_PAIRS(4, false);
+            else PG_PAIRS(4, true);
+#undef PG_PAIRS
+            ctx->launches += 1;
+        }
+        if (j.defer) {
+            k_resolve_pairs<<<ctx->sm_count * 4, 128, 0, st>>>(P);
+            ctx->launches += 1;
+        }
+    }
+    if (int s = check_cuda(cudaGetLastError(), "triangle pairs")) return s;
+    return launch_pair_rays(ctx, a.soup, na, j.a_listed, j.bsoup, j.b_count, j.units.bound, j.G);
+}
+
+// Pair-count bound for output sizing: B's kept groups are taken in runs of
+// `run` consecutive ones; for every step-th run, the different object pairs
+// (A object with a kept triangle whose box meets a group's box, the group's
+// object).  Every overlap pair has such a group and triangle, so step x this
+// count estimates an upper bound on the join's pairs; a run lies on one
+// patch of a mesh, whose groups mostly meet the same objects.  A warp per
+// sampled run: its lanes walk the run's groups together as k_tri_pairs does
+// and keep the pairs found in one set in shared memory, so a sample costs a
+// few steps of latency instead of whole walks by one thread.
+__global__ void __launch_bounds__(32 * kPairWarps) k_unit_incidences(PairParams P, int step, int min_runs,
+                                                                     unsigned long long* count) {
+    constexpr int kSeen = 512;       // slots of a warp's set of pairs
+    constexpr int kSeenMax = 352;    // pairs it takes (+ 32 of one step)
+    __shared__ float boxes[kPairWarps][6][kPairUnits];
+    __shared__ int32_t objs[kPairWarps][kPairUnits];
+    __shared__ uint32_t stacks[kPairWarps][kPairStack];  // node << 5 | group of the run
+    __shared__ unsigned long long seen[kPairWarps][kSeen];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const unsigned below = (1u << lane) - 1u;
+    uint32_t* stack = stacks[w];
+    const int64_t n = (int64_t)*P.b_count;
+    const int G = P.G;
+    // short runs where there are few groups, so that min_runs of them are sampled
+    const int run = (int)min((int64_t)kPairUnits, max((int64_t)1, n / ((int64_t)step * min_runs)));
+    unsigned long long local = 0;
+    for (int64_t s = (int64_t)blockIdx.x * kPairWarps + w; s * step * run < n; s += (int64_t)gridDim.x * kPairWarps) {
+        const int64_t g = s * step * run + lane;
+        int sp = (int)min((int64_t)run, n - s * step * run), ns = 0;
+        if (lane < sp) {
+            const float* gb = P.gbox + 6 * (size_t)__ldg(P.glist + g);
+#pragma unroll
+            for (int k = 0; k < 6; ++k) boxes[w][k][lane] = __ldg(gb + k);
+            objs[w][lane] = __float_as_int(__ldg(&P.bsoup[3 * (size_t)g * G].w));
+            stack[lane] = (uint32_t)lane;
+        }
+        for (int i = lane; i < kSeen; i += 32) seen[w][i] = kEmptyKey;
+        __syncwarp();
+        while (sp > 0) {
+            const int room = (kPairStack - kPairReserve - sp) / 3;
+            const int take = min(min(sp, 32), max(room, 1));
+            sp -= take;
+            const bool in = lane < take;
+            const uint32_t e = in ? stack[sp + lane] : 0u;
+            const uint32_t u = e & 31u;
+            __syncwarp();
+            if (sp + 4 * take > kPairStack) {
+                if (lane == 0) atomicOr(P.err, ERR_STACK_OVERFLOW);
+                break;
+            }
+            const Node4* nd = P.a.nodes4 + (e >> 5);
+            const float4 lx = __ldg(&nd->lox), hx = __ldg(&nd->hix), ly = __ldg(&nd->loy), hy = __ldg(&nd->hiy);
+            const float4 lz = __ldg(&nd->loz), hz = __ldg(&nd->hiz);
+            const int4 ch = __ldg(&nd->ch);
+            const int cnt = __ldg(&nd->meta.x);
+            const float3 lo = make_float3(boxes[w][0][u], boxes[w][1][u], boxes[w][2][u]);
+            const float3 hi = make_float3(boxes[w][3][u], boxes[w][4][u], boxes[w][5][u]);
+            const bool h[4] = {box_overlap(lx.x, hx.x, ly.x, hy.x, lz.x, hz.x, lo, hi),
+                               box_overlap(lx.y, hx.y, ly.y, hy.y, lz.y, hz.y, lo, hi),
+                               box_overlap(lx.z, hx.z, ly.z, hy.z, lz.z, hz.z, lo, hi),
+                               box_overlap(lx.w, hx.w, ly.w, hy.w, lz.w, hz.w, lo, hi)};
+            const int c[4] = {ch.x, ch.y, ch.z, ch.w};
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const bool inner = in && h[j] && c[j] >= 0;
+                const unsigned mi = __ballot_sync(0xFFFFFFFFu, inner);
+                if (inner) stack[sp + __popc(mi & below)] = ((uint32_t)c[j] << 5) | u;
+                sp += __popc(mi);
+                const bool leaf = in && h[j] && c[j] < 0 && ((cnt >> (8 * j)) & 0xFF);
+                if (!__any_sync(0xFFFFFFFFu, leaf)) continue;
+                for (int k = 0; k < G; ++k) {
+                    unsigned long long key = kEmptyKey;
+                    if (leaf) {
+                        const float4* t = P.a.soup + 3 * ((size_t)(~c[j]) + k);
+                        const float4 x = __ldg(t), y = __ldg(t + 1), z = __ldg(t + 2);
+                        if (box_overlap(fminf(x.x, fminf(y.x, z.x)), fmaxf(x.x, fmaxf(y.x, z.x)),
+                                        fminf(x.y, fminf(y.y, z.y)), fmaxf(x.y, fmaxf(y.y, z.y)),
+                                        fminf(x.z, fminf(y.z, z.z)), fmaxf(x.z, fmaxf(y.z, z.z)), lo, hi))
+                            key = pack_key(__float_as_int(x.w), objs[w][u]);
+                    }
+                    // a pair new to the set counts once (a full set takes no
+                    // more: pairs not in it count each time), whatever the
+                    // order of a step's insertions
+                    bool fresh = false;
+                    if (key != kEmptyKey) {
+                        uint32_t at = (uint32_t)fmix64(key) & (kSeen - 1);
+                        for (;;) {
+                            const unsigned long long cur =
+                                ns <= kSeenMax ? atomicCAS(&seen[w][at], kEmptyKey, key)
+                                               : *(volatile unsigned long long*)&seen[w][at];
+                            fresh = cur == kEmptyKey;
+                            if (fresh || cur == key) break;
+                            at = (at + 1) & (kSeen - 1);
+                        }
+                    }
+                    const int nf = __popc(__ballot_sync(0xFFFFFFFFu, fresh));
+                    local += (unsigned long long)nf;
+                    if (ns <= kSeenMax) ns += nf;
+                }
+            }
+            __syncwarp();
+        }
+        __syncwarp();
+    }
+    if (lane == 0 && local) atomicAdd(count, local);
+}
+
+int launch_unit_incidences(pierce_ctx* ctx, const DevDataset& a, const PairJoin& j, int step,
+                           unsigned long long* count) {
+    cudaMemsetAsync(count, 0, sizeof(unsigned long long), ctx->stream);
+    if (j.units.bound <= 0) return check_cuda(cudaGetLastError(), "unit incidences");
+    PairParams P;
+    std::memset(&P, 0, sizeof(P));
+    P.a = a;
+    P.bsoup = j.bsoup;
+    P.b_count = j.b_count;
+    P.gbox = j.units.gbox;
+    P.glist = j.units.glist;
+    P.G = j.G;
+    P.err = ctx->d_err;
+    const int min_runs = 4096;
+    const int64_t runs = std::max<int64_t>(min_runs, j.units.bound / ((int64_t)step * kPairUnits) + 1);
+    const int64_t blocks = std::min<int64_t>((runs + kPairWarps - 1) / kPairWarps, (int64_t)ctx->sm_count * 16);
+    k_unit_incidences<<<(unsigned)blocks, 32 * kPairWarps, 0, ctx->stream>>>(P, step, min_runs, count);
+    ctx->launches += 1;
+    return check_cuda(cudaGetLastError(), "unit incidences");
+}
+
+}  // namespace pgpu

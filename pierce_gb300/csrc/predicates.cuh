@@ -69,7 +69,7 @@ __device__ __forceinline__ void two_prod(double a, double b, double& x, double& 
 }
 
 // h = e + f (both non-overlapping, increasing magnitude); returns |h|.
-__device__ __noinline__ int exp_sum(int elen, const double* e, int flen, const double* f, double* h) {
+static __device__ __noinline__ int exp_sum(int elen, const double* e, int flen, const double* f, double* h) {
     if (elen == 0) {
         for (int i = 0; i < flen; ++i) h[i] = f[i];
         return flen;
@@ -98,7 +98,7 @@ __device__ __noinline__ int exp_sum(int elen, const double* e, int flen, const d
 }
 
 // h = e * b; returns |h|.
-__device__ __noinline__ int exp_scale(int elen, const double* e, double b, double* h) {
+static __device__ __noinline__ int exp_scale(int elen, const double* e, double b, double* h) {
     if (elen == 0 || b == 0.0) {
         h[0] = 0.0;
         return 1;
@@ -120,7 +120,7 @@ __device__ __noinline__ int exp_scale(int elen, const double* e, double b, doubl
 }
 
 // h = e * f for short expansions (|e|, |f| <= 16); returns |h|.
-__device__ __noinline__ int exp_mul(int elen, const double* e, int flen, const double* f, double* h) {
+static __device__ __noinline__ int exp_mul(int elen, const double* e, int flen, const double* f, double* h) {
     double acc[64], tmp[32], sum[64];
     int alen = 0;
     for (int k = 0; k < flen; ++k) {
@@ -158,7 +158,7 @@ __device__ __forceinline__ int exp_diff(float b, float a, double* h) {
 
 // exact sign of det[u, v, w] with u, v, w given as coordinate differences
 // (expansions of length <= 2 each).
-__device__ __noinline__ int exact_det3(const double* u, const int* ul, const double* v, const int* vl,
+static __device__ __noinline__ int exact_det3(const double* u, const int* ul, const double* v, const int* vl,
                                        const double* w, const int* wl) {
     // cofactor c_i = v_j w_k - v_k w_j; det = sum u_i c_i
     double p1[8], p2[8], c[16], t[64], acc[192], acc2[192];
@@ -177,7 +177,7 @@ __device__ __noinline__ int exact_det3(const double* u, const int* ul, const dou
     return alen ? exp_sign(alen, acc) : 0;
 }
 
-__device__ __noinline__ int orient3d_exact(float3 a, float3 b, float3 c, float3 d) {
+static __device__ __noinline__ int orient3d_exact(float3 a, float3 b, float3 c, float3 d) {
     double u[6], v[6], w[6];
     int ul[3], vl[3], wl[3];
     const float A[3] = {a.x, a.y, a.z}, B[3] = {b.x, b.y, b.z}, C[3] = {c.x, c.y, c.z}, D[3] = {d.x, d.y, d.z};
@@ -191,7 +191,7 @@ __device__ __noinline__ int orient3d_exact(float3 a, float3 b, float3 c, float3 
 
 __device__ __forceinline__ float fcomp(float3 p, int k) { return k == 0 ? p.x : (k == 1 ? p.y : p.z); }
 
-__device__ __noinline__ int orient2d_exact(float3 a, float3 b, float3 c, int i, int j) {
+static __device__ __noinline__ int orient2d_exact(float3 a, float3 b, float3 c, int i, int j) {
     double u0[2], u1[2], v0[2], v1[2], p1[8], p2[8], r[16];
     int l_u0 = exp_diff(fcomp(b, i), fcomp(a, i), u0);
     int l_u1 = exp_diff(fcomp(b, j), fcomp(a, j), u1);
@@ -205,7 +205,7 @@ __device__ __noinline__ int orient2d_exact(float3 a, float3 b, float3 c, int i, 
 }
 
 // ------------------------------------------------------------- FP64 stage
-__device__ __noinline__ int orient3d_fp64_or_exact(float3 a, float3 b, float3 c, float3 d, PredCounters& pc) {
+static __device__ __noinline__ int orient3d_fp64_or_exact(float3 a, float3 b, float3 c, float3 d, PredCounters& pc) {
     // two coincident points make the determinant exactly zero
     if ((a.x == b.x && a.y == b.y && a.z == b.z) || (a.x == c.x && a.y == c.y && a.z == c.z) ||
         (a.x == d.x && a.y == d.y && a.z == d.z) || (b.x == c.x && b.y == c.y && b.z == c.z) ||
@@ -226,7 +226,7 @@ __device__ __noinline__ int orient3d_fp64_or_exact(float3 a, float3 b, float3 c,
     return orient3d_exact(a, b, c, d);
 }
 
-__device__ __noinline__ int orient2d_fp64_or_exact(float3 a, float3 b, float3 c, int i, int j, PredCounters& pc) {
+static __device__ __noinline__ int orient2d_fp64_or_exact(float3 a, float3 b, float3 c, int i, int j, PredCounters& pc) {
     const double u0 = (double)fcomp(b, i) - fcomp(a, i), u1 = (double)fcomp(b, j) - fcomp(a, j);
     const double v0 = (double)fcomp(c, i) - fcomp(a, i), v1 = (double)fcomp(c, j) - fcomp(a, j);
     const double det = u0 * v1 - u1 * v0;
@@ -297,7 +297,7 @@ __device__ __forceinline__ bool in_range(float v, float a, float b) { return fmi
 __device__ __forceinline__ bool on_seg_2d(float3 p, float3 q, float3 r, int i, int j) {
     return in_range(fcomp(r, i), fcomp(p, i), fcomp(q, i)) && in_range(fcomp(r, j), fcomp(p, j), fcomp(q, j));
 }
-__device__ __noinline__ bool segs_meet_2d(float3 p, float3 q, float3 u, float3 v, int i, int j, PredCounters& pc) {
+static __device__ __noinline__ bool segs_meet_2d(float3 p, float3 q, float3 u, float3 v, int i, int j, PredCounters& pc) {
     const int d1 = orient2d_robust(p, q, u, i, j, pc), d2 = orient2d_robust(p, q, v, i, j, pc);
     const int d3 = orient2d_robust(u, v, p, i, j, pc), d4 = orient2d_robust(u, v, q, i, j, pc);
     if (d1 * d2 < 0 && d3 * d4 < 0) return true;
@@ -307,12 +307,12 @@ __device__ __noinline__ bool segs_meet_2d(float3 p, float3 q, float3 u, float3 v
     if (d4 == 0 && on_seg_2d(u, v, q, i, j)) return true;
     return false;
 }
-__device__ __noinline__ bool pt_in_tri_2d(float3 p, float3 a, float3 b, float3 c, int o, int i, int j,
+static __device__ __noinline__ bool pt_in_tri_2d(float3 p, float3 a, float3 b, float3 c, int o, int i, int j,
                                           PredCounters& pc) {
     return orient2d_robust(a, b, p, i, j, pc) * o >= 0 && orient2d_robust(b, c, p, i, j, pc) * o >= 0 &&
            orient2d_robust(c, a, p, i, j, pc) * o >= 0;
 }
-__device__ __noinline__ bool seg_tri_coplanar(float3 p, float3 q, float3 a, float3 b, float3 c, PredCounters& pc) {
+static __device__ __noinline__ bool seg_tri_coplanar(float3 p, float3 q, float3 a, float3 b, float3 c, PredCounters& pc) {
     const int nz = orient2d_robust(a, b, c, 0, 1, pc);
     const int nx = orient2d_robust(a, b, c, 1, 2, pc);
     const int ny = orient2d_robust(a, b, c, 2, 0, pc);
