@@ -138,8 +138,9 @@ typedef enum pierce_sizing {
     PIERCE_SIZING_TWO_PASS = 0,   /* count, scan, write, sort + unique */
     PIERCE_SIZING_HASH = 1,       /* hash set sized from expected_pairs */
     PIERCE_SIZING_FIXED = 2,      /* hash set of hash_table_slots slots */
-    PIERCE_SIZING_LEARNED = 3     /* hash set sized by sizing_model's prediction x output_safety;
-                                     two-pass rerun when the pairs do not fit */
+    PIERCE_SIZING_LEARNED = 3     /* hash set sized by sizing_model's prediction x output_safety; pairs past
+                                     the predicted capacity are collected again with their exact count, a
+                                     table that fills up sends the join to the two-pass method */
 } pierce_sizing;
 
 typedef enum pierce_precision {
@@ -243,7 +244,7 @@ typedef struct pierce_stats {
     double predicted_pairs;       /* LEARNED sizing: the network's pair-count prediction */
     double ms_sizing;             /* LEARNED sizing: features + inference */
     int32_t sizing_overflow;      /* LEARNED sizing: 1 when the pairs exceeded the predicted capacity
-                                     and the join was rerun two-pass */
+                                     (collected again, or the join rerun two-pass) */
     int32_t containment_by_pairs; /* containment: 1 when the odd-parity candidate pairs were tested directly
                                      (no per-join hierarchies were built) */
 } pierce_stats;

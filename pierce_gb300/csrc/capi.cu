@@ -15,11 +15,10 @@
 namespace pgpu {
 // join.cu
 int launch_edge_rays(pierce_ctx* ctx, const DevDataset& src, const DevDataset& tgt, int mode, int precision,
-                     int swap, int32_t* counts, const int64_t* offsets, uint64_t* keys, uint64_t* table,
-                     uint64_t slots, const RayOpts* ro);
-int launch_resolve(pierce_ctx* ctx, const DevDataset& src, const DevDataset& tgt, int swap, uint64_t* table,
-                   uint64_t slots, const RayOpts* ro, uint64_t* keys_out, unsigned long long* keys_count,
-                   uint64_t keys_cap);
+                     int swap, int32_t* counts, const int64_t* offsets, uint64_t* keys, const PairSet& set,
+                     const RayOpts* ro);
+int launch_resolve(pierce_ctx* ctx, const DevDataset& src, const DevDataset& tgt, int swap, const PairSet& set,
+                   const RayOpts* ro, uint64_t* keys_out, unsigned long long* keys_count, uint64_t keys_cap);
 int launch_cull(pierce_ctx* ctx, const DevDataset& src, const DevDataset& tgt, uint8_t* active, uint32_t* list,
                 unsigned long long* count);
 int launch_object_active(pierce_ctx* ctx, const DevDataset& src, const DevDataset& tgt, uint8_t* active);
@@ -59,8 +58,7 @@ int keys_to_pairs(pierce_ctx* ctx, uint64_t* keys, int64_t n);
 int pairs_to_keys(pierce_ctx* ctx, const uint64_t* pairs, uint64_t* keys, int64_t n);
 int parity_emit(pierce_ctx* ctx, const uint64_t* ptable, const uint32_t* parity, uint64_t pslots, int mode,
                 const uint64_t* lookup_table, uint64_t lookup_slots, const uint64_t* lookup_sorted, int64_t lookup_n,
-                uint64_t* out_table, uint64_t out_slots, uint64_t* out_keys, unsigned long long* out_count,
-                uint64_t out_cap);
+                const PairSet& out_set, uint64_t* out_keys, unsigned long long* out_count, uint64_t out_cap);
 uint64_t table_slots_for(uint64_t expected, double load_factor);
 int estimate_cells(pierce_ctx* ctx, const void* a, const void* b, int n, float cell_volume, float eps, float gamma,
                    double* total);
@@ -156,6 +154,7 @@ static int join_leaf(const pierce_join_opts& o, const pierce_dataset* ds) {
 // has not used, and the pool's unused memory.  keep_gen 0: free all slots.
 static void release_idle_memory(pierce_ctx* ctx, uint64_t keep_gen) {
     cudaDeviceSynchronize();
+    ctx->set_clean_bytes = 0;
     for (int i = 0; i < kScratchSlots; ++i) {
         if (!ctx->scratch[i] || (keep_gen && ctx->scratch_used[i] == keep_gen)) continue;
         cudaFree(ctx->scratch[i]);
@@ -228,11 +227,23 @@ int result_alloc(pierce_ctx* ctx, void** p, size_t bytes) {
         *p = g->buffers[g->buf_cursor++];
         return PIERCE_OK;
     }
-    if (int s = device_alloc(p, bytes, "result")) return s;
-    if (g && g->mode == 1) {
-        g->buffers.push_back(*p);
-        g->buffer_bytes.push_back(bytes);
+    if (!g) {
+        if (bytes == 0) bytes = 16;
+        cudaError_t e = cudaMallocFromPoolAsync(p, bytes, ctx->pool, ctx->stream);
+        if (e == cudaErrorMemoryAllocation) {
+            cudaGetLastError();
+            release_idle_memory(ctx, ctx->scratch_gen ? ctx->scratch_gen : ~0ull);  // not the running join's slots
+            e = cudaMallocFromPoolAsync(p, bytes, ctx->pool, ctx->stream);
+        }
+        if (e != cudaSuccess) {
+            cudaGetLastError();
+            *p = nullptr;
+        }
+        return check_cuda(e, "result");
     }
+    if (int s = device_alloc(p, bytes, "result")) return s;
+    g->buffers.push_back(*p);
+    g->buffer_bytes.push_back(bytes);
     return PIERCE_OK;
 }
 
@@ -242,6 +253,7 @@ int scratch(pierce_ctx* ctx, int slot, size_t bytes, void** out) {
         return set_error(PIERCE_ERR_CUDA, "join graph capture: scratch would grow");
     ctx->scratch_used[slot] = ctx->scratch_gen;
     if (ctx->scratch_bytes[slot] < bytes) {
+        if (slot == kPairSetSlot) ctx->set_clean_bytes = 0;
         if (ctx->scratch[slot]) {
             cudaStreamSynchronize(ctx->stream);
             cudaFree(ctx->scratch[slot]);
@@ -359,6 +371,9 @@ static int grid_for(pierce_ctx* ctx, int64_t n, int block) {
     return (int)(b < 1 ? 1 : b);
 }
 
+// error word, unique-key count, counters
+constexpr size_t kStateBytes = 16 + sizeof(DevCounters);
+
 static int sync_ctx(pierce_ctx* ctx, const char* what) {
     if (capturing(ctx)) return PIERCE_OK;  // a captured join synchronises after its replay
     return check_cuda(cudaStreamSynchronize(ctx->stream), what);
@@ -375,20 +390,45 @@ static int read_device_error(pierce_ctx* ctx, uint32_t* bits_out) {
     return PIERCE_OK;
 }
 
+// The same with the number of keys in the running join's pair set: one copy
+// and one wait for both.
+static int read_device_state(pierce_ctx* ctx, uint32_t* bits_out, uint64_t* unique_out) {
+    int64_t n = 0;
+    if (ctx->plan) {
+        if (int s = read_device_error(ctx, bits_out)) return s;
+        if (int s = host_value(ctx, ctx->d_unique, 8, &n, "unique pairs")) return s;
+        *unique_out = (uint64_t)n;
+        return PIERCE_OK;
+    }
+    int64_t* h = ctx->h_small + 4;  // error word, unique keys
+    if (int s = check_cuda(cudaMemcpyAsync(h, ctx->d_state, 16, cudaMemcpyDeviceToHost, ctx->stream), "device state"))
+        return s;
+    if (int s = check_cuda(cudaStreamSynchronize(ctx->stream), "device state")) return s;
+    *bits_out = (uint32_t)(h[0] & 0xFFFFFFFF);
+    *unique_out = (uint64_t)h[1];
+    if (*bits_out) cudaMemsetAsync(ctx->d_err, 0, sizeof(uint32_t), ctx->stream);
+    return PIERCE_OK;
+}
+
 struct EventTimer {
-    std::vector<cudaEvent_t> ev;
+    pierce_ctx* ctx;
+    size_t used = 0;  // events of the context's list in use
     std::vector<std::pair<int, int>> spans;  // (begin idx, end idx) per label
     std::vector<double*> targets;
-    cudaStream_t st;
     bool off = false;  // no events inside a captured join
-    explicit EventTimer(cudaStream_t s) : st(s) {}
+    explicit EventTimer(pierce_ctx* c) : ctx(c) {}
     int record() {
         if (off) return -1;
-        cudaEvent_t e;
-        cudaEventCreate(&e);
-        cudaEventRecord(e, st);
-        ev.push_back(e);
-        return (int)ev.size() - 1;
+        if (used == ctx->events.size()) {
+            cudaEvent_t e;
+            if (cudaEventCreate(&e) != cudaSuccess) {
+                cudaGetLastError();
+                return -1;
+            }
+            ctx->events.push_back(e);
+        }
+        cudaEventRecord(ctx->events[used], ctx->stream);
+        return (int)used++;
     }
     void span(int b, int e, double* target) {
         if (off || b < 0 || e < 0) return;
@@ -398,12 +438,9 @@ struct EventTimer {
     void resolve() {
         for (size_t i = 0; i < spans.size(); ++i) {
             float ms = 0.0f;
-            cudaEventElapsedTime(&ms, ev[spans[i].first], ev[spans[i].second]);
+            cudaEventElapsedTime(&ms, ctx->events[spans[i].first], ctx->events[spans[i].second]);
             *targets[i] += ms;
         }
-    }
-    ~EventTimer() {
-        for (auto e : ev) cudaEventDestroy(e);
     }
 };
 
@@ -512,8 +549,12 @@ int pierce_ctx_create(int device, pierce_ctx** out) {
     pierce_ctx* ctx = new pierce_ctx();
     ctx->device = device;
     int st = check_cuda(cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking), "stream create");
-    if (!st) st = device_alloc((void**)&ctx->d_err, sizeof(uint32_t), "error word");
-    if (!st) st = device_alloc((void**)&ctx->d_counters, sizeof(DevCounters), "counters");
+    if (!st) st = device_alloc(&ctx->d_state, kStateBytes, "device state");
+    if (!st) {
+        ctx->d_err = static_cast<uint32_t*>(ctx->d_state);
+        ctx->d_unique = static_cast<unsigned long long*>(ctx->d_state) + 1;
+        ctx->d_counters = reinterpret_cast<DevCounters*>(ctx->d_unique + 1);
+    }
     if (!st) st = check_cuda(cudaMallocHost((void**)&ctx->h_err, sizeof(uint32_t)), "pinned");
     if (!st) st = check_cuda(cudaMallocHost((void**)&ctx->h_counters, sizeof(DevCounters)), "pinned");
     if (!st) st = check_cuda(cudaMallocHost((void**)&ctx->h_small, 8 * sizeof(int64_t)), "pinned");
@@ -543,7 +584,7 @@ int pierce_ctx_create(int device, pierce_ctx** out) {
             st = check_cuda(cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &keep), "pool");
         }
     }
-    if (!st) st = check_cuda(cudaMemsetAsync(ctx->d_err, 0, sizeof(uint32_t), ctx->stream), "memset");
+    if (!st) st = check_cuda(cudaMemsetAsync(ctx->d_state, 0, kStateBytes, ctx->stream), "memset");
     if (!st) st = sync_ctx(ctx, "ctx init");
     if (st) {
         pierce_ctx_destroy(ctx);
@@ -567,8 +608,8 @@ void pierce_ctx_destroy(pierce_ctx* ctx) {
     // arrays of datasets that outlive the context stay valid; the pool's
     // memory is released once they are freed
     if (ctx->pool) cudaMemPoolDestroy(ctx->pool);
-    if (ctx->d_err) cudaFree(ctx->d_err);
-    if (ctx->d_counters) cudaFree(ctx->d_counters);
+    if (ctx->d_state) cudaFree(ctx->d_state);
+    for (cudaEvent_t e : ctx->events) cudaEventDestroy(e);
     if (ctx->h_err) cudaFreeHost(ctx->h_err);
     if (ctx->h_counters) cudaFreeHost(ctx->h_counters);
     if (ctx->h_small) cudaFreeHost(ctx->h_small);
@@ -589,6 +630,7 @@ int pierce_ctx_release_scratch(pierce_ctx* ctx) {
     if (!ctx) return set_error(PIERCE_ERR_INVALID_ARGUMENT, "ctx_release_scratch: null argument");
     cudaSetDevice(ctx->device);
     if (int s = check_cuda(cudaStreamSynchronize(ctx->stream), "release scratch")) return s;
+    ctx->set_clean_bytes = 0;
     for (int i = 0; i < kScratchSlots; ++i) {
         if (ctx->scratch[i]) cudaFree(ctx->scratch[i]);
         ctx->scratch[i] = nullptr;
@@ -920,7 +962,15 @@ int pierce_result_copy(pierce_ctx* ctx, const pierce_result* r, pierce_pair* hos
 
 void pierce_result_destroy(pierce_result* r) {
     if (!r) return;
-    if (r->d_pairs) cudaFree(r->d_pairs);
+    if (r->d_pairs) {
+        // back to the pool once nothing on the device can still read it
+        int dev = r->device;
+        cudaGetDevice(&dev);
+        if (dev != r->device) cudaSetDevice(r->device);
+        cudaDeviceSynchronize();
+        dataset_free(r->d_pairs);
+        if (dev != r->device) cudaSetDevice(dev);
+    }
     delete r;
 }
 
@@ -942,7 +992,7 @@ struct Join {
     EventTimer timer;
     bool ab, ba;
     Join(pierce_ctx* c, pierce_dataset* a, pierce_dataset* b, const pierce_join_opts& opts)
-        : ctx(c), A(a), B(b), o(opts), timer(c->stream) {
+        : ctx(c), A(a), B(b), o(opts), timer(c) {
         ++c->scratch_gen;
         std::memset(&st, 0, sizeof(st));
         timer.off = capturing(c);
@@ -1132,6 +1182,7 @@ struct Join {
         st.containment_pairs = n;
         st.containment_by_pairs = 1;
         pierce_result* r = new pierce_result();
+        r->device = ctx->device;
         r->count = n;
         r->capacity = n;
         r->containment_count = n;
@@ -1140,16 +1191,11 @@ struct Join {
             return s;
         }
         const int tb = timer.record();
-        if (n)
-            if (int s = sort_u64_keys(ctx, ckeys, reinterpret_cast<uint64_t*>(r->d_pairs), (int64_t)n)) {
-                pierce_result_destroy(r);
-                return s;
-            }
-        timer.span(tb, timer.record(), &st.ms_dedup);
-        if (int s = keys_to_pairs(ctx, reinterpret_cast<uint64_t*>(r->d_pairs), (int64_t)n)) {
+        if (int s = sort_pairs(ctx, ckeys, (int64_t)n, A->num_objects, B->num_objects, r->d_pairs)) {
             pierce_result_destroy(r);
             return s;
         }
+        timer.span(tb, timer.record(), &st.ms_dedup);
         *out = r;
         return PIERCE_OK;
     }
@@ -1716,8 +1762,7 @@ struct Join {
     // tests and resolve them right away: into the table (HASH) or into
     // extra_keys (COUNT); WRITE skips them (already resolved by COUNT).
     int edge_rays(int mode, int32_t* counts_ab, int32_t* counts_ba, const int64_t* off_ab, const int64_t* off_ba,
-                  uint64_t* keys, uint64_t* table, uint64_t slots, uint64_t* extra_keys = nullptr,
-                  uint64_t extra_cap = 0) {
+                  uint64_t* keys, const PairSet& set, uint64_t* extra_keys = nullptr, uint64_t extra_cap = 0) {
         const bool dirs[2] = {ab, ba};
         for (int d = 0; d < 2; ++d) {
             if (!dirs[d]) continue;
@@ -1761,19 +1806,62 @@ struct Join {
                 ro.amb_cap = amb_cap;
                 if (mode != 1) cudaMemsetAsync(words + 3, 0, 8, ctx->stream);
             }
-            if (int s = launch_edge_rays(ctx, src, tgt, mode, prec, d, counts, offs, keys, table, slots, &ro))
-                return s;
+            if (int s = launch_edge_rays(ctx, src, tgt, mode, prec, d, counts, offs, keys, set, &ro)) return s;
             if (prec == 2 && mode != 1)
-                if (int s = launch_resolve(ctx, src, tgt, d, mode == 2 ? table : nullptr, slots, &ro, extra_keys,
-                                           words + 4, extra_cap))
+                if (int s = launch_resolve(ctx, src, tgt, d, mode == 2 ? set : PairSet{}, &ro, extra_keys, words + 4,
+                                           extra_cap))
                     return s;
             timer.span(b, timer.record(), &st.ms_edge_rays[d]);
         }
         return PIERCE_OK;
     }
 
-    // Overlap set in a hash table (scratch SLOT_TABLE); returns slots used.
-    int overlap_hash(uint64_t** table_out, uint64_t* slots_out) {
+    // The join's pair set: table in kPairSetSlot, list of its keys in
+    // SLOT_KEYS, sized from the expected count; n_unique once counted.
+    PairSet set_{};
+    uint64_t set_slots = 0;
+    uint64_t n_unique = 0;
+    size_t set_clean = 0;  // leading bytes of the table that were clean before this join used it
+
+    // An empty set of at least `slots` slots.
+    int open_set(uint64_t slots) {
+        uint64_t cap = o.expected_pairs ? (uint64_t)std::ceil((double)o.expected_pairs * std::max(1.0, o.output_safety))
+                                        : (1u << 20);
+        cap = std::max<uint64_t>(std::min<uint64_t>(cap, slots), 1024);
+        void *pt = nullptr, *pk = nullptr;
+        if (int s = scratch(ctx, kPairSetSlot, slots * 8, &pt)) return s;
+        if (int s = scratch(ctx, SLOT_KEYS, cap * 12, &pk)) return s;
+        // a table left clean by the join before it is empty already; a graph's
+        // replays each fill their own
+        set_clean = ctx->plan ? 0 : ctx->set_clean_bytes;
+        if (!ctx->plan) ctx->set_clean_bytes = 0;  // until close_set
+        if (set_clean < slots * 8) {
+            cudaMemsetAsync(pt, 0xFF, slots * 8, ctx->stream);
+            set_clean = slots * 8;
+        }
+        set_ = PairSet{};
+        set_.table = static_cast<uint64_t*>(pt);
+        set_.mask = slots - 1;
+        set_.keys = static_cast<uint64_t*>(pk);
+        set_.slots = reinterpret_cast<uint32_t*>(set_.keys + cap);
+        set_.count = ctx->d_unique;
+        set_.cap = cap;
+        set_slots = slots;
+        st.hash_slots = slots;
+        return check_cuda(cudaMemsetAsync(ctx->d_unique, 0, 8, ctx->stream), "pair set");
+    }
+
+    // Clear the slots the join used (where the list holds them all), so that
+    // the next join finds the table empty.
+    int close_set() {
+        if (!set_.table || ctx->plan || n_unique > set_.cap || set_slots > (1ull << 32)) return PIERCE_OK;
+        if (int s = launch_clear_set(ctx, set_, (int64_t)n_unique)) return s;
+        ctx->set_clean_bytes = set_clean;
+        return PIERCE_OK;
+    }
+
+    // Overlap set in the pair set.
+    int overlap_hash() {
         uint64_t slots;
         if (o.sizing == PIERCE_SIZING_FIXED && o.hash_table_slots > 0) {
             slots = 1;
@@ -1784,20 +1872,17 @@ struct Join {
         }
         while (slots < min_table_slots) slots <<= 1;
         for (int attempt = 0;; ++attempt) {
-            void* p = nullptr;
-            if (int s = scratch(ctx, SLOT_TABLE, slots * 8, &p)) return s;
-            uint64_t* table = static_cast<uint64_t*>(p);
-            cudaMemsetAsync(table, 0xFF, slots * 8, ctx->stream);
+            if (int s = open_set(slots)) return s;
             if (pairs_route) {
                 const int b = timer.record();
                 pj.defer = defer;
-                if (int s = launch_tri_pairs(ctx, va, pj, table, slots)) return s;
+                if (int s = launch_tri_pairs(ctx, va, pj, set_)) return s;
                 timer.span(b, timer.record(), &st.ms_edge_rays[0]);
-            } else if (int s = edge_rays(2, nullptr, nullptr, nullptr, nullptr, nullptr, table, slots)) {
+            } else if (int s = edge_rays(2, nullptr, nullptr, nullptr, nullptr, nullptr, set_)) {
                 return s;
             }
             uint32_t bits = 0;
-            if (int s = read_device_error(ctx, &bits)) return s;
+            if (int s = read_device_state(ctx, &bits, &n_unique)) return s;
             if (bits & ERR_STACK_OVERFLOW) return set_error(PIERCE_ERR_STACK_OVERFLOW, "BVH traversal stack overflow");
             if (bits & ERR_AMBIGUOUS_OVERFLOW) {
                 defer = false;  // too many undecided tests to queue: resolve them inline
@@ -1810,46 +1895,35 @@ struct Join {
                 st.retries++;
                 continue;
             }
-            *table_out = table;
-            *slots_out = slots;
-            st.hash_slots = slots;
             return PIERCE_OK;
         }
     }
 
-    // Occupied slots of a table -> keys in SLOT_KEYS (at offset `base` keys);
-    // the capacity is sized from the expected count and grown on overflow.
-    int compact(const uint64_t* table, uint64_t slots, uint64_t base, uint64_t* n_out, uint64_t** keys_out) {
-        uint64_t cap = o.expected_pairs ? (uint64_t)std::ceil((double)o.expected_pairs * std::max(1.0, o.output_safety))
-                                        : (1u << 20);
-        cap = std::max<uint64_t>(std::min<uint64_t>(cap, slots), 1024);
-        for (int attempt = 0; attempt < 2; ++attempt) {
-            void* p = nullptr;
-            if (int s = scratch(ctx, SLOT_KEYS, (base + cap) * 8, &p)) return s;
-            void* pc = nullptr;
-            if (int s = scratch(ctx, SLOT_AUX, 64, &pc)) return s;
-            unsigned long long* d_count = static_cast<unsigned long long*>(pc);
-            cudaMemsetAsync(d_count, 0, sizeof(unsigned long long), ctx->stream);
-            uint64_t* keys = static_cast<uint64_t*>(p);
-            if (int s = compact_table(ctx, table, slots, keys + base, cap, d_count)) return s;
-            int64_t nv = 0;
-            if (int s = host_value(ctx, d_count, 8, &nv, "compact count")) return s;
-            const uint64_t n = (uint64_t)nv;
-            st.result_capacity = cap;
-            if (n <= cap) {
-                *n_out = n;
-                *keys_out = keys;
-                return PIERCE_OK;
-            }
-            if (strict_capacity) return set_error(PIERCE_ERR_OUTPUT_OVERFLOW, "pairs exceed the predicted capacity");
-            cap = n;  // output overflow: resize to the exact count and compact again
+    // The keys of the pair set (unsorted): its list, or where that proved too
+    // short the table's occupied slots, collected with the exact size.  Under
+    // learned sizing that is an overflow of the prediction.
+    int collect(uint64_t* n_out, uint64_t** keys_out) {
+        st.result_capacity = set_.cap;
+        *n_out = n_unique;
+        *keys_out = set_.keys;
+        if (n_unique <= set_.cap) return PIERCE_OK;
+        if (strict_capacity) {
+            st.sizing_overflow = 1;
+            strict_capacity = false;
+        } else {
             st.retries++;
         }
-        return set_error(PIERCE_ERR_OUTPUT_OVERFLOW, "compaction output overflow");
+        st.result_capacity = n_unique;
+        void* p = nullptr;
+        if (int s = scratch(ctx, SLOT_KEYS, n_unique * 8, &p)) return s;
+        cudaMemsetAsync(ctx->d_unique, 0, 8, ctx->stream);
+        *keys_out = static_cast<uint64_t*>(p);
+        return compact_table(ctx, set_.table, set_slots, *keys_out, n_unique, ctx->d_unique);
     }
 
     // Two-pass overlap: count, scan, write, sort + unique into SLOT_KEYS.
     int overlap_two_pass(uint64_t** keys_out, uint64_t* n_out) {
+        set_ = PairSet{};  // SLOT_KEYS takes the sorted keys: no list of a set remains
         const uint64_t na = ab ? (uint64_t)rays_of(0) : 0, nb = ba ? (uint64_t)rays_of(1) : 0;
         void* pc = nullptr;
         // counts (int32) and offsets (int64) for both directions
@@ -1871,7 +1945,7 @@ struct Join {
             // (the last listed ray differs from run to run, the total does not)
             cudaMemsetAsync(counts + n_all, 0, 4, ctx->stream);
             const size_t span0 = timer.spans.size();
-            if (int s = edge_rays(0, counts, counts + na, nullptr, nullptr, nullptr, nullptr, 0, extra, amb_cap))
+            if (int s = edge_rays(0, counts, counts + na, nullptr, nullptr, nullptr, PairSet{}, extra, amb_cap))
                 return s;
             // the pass-1 (count) spans also feed ms_count_pass
             const size_t span1 = timer.spans.size();
@@ -1908,7 +1982,7 @@ struct Join {
         void* praw = nullptr;
         if (int s = scratch(ctx, SLOT_TABLE, 8 * (size_t)std::max<int64_t>(n_raw, 1), &praw)) return s;
         uint64_t* raw = static_cast<uint64_t*>(praw);
-        if (int s = edge_rays(1, nullptr, nullptr, offs, offs + na, raw, nullptr, 0)) return s;
+        if (int s = edge_rays(1, nullptr, nullptr, offs, offs + na, raw, PairSet{})) return s;
         if (n_extra) cudaMemcpyAsync(raw + total, extra, 8 * n_extra, cudaMemcpyDeviceToDevice, ctx->stream);
         void* pk = nullptr;
         if (int s = scratch(ctx, SLOT_KEYS, 8 * (size_t)std::max<int64_t>(n_raw, 1), &pk)) return s;
@@ -1928,10 +2002,9 @@ struct Join {
     }
 
     // Parity of src first vertices against tgt into the parity table, then
-    // emit odd keys (mode 0: into out_table, mode 1: filtered append).
-    int parity(const DevDataset& src, const DevDataset& tgt, int swap, double* ms, int emit_mode, uint64_t* out_table,
-               uint64_t out_slots, const uint64_t* lookup_table, uint64_t lookup_slots, const uint64_t* lookup_sorted,
-               int64_t lookup_n, uint64_t* out_keys, unsigned long long* out_count, uint64_t out_cap) {
+    // emit odd keys (into out_set, or appended to out_keys).
+    int parity(const DevDataset& src, const DevDataset& tgt, int swap, double* ms, const PairSet& out_set,
+               uint64_t* out_keys, unsigned long long* out_count, uint64_t out_cap) {
         uint64_t pslots = table_slots_for(8 * (uint64_t)std::max(src.num_objects, 1), 0.5);
         for (int attempt = 0;; ++attempt) {
             void* p = nullptr;
@@ -1959,8 +2032,8 @@ struct Join {
                 st.retries++;
                 continue;
             }
-            if (int s = parity_emit(ctx, ptable, par, pslots, emit_mode, lookup_table, lookup_slots, lookup_sorted,
-                                    lookup_n, out_table, out_slots, out_keys, out_count, out_cap))
+            if (int s = parity_emit(ctx, ptable, par, pslots, 0, nullptr, 0, nullptr, 0, out_set, out_keys, out_count,
+                                    out_cap))
                 return s;
             return PIERCE_OK;
         }
@@ -1969,7 +2042,7 @@ struct Join {
     // Parity of both directions into the pair table: both launches, one
     // error check, then both emits.  A full parity table falls back to one
     // direction at a time (each with its own enlarging retries).
-    int parity_both(uint64_t* table, uint64_t slots) {
+    int parity_both(const PairSet& set) {
         const bool need[2] = {ab, ba};
         const int slot_of[2] = {SLOT_BUILD_C, SLOT_BUILD_D};
         uint64_t pslots[2] = {0, 0};
@@ -2004,21 +2077,21 @@ struct Join {
             st.retries++;
             for (int d = 0; d < 2; ++d)
                 if (need[d])
-                    if (int s = parity(d ? vb : va, d ? va : vb, d, &st.ms_parity[d], 0, table, slots, nullptr, 0,
-                                       nullptr, 0, nullptr, nullptr, 0))
+                    if (int s = parity(d ? vb : va, d ? va : vb, d, &st.ms_parity[d], set, nullptr, nullptr, 0))
                         return s;
             return PIERCE_OK;
         }
         for (int d = 0; d < 2; ++d)
             if (need[d])
-                if (int s = parity_emit(ctx, ptable[d], par[d], pslots[d], 0, nullptr, 0, nullptr, 0, table, slots,
-                                        nullptr, nullptr, 0))
+                if (int s = parity_emit(ctx, ptable[d], par[d], pslots[d], 0, nullptr, 0, nullptr, 0, set, nullptr,
+                                        nullptr, 0))
                     return s;
         return PIERCE_OK;
     }
 
     int make_result(const uint64_t* keys_sorted, uint64_t n, pierce_result** out) {
         pierce_result* r = new pierce_result();
+        r->device = ctx->device;
         r->count = n;
         r->capacity = n;
         if (int s = result_alloc(ctx, (void**)&r->d_pairs, std::max<uint64_t>(n, 1) * sizeof(pierce_pair))) {
@@ -2036,15 +2109,24 @@ struct Join {
         return PIERCE_OK;
     }
 
-    // Sort the keys in SLOT_KEYS[0..n) (unsorted, unique) into a result.
-    int sort_into_result(uint64_t* keys, uint64_t n, pierce_result** out) {
-        if (n == 0) return make_result(nullptr, 0, out);
-        void* p = nullptr;
-        if (int s = scratch(ctx, SLOT_BUILD_D, n * 8, &p)) return s;
+    // n different keys (unsorted) into a result.
+    int sort_into_result(const uint64_t* keys, uint64_t n, pierce_result** out) {
+        pierce_result* r = new pierce_result();
+        r->device = ctx->device;
+        r->count = n;
+        r->capacity = n;
+        if (int s = result_alloc(ctx, (void**)&r->d_pairs, std::max<uint64_t>(n, 1) * sizeof(pierce_pair))) {
+            delete r;
+            return s;
+        }
         int tb = timer.record();
-        if (int s = sort_u64_keys(ctx, keys, static_cast<uint64_t*>(p), (int64_t)n)) return s;
+        if (int s = sort_pairs(ctx, keys, (int64_t)n, A->num_objects, B->num_objects, r->d_pairs)) {
+            pierce_result_destroy(r);
+            return s;
+        }
         timer.span(tb, timer.record(), &st.ms_dedup);
-        return make_result(static_cast<uint64_t*>(p), n, out);
+        *out = r;
+        return PIERCE_OK;
     }
 
     // Sort + unique keys[0..n) (may contain duplicates) into a result.
@@ -2060,8 +2142,10 @@ struct Join {
         return make_result(keys, (uint64_t)nu, out);
     }
 
-    // LEARNED sizing: capacity = prediction x output_safety, no enlargement;
-    // pairs that do not fit send the join to the two-pass method.
+    // LEARNED sizing: capacity = prediction x output_safety; a table that
+    // fills up is not enlarged but sends the join to the two-pass method
+    // (pairs past the capacity alone are collected from the table, which
+    // holds them all).
     bool strict_capacity = false;
 
     int run_predicate(pierce_result** out) {
@@ -2071,8 +2155,7 @@ struct Join {
     }
 
     int run(pierce_result** out) {
-        cudaMemsetAsync(ctx->d_counters, 0, sizeof(DevCounters), ctx->stream);
-        cudaMemsetAsync(ctx->d_err, 0, sizeof(uint32_t), ctx->stream);
+        cudaMemsetAsync(ctx->d_state, 0, kStateBytes, ctx->stream);
         const int t0 = timer.record();
         int s = PIERCE_OK;
         if (o.sizing == PIERCE_SIZING_LEARNED) {
@@ -2113,6 +2196,7 @@ struct Join {
             }
             s = run_predicate(out);
         }
+        if (!s) s = close_set();
         const int t1 = timer.record();
         timer.span(t0, t1, &st.ms_total);
         if (s) return s;
@@ -2141,12 +2225,11 @@ struct Join {
             if (int s = overlap_two_pass(&keys, &n)) return s;
             return make_result(keys, n, out);
         }
-        uint64_t* table = nullptr;
-        uint64_t slots = 0, n = 0;
-        if (int s = overlap_hash(&table, &slots)) return s;
+        uint64_t n = 0;
+        if (int s = overlap_hash()) return s;
         uint64_t* keys = nullptr;
         int tb = timer.record();
-        if (int s = compact(table, slots, 0, &n, &keys)) return s;
+        if (int s = collect(&n, &keys)) return s;
         timer.span(tb, timer.record(), &st.ms_dedup);
         return sort_into_result(keys, n, out);
     }
@@ -2169,36 +2252,31 @@ struct Join {
             cudaMemsetAsync(d_count, 0, 8, ctx->stream);
             const uint64_t cap = 8 * extra + 16;
             if (ab)
-                if (int s = parity(va, vb, 0, &st.ms_parity[0], 0, nullptr, 0, nullptr, 0, nullptr, 0, all + n_over,
-                                   d_count, cap))
-                    return s;
+                if (int s = parity(va, vb, 0, &st.ms_parity[0], PairSet{}, all + n_over, d_count, cap)) return s;
             if (ba)
-                if (int s = parity(vb, va, 1, &st.ms_parity[1], 0, nullptr, 0, nullptr, 0, nullptr, 0, all + n_over,
-                                   d_count, cap))
-                    return s;
+                if (int s = parity(vb, va, 1, &st.ms_parity[1], PairSet{}, all + n_over, d_count, cap)) return s;
             int64_t n_par_v = 0;
             if (int s = host_value(ctx, d_count, 8, &n_par_v, "parity count")) return s;
             const uint64_t n_par = (uint64_t)n_par_v;
             if (n_par > cap) return set_error(PIERCE_ERR_OUTPUT_OVERFLOW, "parity output overflow");
             return sort_unique_into_result(all, n_over + n_par, out);
         }
-        uint64_t* table = nullptr;
-        uint64_t slots = 0, n = 0;
+        uint64_t n = 0;
         for (int attempt = 0;; ++attempt) {
-            if (int s = overlap_hash(&table, &slots)) return s;
-            if (int s = parity_both(table, slots)) return s;
+            if (int s = overlap_hash()) return s;
+            if (int s = parity_both(set_)) return s;
             uint32_t bits = 0;
-            if (int s = read_device_error(ctx, &bits)) return s;
+            if (int s = read_device_state(ctx, &bits, &n_unique)) return s;
             if (!(bits & ERR_HASH_FULL)) break;
             // the parity pairs did not fit: a larger table, overlap and parity again
             if (attempt >= o.max_retries)
                 return set_error(PIERCE_ERR_HASH_FULL, "pair table full while adding parity pairs");
-            min_table_slots = 4 * slots;
+            min_table_slots = 4 * set_slots;
             st.retries++;
         }
         uint64_t* keys = nullptr;
         int tb = timer.record();
-        if (int s = compact(table, slots, 0, &n, &keys)) return s;
+        if (int s = collect(&n, &keys)) return s;
         timer.span(tb, timer.record(), &st.ms_dedup);
         return sort_into_result(keys, n, out);
     }
@@ -2215,15 +2293,13 @@ struct Join {
         // parity of B's first vertices against A, filtered by the overlap set.
         const bool save_ab = ab, save_ba = ba;
         ab = ba = true;
-        uint64_t* table = nullptr;
-        uint64_t slots = 0;
         uint64_t* okeys = nullptr;
         uint64_t n_over = 0;
         const bool two_pass = o.sizing == PIERCE_SIZING_TWO_PASS;
         if (two_pass) {
             if (int s = overlap_two_pass(&okeys, &n_over)) return s;
         } else {
-            if (int s = overlap_hash(&table, &slots)) return s;
+            if (int s = overlap_hash()) return s;
         }
         ab = save_ab;
         ba = save_ba;
@@ -2243,8 +2319,8 @@ struct Join {
             if (int s = scratch(ctx, SLOT_AUX, 64, &pc)) return s;
             unsigned long long* d_count = static_cast<unsigned long long*>(pc);
             cudaMemsetAsync(d_count, 0, 8, ctx->stream);
-            if (int s = parity_emit(ctx, cont_ptable, cont_par, cont_pslots, 1, table, slots, okeys, (int64_t)n_over,
-                                    nullptr, 0, ckeys, d_count, cap))
+            if (int s = parity_emit(ctx, cont_ptable, cont_par, cont_pslots, 1, two_pass ? nullptr : set_.table,
+                                    two_pass ? 0 : set_slots, okeys, (int64_t)n_over, PairSet{}, ckeys, d_count, cap))
                 return s;
             int64_t n_cont_v = 0;
             if (int s = host_value(ctx, d_count, 8, &n_cont_v, "containment count")) return s;
@@ -2256,7 +2332,7 @@ struct Join {
         if (!two_pass && o.include_overlap_pairs) {
             // overlap keys of the table after the containment keys
             uint64_t* keys = nullptr;
-            if (int s = compact(table, slots, 0, &n_over, &keys)) return s;
+            if (int s = collect(&n_over, &keys)) return s;
             okeys = keys;
         }
         st.containment_pairs = n_cont;
@@ -2264,6 +2340,7 @@ struct Join {
         // sort containment keys (into the front of a combined buffer)
         const uint64_t n_total = n_cont + (o.include_overlap_pairs ? n_over : 0);
         pierce_result* r = new pierce_result();
+        r->device = ctx->device;
         r->count = n_total;
         r->capacity = n_total;
         r->containment_count = n_cont;
@@ -2271,26 +2348,26 @@ struct Join {
             delete r;
             return s;
         }
-        uint64_t* rk = reinterpret_cast<uint64_t*>(r->d_pairs);
         int tb = timer.record();
-        if (n_cont)
-            if (int s = sort_u64_keys(ctx, ckeys, rk, (int64_t)n_cont)) {
-                pierce_result_destroy(r);
-                return s;
-            }
+        if (int s = sort_pairs(ctx, ckeys, (int64_t)n_cont, A->num_objects, B->num_objects, r->d_pairs)) {
+            pierce_result_destroy(r);
+            return s;
+        }
         if (o.include_overlap_pairs && n_over) {
             if (two_pass) {
-                cudaMemcpyAsync(rk + n_cont, okeys, n_over * 8, cudaMemcpyDeviceToDevice, ctx->stream);
-            } else if (int s = sort_u64_keys(ctx, okeys, rk + n_cont, (int64_t)n_over)) {
+                uint64_t* rk = reinterpret_cast<uint64_t*>(r->d_pairs) + n_cont;
+                cudaMemcpyAsync(rk, okeys, n_over * 8, cudaMemcpyDeviceToDevice, ctx->stream);
+                if (int s = keys_to_pairs(ctx, rk, (int64_t)n_over)) {
+                    pierce_result_destroy(r);
+                    return s;
+                }
+            } else if (int s = sort_pairs(ctx, okeys, (int64_t)n_over, A->num_objects, B->num_objects,
+                                          r->d_pairs + n_cont)) {
                 pierce_result_destroy(r);
                 return s;
             }
         }
         timer.span(tb, timer.record(), &st.ms_dedup);
-        if (int s = keys_to_pairs(ctx, rk, (int64_t)n_total)) {
-            pierce_result_destroy(r);
-            return s;
-        }
         *out = r;
         return PIERCE_OK;
     }
@@ -2461,6 +2538,7 @@ void free_graph(pierce_join_graph* g) {
     if (g->graph) cudaGraphDestroy(g->graph);
     for (void* p : g->plan.buffers)
         if (p) cudaFree(p);
+    if (g->ctx) g->ctx->set_clean_bytes = 0;  // the table may be the graph's from here on
     for (int i = 0; i < kScratchSlots; ++i) {
         if (!g->scratch[i]) continue;
         if (g->ctx && g->ctx->scratch_bytes[i] < g->scratch_bytes[i]) {
@@ -2520,6 +2598,7 @@ int pierce_join_graph_create(pierce_ctx* ctx, pierce_dataset* a, pierce_dataset*
         ctx->scratch[i] = nullptr;
         ctx->scratch_bytes[i] = 0;
     }
+    ctx->set_clean_bytes = 0;
     // 1. the planning run: an ordinary join that records its host decisions
     int s = with_graph_scratch(ctx, g, [&]() {
         g->plan.mode = 1;
@@ -2600,7 +2679,13 @@ int pierce_join_graph_launch(pierce_ctx* ctx, pierce_join_graph* g, pierce_stats
     cudaEventDestroy(e1);
     if (s) return s;
     ctx->launches += (uint64_t)g->launches;
-    // the replay must have met every decision of the plan
+    // the replay must have met every decision of the plan (a replay that did
+    // not may leave error bits behind)
+    auto differs = [&]() {
+        cudaMemset(ctx->d_err, 0, sizeof(uint32_t));
+        return set_error(PIERCE_ERR_OUTPUT_OVERFLOW,
+                         "join graph replay: a data-dependent size differs from the plan (inputs changed?)");
+    };
     for (size_t i = 0; i < p.values.size(); ++i) {
         int64_t v = p.h_check[i];
         if (p.widths[i] == 4) {
@@ -2608,9 +2693,7 @@ int pierce_join_graph_launch(pierce_ctx* ctx, pierce_join_graph* g, pierce_stats
             std::memcpy(&w, &p.h_check[i], 4);
             v = w;
         }
-        if (v != p.values[i])
-            return set_error(PIERCE_ERR_OUTPUT_OVERFLOW,
-                             "join graph replay: a data-dependent size differs from the plan (inputs changed?)");
+        if (v != p.values[i]) return differs();
     }
     cudaMemcpy(ctx->h_err, ctx->d_err, sizeof(uint32_t), cudaMemcpyDeviceToHost);
     if (*ctx->h_err) {
@@ -2678,8 +2761,11 @@ int pierce_launch_edge_rays(pierce_ctx* ctx, const pierce_dataset* src, const pi
         return set_error(PIERCE_ERR_INVALID_ARGUMENT, "HASH needs a power-of-two table");
     cudaSetDevice(ctx->device);
     cudaMemsetAsync(ctx->d_counters, 0, sizeof(DevCounters), ctx->stream);
-    if (int s = launch_edge_rays(ctx, src->view(), tgt->view(), mode, precision, swap, d_counts, d_offsets, d_keys,
-                                 d_table, table_slots, nullptr))
+    PairSet set;
+    set.table = d_table;
+    set.mask = table_slots ? table_slots - 1 : 0;
+    if (int s = launch_edge_rays(ctx, src->view(), tgt->view(), mode, precision, swap, d_counts, d_offsets, d_keys, set,
+                                 nullptr))
         return s;
     uint32_t bits = 0;
     if (int s = read_device_error(ctx, &bits)) return s;

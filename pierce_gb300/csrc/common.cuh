@@ -98,6 +98,18 @@ struct DevDataset {
     int soup_boxes;     // the soup holds boxes as degenerate triangles (lo, hi, hi), not triangles
 };
 
+// Open-addressing set of pair keys (a power of two of slots, empty slot all
+// ones) with an optional list of the keys in it: keys and slots hold the
+// first cap of them, *count all.
+struct PairSet {
+    uint64_t* table = nullptr;
+    uint64_t mask = 0;
+    uint64_t* keys = nullptr;
+    uint32_t* slots = nullptr;
+    unsigned long long* count = nullptr;
+    uint64_t cap = 0;
+};
+
 // Optional inputs of an edge-ray launch: a compacted ray list (object
 // culling) and the queue of deferred exact tests.
 struct RayOpts {
@@ -122,7 +134,8 @@ struct RayOpts {
     int entry_group = 1;
 };
 
-constexpr int kScratchSlots = 40;
+constexpr int kScratchSlots = 44;
+constexpr int kPairSetSlot = 40;  // the joins' pair table
 
 // Uniform xy grid over a dataset's object boxes: per cell the objects whose
 // box covers the cell in x and y (parity candidates).
@@ -192,7 +205,10 @@ struct GraphPlan {
 struct pierce_ctx {
     int device = 0;
     cudaStream_t stream = nullptr;
+    // one block: error word, unique-key count, counters (cleared together)
+    void* d_state = nullptr;
     uint32_t* d_err = nullptr;
+    unsigned long long* d_unique = nullptr;    // keys in the running join's pair set
     pgpu::DevCounters* d_counters = nullptr;
     uint32_t* h_err = nullptr;                 // pinned
     pgpu::DevCounters* h_counters = nullptr;   // pinned
@@ -204,6 +220,10 @@ struct pierce_ctx {
     // short of memory frees the slots it has not touched
     uint64_t scratch_gen = 0;
     uint64_t scratch_used[pgpu::kScratchSlots] = {0};
+    // leading bytes of scratch[kPairSetSlot] known to hold empty slots: a join
+    // clears the slots it used, so the next one need not fill the table
+    size_t set_clean_bytes = 0;
+    std::vector<cudaEvent_t> events;           // timing events, reused by every join
     uint64_t launches = 0;
     int sm_count = 0;
     pgpu::GraphPlan* plan = nullptr;  // set while a join graph is planned or captured
@@ -295,7 +315,8 @@ struct pierce_dataset {
 };
 
 struct pierce_result {
-    pierce_pair* d_pairs = nullptr;
+    pierce_pair* d_pairs = nullptr;  // from the context's pool
+    int device = 0;
     uint64_t count = 0;
     uint64_t capacity = 0;
     uint64_t containment_count = 0;
@@ -371,12 +392,16 @@ int launch_pair_rays(pierce_ctx* ctx, const float4* asoup, int64_t na, const uin
                      const unsigned long long* b_count, int64_t b_bound, int G);
 int launch_unit_incidences(pierce_ctx* ctx, const DevDataset& a, const PairJoin& j, int step,
                            unsigned long long* count);
-int launch_tri_pairs(pierce_ctx* ctx, const DevDataset& a, const PairJoin& j, uint64_t* table, uint64_t slots);
+int launch_tri_pairs(pierce_ctx* ctx, const DevDataset& a, const PairJoin& j, const PairSet& set);
+// n different pair keys (any order) -> pairs sorted by (a, b); object ids
+// below num_a, num_b
+int sort_pairs(pierce_ctx* ctx, const uint64_t* keys, int64_t n, int32_t num_a, int32_t num_b, pierce_pair* out);
+int launch_clear_set(pierce_ctx* ctx, const PairSet& set, int64_t n);
 
 // sortscan.cu (CUB library calls)
 int sort_u32_pairs(pierce_ctx* ctx, uint32_t* keys_in, uint32_t* keys_out, uint32_t* vals_in, uint32_t* vals_out,
                    int64_t n, int end_bit);
-int sort_u64_keys(pierce_ctx* ctx, uint64_t* keys_in, uint64_t* keys_out, int64_t n);
+int sort_u64_keys(pierce_ctx* ctx, const uint64_t* keys_in, uint64_t* keys_out, int64_t n, int end_bit = 64);
 int sort_u64_pairs(pierce_ctx* ctx, uint64_t* keys_in, uint64_t* keys_out, uint32_t* vals_in, uint32_t* vals_out,
                    int64_t n, int end_bit);
 int exclusive_scan_i32_to_i64(pierce_ctx* ctx, const int32_t* in, int64_t* out, int64_t n);

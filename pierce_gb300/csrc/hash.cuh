@@ -42,6 +42,38 @@ __device__ __forceinline__ int64_t hash_insert(uint64_t* table, uint64_t mask, u
     return -1;
 }
 
+// Insert into a pair set; the key's first insertion also appends it, with its
+// slot, to the set's list (keys null: no list).  A join's pairs are few beside
+// its table's slots, so the list replaces a pass over the whole table that
+// collects them, and clearing the listed slots replaces filling the table
+// again (128 MB at the default size: 35 + 20 us of a 490 us join).
+__device__ __forceinline__ void hash_add(const PairSet& S, uint64_t key, uint32_t* err, uint32_t& probes) {
+    uint64_t h = fmix64(key) & S.mask;
+    for (uint64_t i = 0; i <= S.mask; ++i) {
+        ++probes;
+        const uint64_t cur = __ldcg(S.table + h);
+        if (cur == key) return;
+        if (cur == kEmptyKey) {
+            const unsigned long long old =
+                atomicCAS(reinterpret_cast<unsigned long long*>(S.table + h), (unsigned long long)kEmptyKey,
+                          (unsigned long long)key);
+            if (old == key) return;
+            if (old == kEmptyKey) {
+                if (S.keys) {
+                    const unsigned long long pos = atomicAdd(S.count, 1ull);
+                    if (pos < S.cap) {
+                        S.keys[pos] = key;
+                        S.slots[pos] = (uint32_t)h;
+                    }
+                }
+                return;
+            }
+        }
+        h = (h + 1) & S.mask;
+    }
+    atomicOr(err, ERR_HASH_FULL);
+}
+
 // Warp-aggregated counter flush: one atomicAdd per warp.
 __device__ __forceinline__ void flush_counter(unsigned long long* dst, unsigned long long v) {
     for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xFFFFFFFFu, v, off);

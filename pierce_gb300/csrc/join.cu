@@ -74,8 +74,7 @@ struct EdgeRayParams {
     int32_t* counts;
     const int64_t* offsets;
     uint64_t* keys;
-    uint64_t* table;
-    uint64_t mask;
+    PairSet set;
     uint32_t* err;
     DevCounters* ctr;
     // optional compacted list of edges to trace (object culling)
@@ -261,7 +260,7 @@ __device__ __forceinline__ void leaf_tests(const EdgeRayParams& P, int64_t e, in
             P.keys[out++] = key;
         } else {
             ++rc.inserts;
-            hash_insert(P.table, P.mask, key, P.err, rc.probes);
+            hash_add(P.set, key, P.err, rc.probes);
         }
     }
 }
@@ -568,9 +567,9 @@ __global__ void __launch_bounds__(128) k_resolve_ambiguous(EdgeRayParams P, uint
             continue;
         const int32_t obj = __float_as_int(a4.w);
         const uint64_t key = P.swap ? pack_key(obj, src_obj) : pack_key(src_obj, obj);
-        if (P.table) {
+        if (P.set.table) {
             ++inserts;
-            hash_insert(P.table, P.mask, key, P.err, probes);
+            hash_add(P.set, key, P.err, probes);
         } else {
             const unsigned long long pos = atomicAdd(keys_count, 1ull);
             if (pos < keys_cap) keys_out[pos] = key;
@@ -809,8 +808,7 @@ __global__ void __launch_bounds__(128) k_parity(ParityParams P) {
 // table or sorted array) and append them to out_keys.
 __global__ void k_parity_emit(const uint64_t* __restrict__ ptable, const uint32_t* __restrict__ parity, uint64_t pslots,
                               int mode, const uint64_t* lookup_table, uint64_t lookup_mask,
-                              const uint64_t* lookup_sorted, int64_t lookup_n, uint64_t* out_table, uint64_t out_mask,
-                              uint64_t* out_keys, unsigned long long* out_count, uint64_t out_cap, uint32_t* err) {
+                              const uint64_t* lookup_sorted, int64_t lookup_n, PairSet out_set, uint64_t* out_keys, unsigned long long* out_count, uint64_t out_cap, uint32_t* err) {
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < pslots; i += (uint64_t)gridDim.x * blockDim.x) {
         const uint64_t key = ptable[i];
         if (key == kEmptyKey || !(parity[i] & 1u)) continue;
@@ -819,9 +817,9 @@ __global__ void k_parity_emit(const uint64_t* __restrict__ ptable, const uint32_
                                          : sorted_contains(lookup_sorted, lookup_n, key);
             if (in) continue;
         }
-        if (out_table) {
+        if (out_set.table) {
             uint32_t probes = 0;
-            hash_insert(out_table, out_mask, key, err, probes);
+            hash_add(out_set, key, err, probes);
         } else {
             const unsigned long long pos = atomicAdd(out_count, 1ull);
             if (pos < out_cap) out_keys[pos] = key;
@@ -1154,8 +1152,8 @@ static uint64_t next_pow2(uint64_t v) {
 }
 
 int launch_edge_rays(pierce_ctx* ctx, const DevDataset& src, const DevDataset& tgt, int mode, int precision,
-                     int swap, int32_t* counts, const int64_t* offsets, uint64_t* keys, uint64_t* table,
-                     uint64_t slots, const RayOpts* ro) {
+                     int swap, int32_t* counts, const int64_t* offsets, uint64_t* keys, const PairSet& set,
+                     const RayOpts* ro) {
     const int64_t n_rays = (ro && ro->list && ro->bound >= 0) ? ro->bound : src.num_edges;
     if (n_rays == 0) return PIERCE_OK;
     EdgeRayParams P;
@@ -1165,8 +1163,7 @@ int launch_edge_rays(pierce_ctx* ctx, const DevDataset& src, const DevDataset& t
     P.counts = counts;
     P.offsets = offsets;
     P.keys = keys;
-    P.table = table;
-    P.mask = slots ? slots - 1 : 0;
+    P.set = set;
     P.err = ctx->d_err;
     P.ctr = ctx->d_counters;
     P.ray_list = ro ? ro->list : nullptr;
@@ -1228,16 +1225,13 @@ int launch_edge_rays(pierce_ctx* ctx, const DevDataset& src, const DevDataset& t
     return check_cuda(cudaGetLastError(), "edge ray kernel");
 }
 
-int launch_resolve(pierce_ctx* ctx, const DevDataset& src, const DevDataset& tgt, int swap, uint64_t* table,
-                   uint64_t slots, const RayOpts* ro, uint64_t* keys_out, unsigned long long* keys_count,
-                   uint64_t keys_cap) {
-    EdgeRayParams P;
-    std::memset(&P, 0, sizeof(P));
+int launch_resolve(pierce_ctx* ctx, const DevDataset& src, const DevDataset& tgt, int swap, const PairSet& set,
+                   const RayOpts* ro, uint64_t* keys_out, unsigned long long* keys_count, uint64_t keys_cap) {
+    EdgeRayParams P{};
     P.src = src;
     P.tgt = tgt;
     P.swap = swap;
-    P.table = table;
-    P.mask = slots ? slots - 1 : 0;
+    P.set = set;
     P.err = ctx->d_err;
     P.ctr = ctx->d_counters;
     P.amb_queue = ro->amb_queue;
@@ -2423,11 +2417,10 @@ int pairs_to_keys(pierce_ctx* ctx, const uint64_t* pairs, uint64_t* keys, int64_
 
 int parity_emit(pierce_ctx* ctx, const uint64_t* ptable, const uint32_t* parity, uint64_t pslots, int mode,
                 const uint64_t* lookup_table, uint64_t lookup_slots, const uint64_t* lookup_sorted, int64_t lookup_n,
-                uint64_t* out_table, uint64_t out_slots, uint64_t* out_keys, unsigned long long* out_count,
-                uint64_t out_cap) {
+                const PairSet& out_set, uint64_t* out_keys, unsigned long long* out_count, uint64_t out_cap) {
     k_parity_emit<<<grid_cap(ctx, (int64_t)pslots, 256), 256, 0, ctx->stream>>>(
         ptable, parity, pslots, mode, lookup_table, lookup_slots ? lookup_slots - 1 : 0, lookup_sorted, lookup_n,
-        out_table, out_slots ? out_slots - 1 : 0, out_keys, out_count, out_cap, ctx->d_err);
+        out_set, out_keys, out_count, out_cap, ctx->d_err);
     ctx->launches += 1;
     return check_cuda(cudaGetLastError(), "parity emit");
 }

@@ -45,8 +45,7 @@ struct PairParams {
     const uint32_t* glist;                // ... and the kept ones among them
     const int32_t* b_part;                // partition per B object (partitioned joins)
     int G;                                // triangles per group, both sides
-    uint64_t* table;
-    uint64_t mask;
+    PairSet set;
     uint32_t* err;
     DevCounters* ctr;
     unsigned long long* cursor;
@@ -216,7 +215,7 @@ __global__ void __launch_bounds__(32 * kPairWarps, DEFER ? 6 : 4) k_tri_pairs(Pa
                 }
                 if (hit) {
                     ++hits;
-                    hash_insert(P.table, P.mask, pack_key(__float_as_int(a0.w), __float_as_int(b0.w)), P.err, probes);
+                    hash_add(P.set, pack_key(__float_as_int(a0.w), __float_as_int(b0.w)), P.err, probes);
                 }
             }
             __syncwarp();
@@ -422,14 +421,14 @@ __global__ void __launch_bounds__(128) k_resolve_pairs(PairParams P) {
                            pc))
             continue;
         ++hits;
-        hash_insert(P.table, P.mask, pack_key(__float_as_int(a0.w), __float_as_int(b0.w)), P.err, probes);
+        hash_add(P.set, pack_key(__float_as_int(a0.w), __float_as_int(b0.w)), P.err, probes);
     }
     flush_counter(&P.ctr->fp64_ambiguous, pc.fp64_ambiguous);
     flush_counter(&P.ctr->hash_accesses, probes);
     flush_counter(&P.ctr->hash_contentions, probes - hits);
 }
 
-int launch_tri_pairs(pierce_ctx* ctx, const DevDataset& a, const PairJoin& j, uint64_t* table, uint64_t slots) {
+int launch_tri_pairs(pierce_ctx* ctx, const DevDataset& a, const PairJoin& j, const PairSet& set) {
     cudaStream_t st = ctx->stream;
     const int64_t na = a.num_tris / j.G;
     // words of j.work: [0] deferred tests, then per round [1 + 2 r] cursor, [2 + 2 r] spilled entries
@@ -437,8 +436,7 @@ int launch_tri_pairs(pierce_ctx* ctx, const DevDataset& a, const PairJoin& j, ui
     constexpr int kBudget = 192;
     cudaMemsetAsync(j.work, 0, (1 + 2 * kRounds) * sizeof(unsigned long long), st);
     cudaMemsetAsync(j.a_listed, 0, (size_t)na, st);
-    PairParams P;
-    std::memset(&P, 0, sizeof(P));
+    PairParams P{};
     P.a = a;
     P.bsoup = j.bsoup;
     P.b_count = j.b_count;
@@ -446,8 +444,7 @@ int launch_tri_pairs(pierce_ctx* ctx, const DevDataset& a, const PairJoin& j, ui
     P.glist = j.units.glist;
     P.b_part = j.b_part;
     P.G = j.G;
-    P.table = table;
-    P.mask = slots - 1;
+    P.set = set;
     P.err = ctx->d_err;
     P.ctr = ctx->d_counters;
     P.amb_queue = j.amb_queue;
@@ -601,8 +598,7 @@ int launch_unit_incidences(pierce_ctx* ctx, const DevDataset& a, const PairJoin&
                            unsigned long long* count) {
     cudaMemsetAsync(count, 0, sizeof(unsigned long long), ctx->stream);
     if (j.units.bound <= 0) return check_cuda(cudaGetLastError(), "unit incidences");
-    PairParams P;
-    std::memset(&P, 0, sizeof(P));
+    PairParams P{};
     P.a = a;
     P.bsoup = j.bsoup;
     P.b_count = j.b_count;
@@ -616,6 +612,94 @@ int launch_unit_incidences(pierce_ctx* ctx, const DevDataset& a, const PairJoin&
     k_unit_incidences<<<(unsigned)blocks, 32 * kPairWarps, 0, ctx->stream>>>(P, step, min_runs, count);
     ctx->launches += 1;
     return check_cuda(cudaGetLastError(), "unit incidences");
+}
+
+// ---- pair output ---------------------------------------------------------------
+
+// The listed slots of a set back to empty.
+__global__ void __launch_bounds__(256) k_clear_set(PairSet set, int64_t n) {
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+        set.table[set.slots[i]] = kEmptyKey;
+}
+
+int launch_clear_set(pierce_ctx* ctx, const PairSet& set, int64_t n) {
+    if (n <= 0) return PIERCE_OK;
+    k_clear_set<<<(unsigned)std::min<int64_t>((n + 255) / 256, (int64_t)ctx->sm_count * 16), 256, 0, ctx->stream>>>(set, n);
+    ctx->launches += 1;
+    return check_cuda(cudaGetLastError(), "clear pair set");
+}
+
+__device__ __forceinline__ unsigned long long key_to_pair(unsigned long long k) { return (k >> 32) | (k << 32); }
+
+// Different keys -> sorted pairs, each key placed at its rank (the number of
+// smaller keys): a block ranks 32 keys, one per lane, and each of its warps
+// counts over its share of every tile (a broadcast load per key compared).
+constexpr int kRankWarps = 32, kRankTile = 2048;
+constexpr int64_t kRankMax = 1 << 14;
+__global__ void __launch_bounds__(32 * kRankWarps) k_rank_pairs(const uint64_t* __restrict__ keys, int n,
+                                                                unsigned long long* __restrict__ out) {
+    __shared__ uint64_t tile[kRankTile];
+    __shared__ int part[kRankWarps][32];
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const int i = blockIdx.x * 32 + lane;
+    const uint64_t key = i < n ? keys[i] : 0;
+    int rank = 0;
+    for (int base = 0; base < n; base += kRankTile) {
+        const int m = min(n - base, kRankTile);
+        for (int j = tid; j < kRankTile; j += 32 * kRankWarps) tile[j] = j < m ? keys[base + j] : kEmptyKey;
+        __syncthreads();
+        constexpr int kPer = kRankTile / kRankWarps;
+#pragma unroll 16
+        for (int j = 0; j < kPer; ++j) rank += tile[w * kPer + j] < key ? 1 : 0;
+        __syncthreads();
+    }
+    part[w][lane] = rank;
+    __syncthreads();
+    if (w == 0 && i < n) {
+        for (int q = 1; q < kRankWarps; ++q) rank += part[q][lane];
+        out[rank] = key_to_pair(key);
+    }
+}
+
+// a << 32 | b <-> a << bits_b | b
+__global__ void k_pack_keys(const uint64_t* __restrict__ in, uint64_t* __restrict__ out, int64_t n, int bits_b) {
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+        out[i] = ((in[i] >> 32) << bits_b) | (uint32_t)in[i];
+}
+__global__ void k_unpack_pairs(const uint64_t* __restrict__ in, unsigned long long* __restrict__ out, int64_t n,
+                               int bits_b) {
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+        out[i] = (in[i] >> bits_b) | ((in[i] & ((1ull << bits_b) - 1)) << 32);
+}
+
+// Up to kRankMax keys: one launch that compares every key with every other
+// (2.7e8 comparisons at 2^14 keys; 13,247 keys: 35 us).  A radix sort of so
+// few keys is ten launches of 5-10 us each (the same keys, 64 bits: 95 us,
+// then 4 us to make the pairs).  More keys: radix sort over the ids' bits
+// only (167,599 keys of 28 bits: half the passes of 64).
+int sort_pairs(pierce_ctx* ctx, const uint64_t* keys, int64_t n, int32_t num_a, int32_t num_b, pierce_pair* out) {
+    if (n <= 0) return PIERCE_OK;
+    unsigned long long* o = reinterpret_cast<unsigned long long*>(out);
+    if (n <= kRankMax) {
+        k_rank_pairs<<<(unsigned)((n + 31) / 32), 32 * kRankWarps, 0, ctx->stream>>>(keys, (int)n, o);
+        ctx->launches += 1;
+        return check_cuda(cudaGetLastError(), "rank pairs");
+    }
+    auto bits = [](int32_t v) {
+        int b = 1;
+        while (b < 31 && (1ll << b) < (int64_t)v) ++b;
+        return b;
+    };
+    const int ba = bits(num_a), bb = bits(num_b);
+    void* p = nullptr;
+    if (int s = scratch(ctx, 2, 16 * (size_t)n, &p)) return s;
+    uint64_t* packed = static_cast<uint64_t*>(p);
+    const unsigned grid = (unsigned)std::min<int64_t>((n + 255) / 256, (int64_t)ctx->sm_count * 16);
+    k_pack_keys<<<grid, 256, 0, ctx->stream>>>(keys, packed, n, bb);
+    if (int s = sort_u64_keys(ctx, packed, packed + n, n, ba + bb)) return s;
+    k_unpack_pairs<<<grid, 256, 0, ctx->stream>>>(packed + n, o, n, bb);
+    ctx->launches += 2;
+    return check_cuda(cudaGetLastError(), "sort pairs");
 }
 
 }  // namespace pgpu
