@@ -21,7 +21,8 @@ int launch_resolve(pierce_ctx* ctx, const DevDataset& src, const DevDataset& tgt
                    const RayOpts* ro, uint64_t* keys_out, unsigned long long* keys_count, uint64_t keys_cap);
 int launch_cull(pierce_ctx* ctx, const DevDataset& src, const DevDataset& tgt, uint8_t* active, uint32_t* list,
                 unsigned long long* count);
-int launch_object_active(pierce_ctx* ctx, const DevDataset& src, const DevDataset& tgt, uint8_t* active);
+int launch_object_active(pierce_ctx* ctx, const DevDataset& a, const DevDataset& tgt_a, uint8_t* active_a,
+                         const DevDataset& b, const DevDataset& tgt_b, uint8_t* active_b);
 int launch_collect_rays(pierce_ctx* ctx, const DevDataset& src, const uint8_t* active, uint32_t* list,
                         unsigned long long* count);
 int launch_collect_tris(pierce_ctx* ctx, const int32_t* t2o, int64_t nt, const uint8_t* active, uint32_t* list,
@@ -107,6 +108,7 @@ enum : int {
     SLOT_NODES4_OBJ_B = 33,
     SLOT_CONT_PARITY = 35,    // containment: parity table of B's first vertices in A
     SLOT_LISTED_A = 36,       // joins by triangle pairs: A's listed groups
+    SLOT_MASKS = 41,          // kept groups per chunk of a culling pass
     SLOT_SPILL = 37,          // ... their work words and entries left for the next round
     SLOT_ENTRY_AB = 38,       // rays from triangles: entry nodes of the listed groups, A->B
     SLOT_ENTRY_BA = 39,
@@ -379,6 +381,11 @@ static int sync_ctx(pierce_ctx* ctx, const char* what) {
     return check_cuda(cudaStreamSynchronize(ctx->stream), what);
 }
 
+static int timed_out(uint32_t bits) {
+    return bits & ERR_QUEUE_TIMEOUT ? set_error(PIERCE_ERR_QUEUE_TIMEOUT, "a bounded wait between blocks expired")
+                                    : PIERCE_OK;
+}
+
 // Translate device error bits into a status (the bits are cleared).  Inside
 // a captured join the bits of the planning run stand in, and the replay
 // compares the device's bits with them.
@@ -387,7 +394,7 @@ static int read_device_error(pierce_ctx* ctx, uint32_t* bits_out) {
     if (int s = host_value(ctx, ctx->d_err, 4, &v, "device error word")) return s;
     *bits_out = (uint32_t)v;
     cudaMemsetAsync(ctx->d_err, 0, sizeof(uint32_t), ctx->stream);
-    return PIERCE_OK;
+    return timed_out(*bits_out);
 }
 
 // The same with the number of keys in the running join's pair set: one copy
@@ -407,7 +414,7 @@ static int read_device_state(pierce_ctx* ctx, uint32_t* bits_out, uint64_t* uniq
     *bits_out = (uint32_t)(h[0] & 0xFFFFFFFF);
     *unique_out = (uint64_t)h[1];
     if (*bits_out) cudaMemsetAsync(ctx->d_err, 0, sizeof(uint32_t), ctx->stream);
-    return PIERCE_OK;
+    return timed_out(*bits_out);
 }
 
 struct EventTimer {
@@ -1102,7 +1109,8 @@ struct Join {
     // words: [0] list count A->B, [1] list count B->A, [2] warp cursor,
     //        [3] deferred-test count, [4] exactly resolved key count,
     //        [5] active triangles of A, [6] active triangles of B, [7] active chunks (chunk
-    //        hierarchy), [8] chunk count of a culling pass, [9] [10] active chunks of A, B
+    //        hierarchy), [8] chunk count of a culling pass, [11] [12] kept groups of A, B, [13] groups
+    //        spanning partitions, [16 + 8 side] four refit counters, [20 + 8 side] six words of bounds
     unsigned long long* words = nullptr;
     // device views of A and B the kernels traverse (their own BVH, or the
     // per-join BVH over active triangles)
@@ -1324,9 +1332,9 @@ struct Join {
         const size_t nobj_a = (size_t)std::max(A->num_objects, 1), nobj_b = (size_t)std::max(B->num_objects, 1);
         // words, object flags, then chunk flags (triangles A, B, edges A, B)
         const size_t chunks = (A->nt + 31) / 32 + (B->nt + 31) / 32 + (A->ne + 31) / 32 + (B->ne + 31) / 32 + 4;
-        if (int s = scratch(ctx, SLOT_CULL, 128 + nobj_a + nobj_b + chunks, &p)) return s;
+        if (int s = scratch(ctx, SLOT_CULL, 512 + nobj_a + nobj_b + chunks, &p)) return s;
         words = static_cast<unsigned long long*>(p);
-        active = static_cast<uint8_t*>(p) + 128;
+        active = static_cast<uint8_t*>(p) + 512;
         chunk_flags = active + nobj_a + nobj_b;
         if (o.cull_objects || o.active_bvh) {
             // chunk lists round up to whole chunks: 32 spare entries
@@ -1429,8 +1437,8 @@ struct Join {
         if (int s = object_bvh(B, SLOT_OBJ_B, SLOT_NODES4_OBJ_B, &objB_)) return s;
         if (object_parity && o.predicate != PIERCE_OVERLAP)
             if (int s = column_grids()) return s;
-        if (int s = launch_object_active(ctx, va, objB_, active)) return s;
-        if (int s = launch_object_active(ctx, vb, objA_, active + std::max(A->num_objects, 1))) return s;
+        if (int s = launch_object_active(ctx, va, objB_, active, vb, objA_, active + std::max(A->num_objects, 1)))
+            return s;
         return build_hierarchies(b0);
     }
 
@@ -1442,8 +1450,7 @@ struct Join {
         uint8_t* act_a = active;
         uint8_t* act_b = active + std::max(A->num_objects, 1);
         if (int s = object_bvh(B, SLOT_OBJ_B, SLOT_NODES4_OBJ_B, &objB_)) return s;
-        if (int s = launch_object_active(ctx, va, objB_, act_a)) return s;
-        if (int s = launch_object_active(ctx, vb, objA_, act_b)) return s;
+        if (int s = launch_object_active(ctx, va, objB_, act_a, vb, objA_, act_b)) return s;
         if (int s = launch_containment_candidates(ctx, cont_ptable, cont_par, cont_pslots, act_a, A->num_objects, act_b,
                                                   B->num_objects))
             return s;
@@ -1457,8 +1464,8 @@ struct Join {
         uint8_t* act_b = active + std::max(A->num_objects, 1);
         const DevDataset objA = objA_, objB = objB_;
         void *ta = nullptr, *tb = nullptr;
-        if (int s = scratch(ctx, SLOT_TRIS_A, 4 * (A->nt + 64), &ta)) return s;
-        if (int s = scratch(ctx, SLOT_TRIS_B, 4 * (B->nt + 64), &tb)) return s;
+        if (int s = scratch(ctx, SLOT_TRIS_A, 4 * (A->nt + 128), &ta)) return s;
+        if (int s = scratch(ctx, SLOT_TRIS_B, 4 * (B->nt + 128), &tb)) return s;
         void* pcl = nullptr;
         const size_t max_chunks = std::max((A->nt + 31) / 32, std::max((B->nt + 31) / 32,
                                            std::max((A->ne + 31) / 32, (B->ne + 31) / 32)));
@@ -1481,44 +1488,33 @@ struct Join {
         // partitioned dataset no group may span two partitions (instanced
         // meshes never do); otherwise the hierarchies are built over the
         // surviving triangles.
-        bool grouped = tri_chunks;
-        if (grouped && A->num_parts > 0) {
-            int32_t* mixed = reinterpret_cast<int32_t*>(words + 13);
-            cudaMemsetAsync(mixed, 0, sizeof(int32_t), ctx->stream);
-            if (int s = launch_group_mixed(ctx, nullptr, (int64_t)((A->nt + 31) / 32), A->d_tri_to_object,
-                                           A->d_obj_part, (int64_t)A->nt, group_size(leaf_a), mixed))
-                return s;
-            if (int s = launch_group_mixed(ctx, nullptr, (int64_t)((B->nt + 31) / 32), B->d_tri_to_object,
-                                           B->d_obj_part, (int64_t)B->nt, group_size(leaf_b), mixed))
-                return s;
-            int64_t m = 0;
-            if (int s = host_value(ctx, mixed, 4, &m, "group partitions")) return s;
-            grouped = m == 0;
-        }
-        if (grouped) {
-            // 1. A's triangle chunks against B's object boxes; 2. A's per-join
-            // hierarchy over the groups of those chunks that meet a B object
-            // box; 3. B's chunks against A's kept triangles; 4. B's per-join
-            // hierarchy over the groups of those chunks that meet one.  Groups
-            // of a few consecutive triangles have tight boxes (a 32-triangle
-            // chunk can straddle the ends of two tube branches), so B's
-            // culling against A's kept triangles is much finer than against
-            // boxes of A's chunks.  Every round keeps the triangles that
-            // contain a point of the other side.
-            if (int s = launch_chunk_cull(ctx, false, A->d_vertices, A->d_indices, A->d_tri_to_object, va, act_a, objB,
-                                          tchunk_a, (uint32_t*)ta, words + 5, nullptr, chunk_list, words + 8))
-                return s;
-            bool filtered = false;
-            if (int s = grouped_side(0, tchunk_a, (uint32_t*)ta, leaf_a, &objB_, &filtered)) return s;
-            groups_a_ = group_size(leaf_a);
-            if (int s = launch_chunk_cull(ctx, false, B->d_vertices, B->d_indices, B->d_tri_to_object, vb, act_b, va,
-                                          tchunk_b, (uint32_t*)tb, words + 6, nullptr, chunk_list, words + 8))
-                return s;
-            if (int s = pair_side(tchunk_b, (uint32_t*)tb)) return s;
-            if (!pairs_route)
-                if (int s = ray_side()) return s;
-            timer.span(b0, timer.record(), &st.ms_build);
-            return PIERCE_OK;
+        if (tri_chunks) {
+            // 1. A's triangle chunks, then their groups, against B's object
+            // boxes; 2. A's per-join hierarchy over the groups kept; 3. B's
+            // chunks and groups against A's kept triangles; 4. B's kept groups
+            // as they are (joins by triangle pairs) or in a hierarchy of their
+            // own.  Groups of a few consecutive triangles have tight boxes (a
+            // 32-triangle chunk can straddle the ends of two tube branches),
+            // so B's culling against A's kept triangles is much finer than
+            // against boxes of A's chunks.  Every round keeps the triangles
+            // that contain a point of the other side.
+            bool mixed = false;
+            if (A->num_parts > 0) cudaMemsetAsync(words + 13, 0, 4, ctx->stream);
+            if (int s = cull_side(0, act_a, objB_, &mixed)) return s;
+            if (!mixed) {
+                if (int s = group_hierarchy(0)) return s;
+                groups_a_ = group_size(leaf_a);
+                if (int s = cull_side(1, act_b, va, &mixed)) return s;
+            }
+            if (!mixed) {
+                if (int s = pair_side()) return s;
+                if (!pairs_route)
+                    if (int s = ray_side()) return s;
+                timer.span(b0, timer.record(), &st.ms_build);
+                return PIERCE_OK;
+            }
+            va = A->view();
+            groups_a_ = 0;
         }
         if (tri_chunks) {
             // groups spanning partitions: the surviving chunks' triangles
@@ -1609,47 +1605,118 @@ struct Join {
         return PIERCE_OK;
     }
 
-    // B's side of a join by triangle pairs, where it applies (pairs_route):
-    // its kept groups of the flagged chunks, met by A's kept triangles.
-    int pair_side(const uint8_t* flags, uint32_t* ids) {
+    // One side's kept groups (group_size of its leaf size): list and device
+    // count; the host's copy of the count where something is sized by it.
+    uint32_t* group_list[2] = {nullptr, nullptr};
+    int64_t group_bound[2] = {0, 0};   // groups at most
+    int64_t group_count[2] = {-1, -1}; // -1: not read yet
+    bool group_filter[2] = {false, false};
+
+    int cull_side(int sd, const uint8_t* active_flags, const DevDataset& other, bool* mixed) {
+        pierce_dataset* ds = sd ? B : A;
+        const int G = group_size(join_leaf(o, ds));
+        const int64_t chunks = (int64_t)((ds->nt + 31) / 32);
+        void *mem = nullptr, *lp = nullptr;
+        if (int s = scratch(ctx, SLOT_MASKS, group_cull_bytes((int64_t)ds->nt, G), &mem)) return s;
+        group_bound[sd] = chunks * (32 / G);
+        if (int s = scratch(ctx, sd ? SLOT_TRIS_B : SLOT_TRIS_A, 4 * ((size_t)group_bound[sd] + 64), &lp)) return s;
+        group_list[sd] = static_cast<uint32_t*>(lp);
+        group_filter[sd] = other.nodes4 != nullptr;
+        if (int s = cull_groups(ctx, ds->view(), ds->d_tri_to_object, active_flags, other, group_filter[sd], G, mem,
+                                group_list[sd], words + 11 + sd, reinterpret_cast<int32_t*>(words + 13),
+                                reinterpret_cast<uint32_t*>(words + 20 + 8 * sd), words + 16 + 8 * sd))
+            return s;
+        group_count[sd] = -1;
+        // A's hierarchy is sized by its count; B's groups are sized by it
+        // only where all of them would take more than 256 MB
+        if (sd == 0 || group_bound[sd] * G > (int64_t(256) << 20) / 48 || ds->num_parts > 0) {
+            if (int s = host_value(ctx, words + 11 + sd, 8, &group_count[sd], "kept groups")) return s;
+            group_bound[sd] = group_count[sd];
+        }
+        if (ds->num_parts > 0) {
+            int64_t m = 0;
+            if (int s = host_value(ctx, words + 13, 4, &m, "group partitions")) return s;
+            *mixed = m != 0;
+        }
+        return PIERCE_OK;
+    }
+
+    // One side's per-join hierarchy over its kept groups.
+    int group_hierarchy(int sd) {
+        pierce_dataset* ds = sd ? B : A;
+        const int G = group_size(join_leaf(o, ds));
+        if (group_count[sd] < 0) {
+            if (int s = host_value(ctx, words + 11 + sd, 8, &group_count[sd], "kept groups")) return s;
+            group_bound[sd] = group_count[sd];
+        }
+        const int64_t n = group_count[sd];
+        const size_t m = (size_t)std::max<int64_t>(n, 1);
+        const int32_t parts = ds->num_parts;
+        void *sp = nullptr, *np = nullptr, *gp = nullptr;
+        if (int s = scratch(ctx, sd ? SLOT_RED_SOUP_B : SLOT_RED_SOUP_A, 48 * (size_t)G * m, &sp)) return s;
+        if (int s = scratch(ctx, sd ? SLOT_RED_NODES_B : SLOT_RED_NODES_A, 64 * m + 8 * (size_t)parts, &np)) return s;
+        if (int s = scratch(ctx, SLOT_GROUPS, 24 * m, &gp)) return s;
+        int2* roots = parts ? reinterpret_cast<int2*>((Node*)np + m) : nullptr;
+        BvhShape sh;
+        if (int s = build_group_lbvh(ctx, ds->view(), ds->d_tri_to_object, group_list[sd], words + 11 + sd, n, G,
+                                     reinterpret_cast<uint32_t*>(words + 20 + 8 * sd), words + 16 + 8 * sd, gp,
+                                     (float4*)sp, (Node*)np, &sh, parts, roots))
+            return s;
+        DevDataset& v = sd ? vb : va;
+        v.soup = (const float4*)sp;
+        v.nodes = (const Node*)np;
+        v.num_tris = n * G;
+        v.root_is_leaf = sh.root_is_leaf;
+        v.root_leaf_count = sh.root_leaf_count;
+        v.part_roots = roots;
+        // four-wide copy in every traversal mode: it also culls the other
+        // side's chunks and filters its groups and rays
+        if (int s = wide_nodes(v, sh.num_nodes, sd ? SLOT_NODES4_B : SLOT_NODES4_A, true, G)) return s;
+        if (o.traversal != 0 || !v.nodes4)
+            if (int s = group_leaves(ctx, (Node*)np, (int64_t)sh.num_nodes, G)) return s;
+        st.active_triangles[sd] = (uint64_t)(n * G);
+        return PIERCE_OK;
+    }
+
+    // B's side of a join by triangle pairs, where it applies (pairs_route).
+    int pair_side() {
         pairs_route = false;
         const int G = group_size(join_leaf(o, A));
-        if (!triangle_pairs_wanted() || G != group_size(join_leaf(o, B)) || G > 16 || va.root_is_leaf || !va.nodes4 ||
-            va.num_tris / G >= (int64_t(1) << 27) || !triangle_edges(0, va.num_tris))
+        if (!triangle_pairs_wanted() || G != group_size(join_leaf(o, B)) || va.root_is_leaf || !va.nodes4 ||
+            va.num_tris / G >= (int64_t(1) << 27) || !triangle_edges(0, va.num_tris) ||
+            group_bound[1] * G >= (int64_t(1) << 30))
             return PIERCE_OK;
-        const int64_t chunks = (int64_t)((B->nt + 31) / 32);
-        if (int s = launch_flag_list(ctx, flags, chunks, ids, words + 10)) return s;
-        int64_t nc = 0;
-        if (int s = host_value(ctx, words + 10, 8, &nc, "active chunks")) return s;
-        const int64_t ng = nc * (32 / G);
-        if (ng * G >= (int64_t(1) << 30)) return PIERCE_OK;
-        void *sp = nullptr, *gp = nullptr, *fp = nullptr;
-        if (int s = scratch(ctx, SLOT_RED_SOUP_B, 48 * 32 * (size_t)std::max<int64_t>(nc, 1), &sp)) return s;
-        if (int s = scratch(ctx, SLOT_GROUPS, 96 * (size_t)std::max<int64_t>(ng, 1) + 512, &gp)) return s;
+        if (!triangle_edges(1, group_bound[1] * G)) {
+            // the exact count decides
+            if (group_count[1] < 0) {
+                if (int s = host_value(ctx, words + 12, 8, &group_count[1], "kept groups")) return s;
+                group_bound[1] = group_count[1];
+            }
+            if (!triangle_edges(1, group_count[1] * G)) return PIERCE_OK;
+        }
+        const int64_t bound = group_bound[1];
+        const size_t m = (size_t)std::max<int64_t>(bound, 1);
+        void *sp = nullptr, *gp = nullptr, *fp = nullptr, *wp = nullptr;
+        if (int s = scratch(ctx, SLOT_RED_SOUP_B, 48 * (size_t)G * m, &sp)) return s;
+        if (int s = scratch(ctx, SLOT_GROUPS, 24 * m, &gp)) return s;
         if (int s = scratch(ctx, SLOT_LISTED_A, (size_t)(va.num_tris / G) + 64, &fp)) return s;
-        if (int s = build_group_units(ctx, B->d_vertices, B->d_indices, B->d_tri_to_object, (int64_t)B->nt, ids, nc, G,
-                                      gp, (float4*)sp, va, words + 12, B->num_parts ? B->d_obj_part : nullptr,
-                                      &pj.units))
+        if (int s = group_units(ctx, B->view(), B->d_tri_to_object, group_list[1], words + 12, bound, G, (float*)gp,
+                                (float4*)sp))
             return s;
         pj.bsoup = (const float4*)sp;
+        pj.gbox = (const float*)gp;
         pj.b_count = words + 12;
+        pj.b_bound = bound;
         pj.b_part = B->d_obj_part;
         pj.G = G;
         pj.a_listed = (uint8_t*)fp;
         // entries left for the next round: up to 512 of each resident warp's
-        pj.spill_cap = std::min<uint64_t>((uint64_t)std::max<int64_t>(ng, 32) * 512, 1ull << 22);
-        void* wp = nullptr;
+        pj.spill_cap = std::min<uint64_t>((uint64_t)std::max<int64_t>(bound, 32) * 512, 1ull << 22);
         if (int s = scratch(ctx, SLOT_SPILL, 64 + 2 * 8 * pj.spill_cap, &wp)) return s;
         pj.work = static_cast<unsigned long long*>(wp);
         pj.spill = reinterpret_cast<uint2*>(pj.work + 8);
         pj.amb_queue = amb_queue;
         pj.amb_cap = amb_cap;
-        int64_t kept = nc * 32;  // at most; the exact count only where it decides
-        if (!triangle_edges(1, kept)) {
-            if (int s = host_value(ctx, words + 12, 8, &kept, "kept groups")) return s;
-            kept *= G;
-            if (!triangle_edges(1, kept)) return PIERCE_OK;
-        }
         pairs_route = true;
         return PIERCE_OK;
     }
@@ -1659,18 +1726,13 @@ struct Join {
     int ray_side() {
         uint8_t* act_a = active;
         uint8_t* act_b = active + std::max(A->num_objects, 1);
-        uint8_t* tchunk_b = chunk_flags + (A->nt + 31) / 32 + 1;
-        uint8_t* echunk_a = tchunk_b + (B->nt + 31) / 32 + 1;
+        uint8_t* echunk_a = chunk_flags + (A->nt + 31) / 32 + 1 + (B->nt + 31) / 32 + 1;
         uint8_t* echunk_b = echunk_a + (A->ne + 31) / 32 + 1;
-        const int leaf_a = join_leaf(o, A), leaf_b = join_leaf(o, B);
-        void* tb = nullptr;
-        if (int s = scratch(ctx, SLOT_TRIS_B, 4 * (B->nt + 64), &tb)) return s;
-        bool filtered = false;
-        if (int s = grouped_side(1, tchunk_b, (uint32_t*)tb, leaf_b, &va, &filtered)) return s;
+        if (int s = group_hierarchy(1)) return s;
         const bool use[2] = {triangle_rays(0, true), triangle_rays(1, true)};
-        const int G[2] = {group_size(leaf_a), group_size(leaf_b)};
+        const int G[2] = {group_size(join_leaf(o, A)), group_size(join_leaf(o, B))};
         // rays: A's groups against B's kept triangles; B's groups met A's already
-        const bool pre[2] = {false, filtered};
+        const bool pre[2] = {false, group_filter[1]};
         if (int s = soup_ray_lists(use, G, pre)) return s;
         if (!use[0])
             if (int s = launch_chunk_cull(ctx, true, nullptr, nullptr, nullptr, va, act_a, vb, echunk_a, list[0],
@@ -1687,7 +1749,7 @@ struct Join {
     // Four-wide copy of a hierarchy: per-join hierarchies for the
     // one-ray-per-thread walk (traversal 0; the other traversals walk the
     // binary nodes) and, always, the hierarchies that culling walks.
-    int wide_nodes(DevDataset& v, uint64_t num_nodes, int slot, bool always = false) {
+    int wide_nodes(DevDataset& v, uint64_t num_nodes, int slot, bool always = false, int G = 1) {
         v.nodes4 = nullptr;
         if ((o.traversal != 0 && !always) || num_nodes == 0 || v.root_is_leaf) return PIERCE_OK;
         void* p = nullptr;
@@ -1697,60 +1759,16 @@ struct Join {
             return PIERCE_OK;
         }
         // Node4 is 128-byte aligned; cudaMalloc returns 256-byte aligned memory
-        if (int s = collapse4(ctx, v.nodes, (int64_t)num_nodes, static_cast<Node4*>(p))) return s;
+        if (int s = collapse4(ctx, v.nodes, (int64_t)num_nodes, static_cast<Node4*>(p), G)) return s;
         v.nodes4 = static_cast<const Node4*>(p);
         return PIERCE_OK;
     }
 
-    // Per side: active chunk ids (into the side's triangle-list buffer), then
-    // a hierarchy over groups of G consecutive triangles of those chunks.
     // triangles per group of a grouped build for leaf size `leaf`
     static int group_size(int leaf) {
         int g = 1;
         while (g < leaf && g < 32) g <<= 1;
         return g;
-    }
-
-    // One side's per-join hierarchy over groups of G consecutive triangles of
-    // its flagged 32-triangle chunks (ids: the side's chunk-list buffer),
-    // keeping only the groups whose box meets a leaf item of `filter` (a
-    // four-wide hierarchy of the other side; none: every group).
-    // *filtered tells whether the filter ran.
-    int grouped_side(int sd, const uint8_t* flags, uint32_t* ids, int leaf, const DevDataset* filter, bool* filtered) {
-        pierce_dataset* ds = sd ? B : A;
-        const int G = group_size(leaf);
-        const int64_t chunks = (int64_t)((ds->nt + 31) / 32);
-        if (int s = launch_flag_list(ctx, flags, chunks, ids, words + 9 + sd)) return s;
-        int64_t nc = 0;
-        if (int s = host_value(ctx, words + 9 + sd, 8, &nc, "active chunks")) return s;
-        const int64_t ng = nc * (32 / G);
-        const int32_t parts = ds->num_parts;
-        const int soup_slot = sd ? SLOT_RED_SOUP_B : SLOT_RED_SOUP_A, node_slot = sd ? SLOT_RED_NODES_B : SLOT_RED_NODES_A;
-        void *sp = nullptr, *np = nullptr, *gp = nullptr;
-        if (int s = scratch(ctx, soup_slot, 48 * 32 * (size_t)std::max<int64_t>(nc, 1), &sp)) return s;
-        if (int s = scratch(ctx, node_slot, 64 * (size_t)std::max<int64_t>(ng, 1) + 8 * (size_t)parts, &np)) return s;
-        int2* roots = parts ? reinterpret_cast<int2*>((Node*)np + std::max<int64_t>(ng, 1)) : nullptr;
-        if (int s = scratch(ctx, SLOT_GROUPS, 96 * (size_t)std::max<int64_t>(ng, 1) + 512, &gp)) return s;
-        if (filter && !filter->nodes4) filter = nullptr;
-        *filtered = filter != nullptr;
-        BvhShape sh;
-        int64_t kept = ng;
-        if (int s = build_grouped_lbvh(ctx, ds->d_vertices, ds->d_indices, ds->d_tri_to_object, (int64_t)ds->nt, ids,
-                                       nc, G, gp, (float4*)sp, (Node*)np, &sh, filter, words + 11 + sd, &kept,
-                                       ds->d_obj_part, parts, roots))
-            return s;
-        DevDataset& v = sd ? vb : va;
-        v.soup = (const float4*)sp;
-        v.nodes = (const Node*)np;
-        v.num_tris = kept * G;
-        v.root_is_leaf = sh.root_is_leaf;
-        v.root_leaf_count = sh.root_leaf_count;
-        v.part_roots = roots;
-        // four-wide copy in every traversal mode: it also culls the other
-        // side's chunks and filters its groups and rays
-        if (int s = wide_nodes(v, sh.num_nodes, sd ? SLOT_NODES4_B : SLOT_NODES4_A, true)) return s;
-        st.active_triangles[sd] = (uint64_t)(kept * G);
-        return PIERCE_OK;
     }
 
     int precision_mode() const {

@@ -148,19 +148,13 @@ struct ColumnGrid {
 
 constexpr int kSizingScratchSlot = 21;  // 21 and 22: learned sizing (sizing.cu)
 
-// The walking side of a join by triangle pairs (pairs.cu): B's kept groups of
-// triangles without a hierarchy.
-struct GroupUnits {
-    int64_t bound = 0;                // candidate groups; the kept count is on the device
-    const float* gbox = nullptr;      // boxes of the candidates
-    const uint32_t* glist = nullptr;  // the kept candidates
-};
-
 // A join by triangle pairs: B's kept groups against A's per-join hierarchy.
 struct PairJoin {
-    GroupUnits units;
-    const float4* bsoup = nullptr;               // the kept groups' triangles, G each
-    const unsigned long long* b_count = nullptr; // kept groups
+    // the walking side: B's kept groups, without a hierarchy
+    const float4* bsoup = nullptr;               // their triangles, G each
+    const float* gbox = nullptr;                 // their boxes
+    const unsigned long long* b_count = nullptr; // their number, at most b_bound
+    int64_t b_bound = 0;
     const int32_t* b_part = nullptr;             // partition per B object (partitioned joins)
     int G = 4;                                   // triangles per group, both sides
     uint8_t* a_listed = nullptr;                 // a byte per A leaf group
@@ -363,28 +357,33 @@ int build_lbvh(pierce_ctx* ctx, const float* verts, const uint32_t* idx, const i
 // Chunk boxes, object boxes, ranges and flags.  With edges_ready (the edge
 // upload kernel already wrote the edge chunk boxes and the edge-order flag
 // *grouped_flag), the edge-side work waits for ev_edges instead.
-// Node4 copy of a binary hierarchy with num_nodes internal nodes
-int collapse4(pierce_ctx* ctx, const Node* nodes, int64_t num_nodes, Node4* out);
+// Node4 copy of a binary hierarchy with num_nodes internal nodes (G soup
+// triangles per leaf item)
+int collapse4(pierce_ctx* ctx, const Node* nodes, int64_t num_nodes, Node4* out, int G = 1);
 int prepare_objects(pierce_ctx* ctx, pierce_dataset* ds, cudaEvent_t edges_ready = nullptr,
                     const int32_t* grouped_flag = nullptr);
-// hierarchy over groups of G consecutive triangles (G divides 32) of the
-// listed 32-triangle chunks; group_scratch holds 96 bytes per group (+ 512).
-// With `filter` only the groups whose box meets a leaf of that four-wide
-// hierarchy are kept (join.cu k_group_filter); *kept receives their number.
-int build_grouped_lbvh(pierce_ctx* ctx, const float* verts, const uint32_t* idx, const int32_t* t2o, int64_t nt,
-                       const uint32_t* chunk_list, int64_t n_chunks, int G, void* group_scratch, float4* soup,
-                       Node* nodes, BvhShape* shape, const DevDataset* filter = nullptr,
-                       unsigned long long* d_count = nullptr, int64_t* kept = nullptr,
-                       const int32_t* obj_part = nullptr, int32_t num_parts = 0, int2* part_roots = nullptr);
-int build_group_units(pierce_ctx* ctx, const float* verts, const uint32_t* idx, const int32_t* t2o, int64_t nt,
-                      const uint32_t* chunk_list, int64_t n_chunks, int G, void* group_scratch, float4* soup,
-                      const DevDataset& filter, unsigned long long* d_count, const int32_t* obj_part,
-                      GroupUnits* out);
-int launch_group_filter(pierce_ctx* ctx, const float* gbox, int64_t ng, const DevDataset& other,
-                        const int32_t* gt2o, const int32_t* obj_part, uint8_t* flags);
-// partitioned datasets: *mixed |= some group of a flagged chunk spans two partitions
-int launch_group_mixed(pierce_ctx* ctx, const uint8_t* chunk_flags, int64_t n_chunks, const int32_t* t2o,
-                       const int32_t* obj_part, int64_t nt, int G, int32_t* mixed);
+// Groups of G consecutive triangles (G divides 32; each in one of the
+// dataset's 32-triangle chunks) that can meet the other side: list[k] =
+// chunk * (32 / G) + group in order, *d_count their number.  mem:
+// group_cull_bytes; with `filter` groups are tested too (other.nodes4);
+// *d_mixed |= a group of a kept chunk spans two partitions.  bounds (6
+// words) and zero (4 words) are prepared for build_group_lbvh.
+size_t group_cull_bytes(int64_t nt, int G);
+int cull_groups(pierce_ctx* ctx, const DevDataset& src, const int32_t* t2o, const uint8_t* active,
+                const DevDataset& other, bool filter, int G, void* mem, uint32_t* list, unsigned long long* d_count,
+                int32_t* d_mixed, uint32_t* bounds, unsigned long long* zero);
+// the listed groups (at most `bound`) as boxes and a soup in list order
+int group_units(pierce_ctx* ctx, const DevDataset& src, const int32_t* t2o, const uint32_t* list,
+                const unsigned long long* d_count, int64_t bound, int G, float* gbox, float4* soup);
+// hierarchy over the n listed groups, one per leaf (group_scratch: 24 bytes
+// per group); soup in leaf order, G triangles per leaf.  The binary nodes'
+// leaves count groups until group_leaves turns them into soup ranges
+// (collapse4 with G does so for the four-wide copy).
+int build_group_lbvh(pierce_ctx* ctx, const DevDataset& src, const int32_t* t2o, const uint32_t* list,
+                     const unsigned long long* d_count, int64_t n, int G, uint32_t* bounds,
+                     unsigned long long* wave_count, void* group_scratch, float4* soup, Node* nodes, BvhShape* shape,
+                     int32_t num_parts, int2* part_roots);
+int group_leaves(pierce_ctx* ctx, Node* nodes, int64_t num_nodes, int G);
 
 // join.cu, pairs.cu: the pair tests of a join by triangle pairs into a pair
 // hash set, and its ray count

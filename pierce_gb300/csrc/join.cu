@@ -32,6 +32,7 @@
 #include "common.cuh"
 #include "hash.cuh"
 #include "predicates.cuh"
+#include "walk.cuh"
 
 namespace pgpu {
 
@@ -136,47 +137,6 @@ __device__ __forceinline__ void load_ray(const EdgeRayParams& P, int64_t e, floa
     obj = __float_as_int(s4.w);
     p = make_float3(s4.x, s4.y, s4.z);
     q = make_float3(e4.x, e4.y, e4.z);
-}
-
-// Any-hit box query over a Node4 hierarchy from internal node `node`: true
-// as soon as leaf_hit(first, count) is true for a leaf whose box meets
-// [lo, hi] (and, conservatively, if the stack would overflow).
-template <class LeafHit>
-__device__ __forceinline__ bool any_hit4(const Node4* nodes4, int node, const float3& lo, const float3& hi,
-                                         LeafHit&& leaf_hit) {
-    int stack[kStackSize4];
-    int sp = 0;
-    for (;;) {
-        const Node4* nd = nodes4 + node;
-        const float4 lx = __ldg(&nd->lox), hx = __ldg(&nd->hix), ly = __ldg(&nd->loy), hy = __ldg(&nd->hiy);
-        const float4 lz = __ldg(&nd->loz), hz = __ldg(&nd->hiz);
-        const int4 ch = __ldg(&nd->ch);
-        const int cnt = __ldg(&nd->meta.x);
-        const bool h[4] = {box_overlap(lx.x, hx.x, ly.x, hy.x, lz.x, hz.x, lo, hi),
-                           box_overlap(lx.y, hx.y, ly.y, hy.y, lz.y, hz.y, lo, hi),
-                           box_overlap(lx.z, hx.z, ly.z, hy.z, lz.z, hz.z, lo, hi),
-                           box_overlap(lx.w, hx.w, ly.w, hy.w, lz.w, hz.w, lo, hi)};
-        const int c[4] = {ch.x, ch.y, ch.z, ch.w};
-        int next = -1;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            if (!h[j]) continue;
-            if (c[j] < 0) {
-                if (leaf_hit(~c[j], (cnt >> (8 * j)) & 0xFF)) return true;
-            } else if (next < 0) {
-                next = c[j];
-            } else {
-                if (sp >= kStackSize4) return true;
-                stack[sp++] = c[j];
-            }
-        }
-        if (next >= 0) {
-            node = next;
-        } else {
-            if (sp == 0) return false;
-            node = stack[--sp];
-        }
-    }
 }
 
 struct RayCounters {
@@ -585,11 +545,20 @@ __global__ void __launch_bounds__(128) k_resolve_ambiguous(EdgeRayParams P, uint
 // Object culling: a source object is active when its box overlaps the box
 // of at least one target triangle (exact comparisons).  A segment's box lies
 // inside its object's box, so inactive objects' edges cannot hit anything.
-__global__ void __launch_bounds__(128) k_object_active(DevDataset src, DevDataset tgt, uint8_t* active) {
+// Both sides of a join in one launch: the first blocks0 blocks take side 0.
+struct ActiveSide {
+    DevDataset src, tgt;
+    uint8_t* active;
+};
+__global__ void __launch_bounds__(128) k_object_active(ActiveSide side0, ActiveSide side1, unsigned blocks0) {
     __shared__ int sstack[kShortStack][128];
     int lstack[kStackSize - kShortStack];
     const int tid = threadIdx.x;
-    const int64_t o = blockIdx.x * (int64_t)blockDim.x + tid;
+    const bool second = blockIdx.x >= blocks0;
+    const DevDataset& src = second ? side1.src : side0.src;
+    const DevDataset& tgt = second ? side1.tgt : side0.tgt;
+    uint8_t* active = second ? side1.active : side0.active;
+    const int64_t o = (blockIdx.x - (second ? blocks0 : 0u)) * (int64_t)blockDim.x + tid;
     if (o >= src.num_objects) return;
     const float* b = src.obj_box + 6 * o;
     const float3 lo = make_float3(b[0], b[1], b[2]), hi = make_float3(b[3], b[4], b[5]);
@@ -1243,9 +1212,14 @@ int launch_resolve(pierce_ctx* ctx, const DevDataset& src, const DevDataset& tgt
     return check_cuda(cudaGetLastError(), "resolve ambiguous tests");
 }
 
-int launch_object_active(pierce_ctx* ctx, const DevDataset& src, const DevDataset& tgt, uint8_t* active) {
-    if (src.num_objects <= 0) return PIERCE_OK;
-    k_object_active<<<(unsigned)((src.num_objects + 127) / 128), 128, 0, ctx->stream>>>(src, tgt, active);
+// Activity flags of a's objects against tgt_a and (num_objects > 0) of b's
+// against tgt_b.
+int launch_object_active(pierce_ctx* ctx, const DevDataset& a, const DevDataset& tgt_a, uint8_t* active_a,
+                         const DevDataset& b, const DevDataset& tgt_b, uint8_t* active_b) {
+    const unsigned n0 = (unsigned)((std::max(a.num_objects, 0) + 127) / 128);
+    const unsigned n1 = (unsigned)((std::max(b.num_objects, 0) + 127) / 128);
+    if (n0 + n1 == 0) return PIERCE_OK;
+    k_object_active<<<n0 + n1, 128, 0, ctx->stream>>>(ActiveSide{a, tgt_a, active_a}, ActiveSide{b, tgt_b, active_b}, n0);
     ctx->launches += 1;
     return check_cuda(cudaGetLastError(), "object activity");
 }
@@ -1263,7 +1237,7 @@ int launch_collect_rays(pierce_ctx* ctx, const DevDataset& src, const uint8_t* a
 
 int launch_cull(pierce_ctx* ctx, const DevDataset& src, const DevDataset& tgt, uint8_t* active, uint32_t* list,
                 unsigned long long* count) {
-    if (int s = launch_object_active(ctx, src, tgt, active)) return s;
+    if (int s = launch_object_active(ctx, src, tgt, active, DevDataset{}, DevDataset{}, nullptr)) return s;
     return launch_collect_rays(ctx, src, active, list, count);
 }
 
@@ -1275,68 +1249,6 @@ int launch_cull(pierce_ctx* ctx, const DevDataset& src, const DevDataset& tgt, u
 // its object's box).  A warp forms the boxes of 32 chunks, one per lane, and
 // every lane then queries the other side's object hierarchy with its box.
 constexpr int kChunk = 32;
-
-// Does leaf [first, first + count) of `h` meet [lo, hi]?  A soup of boxes
-// (degenerate triangles lo, hi, hi) is tested box by box, a soup of
-// triangles by each triangle's box.
-__device__ __forceinline__ bool leaf_meets_box(const DevDataset& h, int first, int count, const float3& lo,
-                                               const float3& hi) {
-    for (int k = 0; k < count; ++k) {
-        const int64_t t = (int64_t)first + k;
-        const float4 a4 = __ldg(h.soup + 3 * t), b4 = __ldg(h.soup + 3 * t + 1);
-        if (h.soup_boxes) {
-            if (box_overlap(a4.x, b4.x, a4.y, b4.y, a4.z, b4.z, lo, hi)) return true;
-        } else {
-            const float4 c4 = __ldg(h.soup + 3 * t + 2);
-            if (box_overlap(fminf(a4.x, fminf(b4.x, c4.x)), fmaxf(a4.x, fmaxf(b4.x, c4.x)),
-                            fminf(a4.y, fminf(b4.y, c4.y)), fmaxf(a4.y, fmaxf(b4.y, c4.y)),
-                            fminf(a4.z, fminf(b4.z, c4.z)), fmaxf(a4.z, fmaxf(b4.z, c4.z)), lo, hi))
-                return true;
-        }
-    }
-    return false;
-}
-
-// Per-join builds over groups of triangles keep only the groups whose box
-// meets a leaf item of `other`, a four-wide hierarchy of the other side:
-// object boxes, surviving chunk boxes, or the other side's kept triangles.
-// A group that meets none cannot meet the other side's edges, which lie in
-// those boxes.
-// Partitioned sides (gt2o and obj_part given): a group only meets the other
-// side's subtree of its own partition.
-__global__ void __launch_bounds__(256) k_group_filter(const float* __restrict__ gbox, int64_t ng, DevDataset other,
-                                                      const int32_t* __restrict__ gt2o,
-                                                      const int32_t* __restrict__ obj_part,
-                                                      uint8_t* __restrict__ flags) {
-    for (int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; g < ng; g += (int64_t)gridDim.x * blockDim.x) {
-        const float* b = gbox + 6 * g;
-        const float3 lo = make_float3(b[0], b[1], b[2]), hi = make_float3(b[3], b[4], b[5]);
-        auto leaf_hit = [&](int first, int count) { return leaf_meets_box(other, first, count, lo, hi); };
-        bool keep = true;  // without a hierarchy (a single root leaf) keep everything
-        if (gt2o && obj_part && other.part_roots) {
-            const int32_t o = __ldg(gt2o + g);
-            const int2 r = o >= 0 ? __ldg(other.part_roots + __ldg(obj_part + o)) : make_int2(-1, 0);
-            if (!(lo.x <= hi.x)) keep = true;
-            else if (r.x >= 0) keep = other.nodes4 ? any_hit4(other.nodes4, r.x, lo, hi, leaf_hit) : true;
-            else keep = r.y > 0 && leaf_hit(~r.x, r.y);
-        } else if (!other.root_is_leaf && other.nodes4 && lo.x <= hi.x) {
-            keep = any_hit4(other.nodes4, 0, lo, hi, leaf_hit);
-        } else if (other.num_tris == 0) {
-            keep = false;
-        }
-        flags[g] = keep ? 1 : 0;
-    }
-}
-
-int launch_group_filter(pierce_ctx* ctx, const float* gbox, int64_t ng, const DevDataset& other,
-                        const int32_t* gt2o, const int32_t* obj_part, uint8_t* flags) {
-    if (ng <= 0) return PIERCE_OK;
-    const int64_t blocks = std::min<int64_t>((ng + 255) / 256, (int64_t)ctx->sm_count * 16);
-    k_group_filter<<<(unsigned)std::max<int64_t>(blocks, 1), 256, 0, ctx->stream>>>(gbox, ng, other, gt2o, obj_part,
-                                                                                  flags);
-    ctx->launches += 1;
-    return check_cuda(cudaGetLastError(), "group filter");
-}
 
 // ---- rays from the kept triangles ---------------------------------------------
 // A join that builds per-join hierarchies over the triangles that can take
@@ -1733,53 +1645,6 @@ int launch_soup_rays(pierce_ctx* ctx, const float4* soup, int64_t n_tris, int G,
                                                              shard_index, shard_count, entry_nodes4, entries);
     ctx->launches += 1;
     return check_cuda(cudaGetLastError(), "rays from triangles");
-}
-
-// Does [lo, hi] meet an item of `objs` within partition `part`?  Items are
-// the boxes of a box hierarchy (object or chunk boxes as degenerate
-// triangles) or the triangles of a per-join hierarchy (by their boxes).
-__device__ bool meets_any_object(const DevDataset& objs, int32_t part, const float3& lo, const float3& hi) {
-    auto leaf_hit = [&](int first, int count) { return leaf_meets_box(objs, first, count, lo, hi); };
-    int node;
-    if (objs.part_roots) {
-        const int2 r = __ldg(objs.part_roots + part);
-        if (r.x < 0) return leaf_hit(~r.x, r.y);
-        node = r.x;
-    } else if (objs.root_is_leaf) {
-        return leaf_hit(0, objs.root_leaf_count);
-    } else {
-        node = 0;
-    }
-    if (objs.nodes4) return any_hit4(objs.nodes4, node, lo, hi, leaf_hit);
-    int stack[kStackSize];
-    int sp = 0;
-    for (;;) {
-        const Node* nd = objs.nodes + node;
-        const float4 bx = __ldg(&nd->bx), by = __ldg(&nd->by), bz = __ldg(&nd->bz);
-        const int4 ch = __ldg(&nd->ch);
-        bool h0 = box_overlap(bx.x, bx.y, by.x, by.y, bz.x, bz.y, lo, hi);
-        bool h1 = box_overlap(bx.z, bx.w, by.z, by.w, bz.z, bz.w, lo, hi);
-        if (h0 && ch.x < 0) {
-            if (leaf_hit(~ch.x, ch.z & 0xFF)) return true;
-            h0 = false;
-        }
-        if (h1 && ch.y < 0) {
-            if (leaf_hit(~ch.y, (ch.z >> 8) & 0xFF)) return true;
-            h1 = false;
-        }
-        if (h0 && h1) {
-            if (sp >= kStackSize) return true;  // cannot happen for an LBVH; stay conservative
-            stack[sp++] = ch.y;
-            node = ch.x;
-        } else if (h0) {
-            node = ch.x;
-        } else if (h1) {
-            node = ch.y;
-        } else {
-            if (sp == 0) return false;
-            node = stack[--sp];
-        }
-    }
 }
 
 // Per chunk of triangles (EDGES = false) or edges (EDGES = true) of `src`:

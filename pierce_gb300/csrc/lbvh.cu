@@ -24,6 +24,7 @@
 #include <cstdio>
 
 #include "common.cuh"
+#include "walk.cuh"
 
 namespace pgpu {
 
@@ -99,10 +100,11 @@ __device__ __forceinline__ uint32_t expand_bits10(uint32_t v) {
 }
 
 // 2. Morton codes
+// (inverted: all ones when the bounds' maxima are stored inverted, else 0)
 __global__ void k_morton(const float4* __restrict__ cen, int64_t nt, const uint32_t* __restrict__ bounds,
-                         uint32_t* __restrict__ keys, uint32_t* __restrict__ vals) {
+                         uint32_t* __restrict__ keys, uint32_t* __restrict__ vals, uint32_t inverted) {
     const float lo[3] = {o2f(bounds[0]), o2f(bounds[1]), o2f(bounds[2])};
-    const float hi[3] = {o2f(bounds[3]), o2f(bounds[4]), o2f(bounds[5])};
+    const float hi[3] = {o2f(bounds[3] ^ inverted), o2f(bounds[4] ^ inverted), o2f(bounds[5] ^ inverted)};
     float inv[3];
     for (int k = 0; k < 3; ++k) inv[k] = hi[k] > lo[k] ? 1.0f / (hi[k] - lo[k]) : 0.0f;
     for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < nt; t += (int64_t)gridDim.x * blockDim.x) {
@@ -170,7 +172,7 @@ __global__ void k_centroids_parts(const float* __restrict__ verts, const uint32_
 }
 
 __global__ void k_morton_parts(const float4* __restrict__ cen, int64_t nt, const uint32_t* __restrict__ bounds,
-                               uint64_t* __restrict__ keys, uint32_t* __restrict__ vals) {
+                               uint64_t* __restrict__ keys, uint32_t* __restrict__ vals, uint32_t inverted) {
     for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < nt; t += (int64_t)gridDim.x * blockDim.x) {
         const float4 c = cen[t];
         const int32_t part = __float_as_int(c.w);
@@ -178,7 +180,7 @@ __global__ void k_morton_parts(const float4* __restrict__ cen, int64_t nt, const
         const float cc[3] = {c.x, c.y, c.z};
         uint32_t q[3];
         for (int k = 0; k < 3; ++k) {
-            const float lo = o2f(b[k]), hi = o2f(b[3 + k]);
+            const float lo = o2f(b[k]), hi = o2f(b[3 + k] ^ inverted);
             const float inv = hi > lo ? 1.0f / (hi - lo) : 0.0f;
             float u = (cc[k] - lo) * inv;
             u = fminf(fmaxf(u, 0.0f), 1.0f);
@@ -750,6 +752,27 @@ int prepare_objects(pierce_ctx* ctx, pierce_dataset* ds, cudaEvent_t edges_ready
     return PIERCE_OK;
 }
 
+// Refit above the leaf wave: waves for the wide bottom levels, then one chain
+// launch for the rest.  lists: n + 3 words, the leaf wave's list first;
+// wave_count: four counters, zero but for the leaf wave's.  Small hierarchies
+// (object boxes, small joins) go straight to the chain: their waves would be
+// launches of a few blocks each.
+static void refit_above(pierce_ctx* ctx, Node* nodes, int64_t n, uint32_t* list0, unsigned long long* wave_count,
+                        float* d_root_box) {
+    const int B = 256;
+    cudaStream_t st = ctx->stream;
+    uint32_t* lists[2] = {list0, list0 + (n + 1) / 2 + 1};
+    const int kWaves = n >= (1 << 18) ? 3 : 0;
+    for (int wave = 0; wave < kWaves; ++wave) {
+        const int in = wave & 1, out = in ^ 1;
+        k_refit_wave<<<grid_for(ctx, n / 2 + 1, B), B, 0, st>>>(nodes, n - 1, lists[in], wave_count + wave, n / 2 + 1,
+                                                                lists[out], wave_count + wave + 1, d_root_box);
+    }
+    k_refit_chain<<<grid_for(ctx, n / 2 + 1, B), B, 0, st>>>(nodes, n - 1, lists[kWaves & 1], wave_count + kWaves,
+                                                             n / 2 + 1, d_root_box, ctx->d_err);
+    ctx->launches += 1 + kWaves;
+}
+
 // Triangles -> LBVH.  The n triangles are idx[3t..3t+2] for t = list[i]
 // (or t = i without a list); soup and nodes receive the structure; build
 // temporaries live in scratch slots 1..4.  Everything is enqueued on the
@@ -784,7 +807,7 @@ int build_lbvh(pierce_ctx* ctx, const float* verts, const uint32_t* idx, const i
     if (int s = scratch(ctx, 2, 2 * key_bytes * (size_t)n, &pk)) return s;
     if (int s = scratch(ctx, 3, 2 * sizeof(uint32_t) * (size_t)n, &pv)) return s;
     const size_t part_bounds = parts ? 24 * (size_t)num_parts : 0;
-    if (int s = scratch(ctx, 4, sizeof(unsigned long long) * (size_t)n + 64 + 64 + part_bounds, &pm)) return s;
+    if (int s = scratch(ctx, 4, sizeof(unsigned long long) * (size_t)n + 64 + 64 + part_bounds + 64, &pm)) return s;
     float4* cen = static_cast<float4*>(pc);
     uint32_t* keys = static_cast<uint32_t*>(pk);
     uint32_t* vals = static_cast<uint32_t*>(pv);
@@ -792,7 +815,7 @@ int build_lbvh(pierce_ctx* ctx, const float* verts, const uint32_t* idx, const i
     uint32_t* bounds = reinterpret_cast<uint32_t*>(leaf_rec + n);  // 6 words
     float* d_root_box = reinterpret_cast<float*>(bounds + 6);        // 6 floats
     // byte layout after the n leaf records: bounds [8n, 8n+24), root box
-    // [8n+24, 8n+48), two wave counters [8n+64, 8n+80); allocation 8n+128
+    // [8n+24, 8n+48), four wave counters [8n+64, 8n+96); allocation 8n+192
     unsigned long long* wave_count = leaf_rec + n + 8;
     // partitioned: per-partition bounds after that, [8n+128, ...)
     uint32_t* pbounds = reinterpret_cast<uint32_t*>(leaf_rec + n + 16);
@@ -803,7 +826,7 @@ int build_lbvh(pierce_ctx* ctx, const float* verts, const uint32_t* idx, const i
         const int64_t nb = 6 * (int64_t)num_parts;
         k_obj_box_init<<<grid_for(ctx, nb, B), B, 0, st>>>(pbounds, num_parts);  // ordered (+max, -max)
         k_centroids_parts<<<grid_for(ctx, n, B), B, 0, st>>>(verts, idx, list, t2o, obj_part, n, cen, pbounds);
-        k_morton_parts<<<grid_for(ctx, n, B), B, 0, st>>>(cen, n, pbounds, keys64, vals);
+        k_morton_parts<<<grid_for(ctx, n, B), B, 0, st>>>(cen, n, pbounds, keys64, vals, 0u);
         ctx->launches += 3;
         int bits = 0;
         while (bits < 32 && (1ll << bits) < (int64_t)num_parts) ++bits;
@@ -812,7 +835,7 @@ int build_lbvh(pierce_ctx* ctx, const float* verts, const uint32_t* idx, const i
         k_fill_u32<<<1, 32, 0, st>>>(bounds, 0xFFFFFFFFu, 3);  // ordered +max
         k_fill_u32<<<1, 32, 0, st>>>(bounds + 3, 0u, 3);       // ordered -max
         k_centroids<<<std::min(grid_for(ctx, n, B), ctx->sm_count * 4), B, 0, st>>>(verts, idx, list, n, cen, bounds);
-        k_morton<<<grid_for(ctx, n, B), B, 0, st>>>(cen, n, bounds, keys, vals);
+        k_morton<<<grid_for(ctx, n, B), B, 0, st>>>(cen, n, bounds, keys, vals, 0u);
         ctx->launches += 4;
         if (int s = sort_u32_pairs(ctx, keys, keys + n, vals, vals + n, n, 30)) return s;
     }
@@ -841,25 +864,11 @@ int build_lbvh(pierce_ctx* ctx, const float* verts, const uint32_t* idx, const i
         else
             k_karras<uint32_t><<<grid_for(ctx, n - 1, B), B, 0, st>>>(skeys, n, leaf_size, nodes, leaf_rec,
                                                                       nullptr);
-        // waves for the wide bottom levels, then one chain launch for the rest;
-        // the lists reuse the Morton key buffer (free after the hierarchy step)
-        uint32_t* lists[2] = {keys, keys + (n + 1) / 2 + 1};
-        cudaMemsetAsync(wave_count, 0, 2 * sizeof(unsigned long long), st);
-        k_refit_leaves<<<grid_for(ctx, n, B), B, 0, st>>>(soup, n, nodes, leaf_rec, lists[0], wave_count);
-        // small hierarchies (object and chunk boxes) go straight to the chain:
-        // their waves would be launches of a few blocks each
-        const int kWaves = n >= (1 << 18) ? 3 : 0;
-        for (int wave = 0; wave < kWaves; ++wave) {
-            const int in = wave & 1, out = in ^ 1;
-            cudaMemsetAsync(wave_count + out, 0, sizeof(unsigned long long), st);
-            k_refit_wave<<<grid_for(ctx, n / 2 + 1, B), B, 0, st>>>(nodes, n - 1, lists[in], wave_count + in,
-                                                                       n / 2 + 1, lists[out], wave_count + out,
-                                                                       d_root_box);
-        }
-        const int last = kWaves & 1;
-        k_refit_chain<<<grid_for(ctx, n / 2 + 1, B), B, 0, st>>>(nodes, n - 1, lists[last], wave_count + last,
-                                                                    n / 2 + 1, d_root_box, ctx->d_err);
-        ctx->launches += 3 + kWaves;
+        // the wave lists reuse the Morton key buffer (free after the hierarchy step)
+        cudaMemsetAsync(wave_count, 0, 4 * sizeof(unsigned long long), st);
+        k_refit_leaves<<<grid_for(ctx, n, B), B, 0, st>>>(soup, n, nodes, leaf_rec, keys, wave_count);
+        ctx->launches += 2;
+        refit_above(ctx, nodes, n, keys, wave_count, d_root_box);
         shape->num_nodes = (uint64_t)(n - 1);
         shape->root_is_leaf = 0;
         shape->root_leaf_count = 0;
@@ -895,82 +904,430 @@ __device__ __forceinline__ int64_t group_item(int64_t c, int j, int G, int k, in
     return first < nt ? first : c * 32;
 }
 
-__global__ void __launch_bounds__(256) k_group_boxes(const float* __restrict__ verts, const uint32_t* __restrict__ idx,
-                                                     const int32_t* __restrict__ t2o, int64_t nt,
-                                                     const uint32_t* __restrict__ chunk_list, int64_t n_chunks,
-                                                     int G, float* __restrict__ gbox, uint32_t* __restrict__ gidx,
-                                                     int32_t* __restrict__ gt2o) {
+// ---- culling a side to the groups that can meet the other side -----------------
+// Two passes, each with its walks shared by a warp (warp_any_hit).
+// k_cull_chunks: 32 chunks of 32 triangles to a warp, a lane per chunk's
+// stored box; the chunks that meet the other side are listed (any order).  A
+// word of 32 chunks that lies in inactive objects costs two object ids and
+// two ranges, not 32 boxes (objects are stored contiguously; most meshes are
+// longer than a word).  k_cull_groups: the listed chunks' groups, formed a
+// lane per triangle and tested 32 groups at a time; masks[c] are chunk c's
+// kept groups.  Bound by issue and L1 (48-67 % of issue slots, 71-77 % of the
+// L1 on the dense join).  With k_list_groups they take the place of chunk
+// flags, chunk lists, group boxes, group flags and group lists (13 launches a
+// side): 400,000 x 100,000 ellipsoids 0.93 -> 0.81 ms, 64 batched joins 5.0
+// -> 1.75 ms (their chunks' stored boxes are read now, not their vertices),
+// 60 x 60 spheres 18 launches fewer.
+template <int G>
+struct GroupMask { using type = uint8_t; };
+template <>
+struct GroupMask<2> { using type = uint16_t; };
+template <>
+struct GroupMask<1> { using type = uint32_t; };
+
+struct CullParams {
+    const float* verts;
+    const uint32_t* idx;
+    const int32_t* t2o;
+    int64_t nt;
+    const float* chunk_box;
+    const int2* obj_range;       // null: objects not contiguous
+    const uint8_t* active;       // per object
+    const int32_t* obj_part;     // partitioned datasets
+    DevDataset other;            // the other side's object boxes or kept triangles
+    int filter;                  // groups too are tested (the hierarchy has four-wide nodes)
+    int wide;                    // node ids fit the shared walk's stack
+    int mask_bytes;
+    void* masks;
+    uint32_t* chunk_list;
+    unsigned long long* chunk_count;
+    int32_t* mixed;              // set when a group of a kept chunk spans two partitions
+    // words the kernels after this one start from
+    uint32_t* bounds;            // 6 words set to all ones
+    unsigned long long* zero;    // 4 words set to zero
+};
+
+// Does each lane's box (live lanes) meet an item of P.other within partition
+// `part`?
+static __device__ __forceinline__ bool cull_query(const CullParams& P, WarpBoxes& W, bool live, int32_t part,
+                                                  const float3& lo, const float3& hi) {
+    if (!P.wide || (!P.other.part_roots && P.other.root_is_leaf))
+        return live && meets_any_object(P.other, part, lo, hi);
+    int start = live ? 0 : -1;
+    bool hit = false;
+    if (live && P.other.part_roots) {
+        const int2 r = part >= 0 ? __ldg(P.other.part_roots + part) : make_int2(-1, 0);
+        start = r.x;
+        if (r.x < 0) hit = r.y > 0 && leaf_meets_box(P.other, ~r.x, r.y, lo, hi);
+    }
+    return ((warp_any_hit(P.other, W, start, lo, hi) >> (threadIdx.x & 31)) & 1u) || hit;
+}
+
+__global__ void __launch_bounds__(128) k_cull_chunks(CullParams P) {
+    __shared__ WarpBoxes boxes[4];
+    WarpBoxes& W = boxes[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
+    const int64_t n_chunks = (P.nt + 31) / 32, n_words = (n_chunks + 31) / 32;
     const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-    for (int64_t k = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); k < n_chunks; k += warps) {
-        const int64_t c = chunk_list[k];
-        int64_t t = group_item(c, lane / G, G, lane % G, nt);
-        float lo[3] = {3.4e38f, 3.4e38f, 3.4e38f}, hi[3] = {-3.4e38f, -3.4e38f, -3.4e38f};
-        for (int v = 0; v < 3; ++v) {
-            const float3 p = load_vertex(verts, __ldg(idx + 3 * t + v));
-            lo[0] = fminf(lo[0], p.x); lo[1] = fminf(lo[1], p.y); lo[2] = fminf(lo[2], p.z);
-            hi[0] = fmaxf(hi[0], p.x); hi[1] = fmaxf(hi[1], p.y); hi[2] = fmaxf(hi[2], p.z);
-        }
-        for (int off = 1; off < G; off <<= 1)
-            for (int d = 0; d < 3; ++d) {
-                lo[d] = fminf(lo[d], __shfl_xor_sync(0xFFFFFFFFu, lo[d], off));
-                hi[d] = fmaxf(hi[d], __shfl_xor_sync(0xFFFFFFFFu, hi[d], off));
+    if (blockIdx.x == 0 && threadIdx.x < 6) P.bounds[threadIdx.x] = 0xFFFFFFFFu;
+    if (blockIdx.x == 0 && threadIdx.x < 4) P.zero[threadIdx.x] = 0ull;
+    for (int64_t w = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); w < n_words; w += warps) {
+        const int64_t c = w * 32 + lane;
+        const bool in = c < n_chunks;
+        const int64_t i0 = c * 32, i1 = min(i0 + 32, P.nt) - 1;
+        // the chunk's object(s) o0, o1: whole 1 one object, 2 two adjacent ones, 0 unknown
+        int32_t o0 = -1, o1 = -1;
+        int whole = 0;
+        bool dead = !in;
+        if (P.obj_range) {
+            const int32_t os = __ldg(P.t2o + w * 1024), oe = __ldg(P.t2o + min(w * 1024 + 1024, P.nt) - 1);
+            bool known = os == oe;
+            int64_t edge = P.nt;
+            if (!known && os >= 0 && oe >= 0) {
+                const int2 rs = __ldg(P.obj_range + os);
+                edge = __ldg(&P.obj_range[oe].x);
+                known = (int64_t)rs.x + rs.y == edge;
             }
-        if (lane % G == 0) {
-            const int64_t g = k * (32 / G) + lane / G;
-            float* b = gbox + 6 * g;
+            if (known) {
+                o0 = i0 < edge ? os : oe;
+                o1 = i1 < edge ? os : oe;
+                whole = o0 == o1 ? 1 : 2;
+            } else if (in) {
+                o0 = __ldg(P.t2o + i0);
+                o1 = __ldg(P.t2o + i1);
+                whole = o0 == o1 ? 1 : 0;
+                if (!whole && o0 >= 0 && o1 >= 0 && P.obj_part) {
+                    const int2 r = __ldg(P.obj_range + o0);
+                    if ((int64_t)r.x + r.y == __ldg(&P.obj_range[o1].x)) whole = 2;
+                }
+            }
+            dead = dead || (whole == 1 && (o0 < 0 || __ldg(P.active + o0) == 0));
+        }
+        if (in) {
+            if (P.mask_bytes == 1) static_cast<uint8_t*>(P.masks)[c] = 0;
+            else if (P.mask_bytes == 2) static_cast<uint16_t*>(P.masks)[c] = 0;
+            else static_cast<uint32_t*>(P.masks)[c] = 0;
+        }
+        if (!__any_sync(0xFFFFFFFFu, !dead)) continue;
+        float3 lo = make_float3(0, 0, 0), hi = make_float3(0, 0, 0);
+        bool live = false, act = false;
+        int32_t part = 0;
+        if (!dead) {
+            const float* b = P.chunk_box + 6 * c;
+            lo = make_float3(__ldg(b), __ldg(b + 1), __ldg(b + 2));
+            hi = make_float3(__ldg(b + 3), __ldg(b + 4), __ldg(b + 5));
+            live = lo.x <= hi.x;
+            if (live && P.obj_part) {
+                // a chunk that may span partitions stays
+                act = true;
+                if (whole != 0 && o0 >= 0 && o1 >= 0) {
+                    part = __ldg(P.obj_part + o0);
+                    act = __ldg(P.obj_part + o1) != part;
+                }
+                live = !act;
+            }
+        }
+        act = cull_query(P, W, live, part, lo, hi) || act;
+        const unsigned m = __ballot_sync(0xFFFFFFFFu, act);
+        if (!m) continue;
+        unsigned long long at = 0;
+        if (lane == 0) at = atomicAdd(P.chunk_count, (unsigned long long)__popc(m));
+        at = __shfl_sync(0xFFFFFFFFu, at, 0);
+        if (act) P.chunk_list[at + __popc(m & ((1u << lane) - 1u))] = (uint32_t)c;
+    }
+}
+
+template <int G>
+__global__ void __launch_bounds__(128) k_cull_groups(CullParams P) {
+    constexpr int PER = 32 / G;  // groups per chunk; G chunks' groups fill a warp
+    __shared__ WarpBoxes boxes[4];
+    WarpBoxes& W = boxes[threadIdx.x >> 5];
+    typename GroupMask<G>::type* masks = static_cast<typename GroupMask<G>::type*>(P.masks);
+    const int lane = threadIdx.x & 31;
+    const int64_t n = (int64_t)*P.chunk_count;
+    const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+    for (int64_t b = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); b * G < n; b += warps) {
+        // lane q's chunk of the batch
+        const int64_t mine = lane < G && b * G + lane < n ? (int64_t)__ldg(P.chunk_list + b * G + lane) : -1;
+        float3 glo = make_float3(0, 0, 0), ghi = make_float3(0, 0, 0);
+        int32_t gpart = 0;
+        bool have = false;
+#pragma unroll
+        for (int q = 0; q < G; ++q) {
+            const int64_t c = __shfl_sync(0xFFFFFFFFu, mine, q);
+            if (c < 0) continue;
+            const int64_t t = group_item(c, lane / G, G, lane % G, P.nt);
+            float lo[3] = {3.4e38f, 3.4e38f, 3.4e38f}, hi[3] = {-3.4e38f, -3.4e38f, -3.4e38f};
+            for (int v = 0; v < 3; ++v) {
+                const float3 p = load_vertex(P.verts, __ldg(P.idx + 3 * t + v));
+                lo[0] = fminf(lo[0], p.x); lo[1] = fminf(lo[1], p.y); lo[2] = fminf(lo[2], p.z);
+                hi[0] = fmaxf(hi[0], p.x); hi[1] = fmaxf(hi[1], p.y); hi[2] = fmaxf(hi[2], p.z);
+            }
+            int32_t part = 0;
+            if (P.obj_part) {
+                const int32_t o = __ldg(P.t2o + t);
+                part = o >= 0 ? __ldg(P.obj_part + o) : -1;
+                const int32_t p0 = __shfl_sync(0xFFFFFFFFu, part, lane & ~(G - 1));
+                if (__any_sync(0xFFFFFFFFu, part != p0) && lane == 0) atomicOr(P.mixed, 1);
+            }
+#pragma unroll
+            for (int off = 1; off < G; off <<= 1)
+                for (int d = 0; d < 3; ++d) {
+                    lo[d] = fminf(lo[d], __shfl_xor_sync(0xFFFFFFFFu, lo[d], off));
+                    hi[d] = fmaxf(hi[d], __shfl_xor_sync(0xFFFFFFFFu, hi[d], off));
+                }
+            const int src = (lane % PER) * G;
+            const float l0 = __shfl_sync(0xFFFFFFFFu, lo[0], src), l1 = __shfl_sync(0xFFFFFFFFu, lo[1], src),
+                        l2 = __shfl_sync(0xFFFFFFFFu, lo[2], src), h0 = __shfl_sync(0xFFFFFFFFu, hi[0], src),
+                        h1 = __shfl_sync(0xFFFFFFFFu, hi[1], src), h2 = __shfl_sync(0xFFFFFFFFu, hi[2], src);
+            const int32_t p = __shfl_sync(0xFFFFFFFFu, part, src);
+            if (lane / PER == q) {
+                glo = make_float3(l0, l1, l2);
+                ghi = make_float3(h0, h1, h2);
+                gpart = p;
+                have = true;
+            }
+        }
+        bool keep = have;
+        if (P.filter) {
+            const bool query = have && glo.x <= ghi.x;
+            const bool hit = cull_query(P, W, query, gpart, glo, ghi);
+            if (query) keep = hit;
+        }
+        const unsigned r = __ballot_sync(0xFFFFFFFFu, keep);
+        if (mine >= 0)
+            masks[mine] = (typename GroupMask<G>::type)(PER == 32 ? r : (r >> (lane * (PER & 31))) & ((1u << (PER & 31)) - 1u));
+    }
+}
+
+// Kept groups in order: list[k] = chunk * (32 / G) + group.  One pass: a tile
+// of 2,048 chunks per block, its place from the tiles before it (decoupled
+// look-back over status words: count << 2 | 1 own count, | 2 count up to and
+// with the tile).  Tiles are taken in ticket order, so a block only waits for
+// blocks that already run; a wait that runs out sets the error word.
+constexpr int kListTile = 2048;
+template <int G>
+__global__ void __launch_bounds__(256) k_list_groups(const void* __restrict__ masks_in, int64_t n_chunks,
+                                                     unsigned long long* status, unsigned int* ticket,
+                                                     uint32_t* __restrict__ list, unsigned long long* total,
+                                                     uint32_t* err) {
+    constexpr int PER = 32 / G;
+    const typename GroupMask<G>::type* masks = static_cast<const typename GroupMask<G>::type*>(masks_in);
+    __shared__ unsigned int s_tile;
+    __shared__ uint32_t s_warp[8];
+    __shared__ unsigned long long s_before;
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    if (tid == 0) s_tile = atomicAdd(ticket, 1u);
+    __syncthreads();
+    const int64_t tile = s_tile, tiles = (n_chunks + kListTile - 1) / kListTile;
+    const int64_t c0 = tile * kListTile + tid * 8;
+    uint32_t mask[8];
+    uint32_t count = 0;
+    if (c0 + 8 <= n_chunks) {
+        // 8, 16 or 32 bytes: masks start a buffer and c0 is a multiple of 8
+        constexpr int kWords = 8 * (int)sizeof(typename GroupMask<G>::type) / 8;
+        constexpr int kBits = 8 * (int)sizeof(typename GroupMask<G>::type);
+        const unsigned long long* v = reinterpret_cast<const unsigned long long*>(masks + c0);
+#pragma unroll
+        for (int q = 0; q < kWords; ++q) {
+            const unsigned long long x = __ldg(v + q);
+#pragma unroll
+            for (int k = 0; k < 8 / kWords; ++k)
+                mask[q * (8 / kWords) + k] = (uint32_t)(x >> (k * kBits)) & (kBits == 32 ? ~0u : (1u << (kBits & 31)) - 1u);
+        }
+    } else {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) mask[k] = c0 + k < n_chunks ? (uint32_t)masks[c0 + k] : 0u;
+    }
+#pragma unroll
+    for (int k = 0; k < 8; ++k) count += __popc(mask[k]);
+    uint32_t incl = count;
+    for (int off = 1; off < 32; off <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, incl, off);
+        if (lane >= off) incl += v;
+    }
+    if (lane == 31) s_warp[w] = incl;
+    __syncthreads();
+    uint32_t before = 0, all = 0;
+    for (int q = 0; q < 8; ++q) {
+        if (q < w) before += s_warp[q];
+        all += s_warp[q];
+    }
+    if (w == 0) {
+        volatile unsigned long long* vs = status;
+        if (lane == 0) {
+            __threadfence();
+            vs[tile] = ((unsigned long long)all << 2) | (tile == 0 ? 2ull : 1ull);
+        }
+        unsigned long long prefix = 0;
+        int64_t at = tile - 1;  // the nearest tile not yet counted
+        bool failed = false;
+        while (at >= 0 && !failed) {
+            // 32 tiles back at a time; lane 0 the nearest
+            const int64_t t = at - lane;
+            unsigned long long v = 2ull;  // before the first tile: nothing
+            int polls = 0;
+            if (t >= 0)
+                while (((v = vs[t]) & 3ull) == 0 && ++polls < (1 << 20)) {}
+            failed = __any_sync(0xFFFFFFFFu, (v & 3ull) == 0);
+            const unsigned done = __ballot_sync(0xFFFFFFFFu, (v & 3ull) == 2ull);
+            const int stop = done ? __ffs(done) - 1 : 31;
+            unsigned long long add = lane <= stop ? v >> 2 : 0ull;
+            for (int off = 16; off > 0; off >>= 1) add += __shfl_xor_sync(0xFFFFFFFFu, add, off);
+            prefix += add;
+            if (done) break;
+            at -= 32;
+        }
+        if (lane == 0) {
+            if (failed) atomicOr(err, ERR_QUEUE_TIMEOUT);
+            __threadfence();
+            vs[tile] = ((prefix + all) << 2) | 2ull;
+            s_before = failed ? ~0ull : prefix;
+            if (tile == tiles - 1) *total = failed ? 0ull : prefix + all;
+        }
+    }
+    __syncthreads();
+    if (s_before == ~0ull) return;
+    unsigned long long pos = s_before + before + (incl - count);
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+        for (uint32_t b = mask[k]; b; b &= b - 1) list[pos++] = (uint32_t)((c0 + k) * PER + __ffs(b) - 1);
+}
+
+// Kept groups -> boxes, box centres (w: partition) and the centres' bounds
+// (ordered integers; the maxima stored inverted, so that all six start as all
+// ones).  One thread per group.
+template <int G, bool PARTS>
+__global__ void __launch_bounds__(256) k_group_prims(const float* __restrict__ verts, const uint32_t* __restrict__ idx,
+                                                     const int32_t* __restrict__ t2o, int64_t nt,
+                                                     const uint32_t* __restrict__ list,
+                                                     const unsigned long long* __restrict__ count,
+                                                     const int32_t* __restrict__ obj_part, float* __restrict__ gbox,
+                                                     float4* __restrict__ cen, uint32_t* __restrict__ bounds) {
+    constexpr int PER = 32 / G;
+    const int64_t n = (int64_t)*count;
+    float mn[3] = {3.4e38f, 3.4e38f, 3.4e38f}, mx[3] = {-3.4e38f, -3.4e38f, -3.4e38f};
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t base = blockIdx.x * (int64_t)blockDim.x; base < n; base += stride) {
+        const int64_t j = base + threadIdx.x;
+        int32_t part = -1;
+        float m[3] = {0.0f, 0.0f, 0.0f};
+        if (j < n) {
+            const uint32_t g = __ldg(list + j);
+            float lo[3] = {3.4e38f, 3.4e38f, 3.4e38f}, hi[3] = {-3.4e38f, -3.4e38f, -3.4e38f};
+#pragma unroll
+            for (int k = 0; k < G; ++k) {
+                const int64_t t = group_item(g / PER, (int)(g % PER), G, k, nt);
+#pragma unroll
+                for (int v = 0; v < 3; ++v) {
+                    const float3 p = load_vertex(verts, __ldg(idx + 3 * t + v));
+                    lo[0] = fminf(lo[0], p.x); lo[1] = fminf(lo[1], p.y); lo[2] = fminf(lo[2], p.z);
+                    hi[0] = fmaxf(hi[0], p.x); hi[1] = fmaxf(hi[1], p.y); hi[2] = fmaxf(hi[2], p.z);
+                }
+            }
+            float* b = gbox + 6 * j;
             b[0] = lo[0]; b[1] = lo[1]; b[2] = lo[2];
             b[3] = hi[0]; b[4] = hi[1]; b[5] = hi[2];
-            gidx[3 * g] = (uint32_t)(2 * g);
-            gidx[3 * g + 1] = (uint32_t)(2 * g + 1);
-            gidx[3 * g + 2] = (uint32_t)(2 * g + 1);
-            gt2o[g] = __ldg(t2o + t);
+            if (cen) {
+                for (int d = 0; d < 3; ++d) m[d] = 0.5f * lo[d] + 0.5f * hi[d];
+                if (PARTS) part = __ldg(obj_part + __ldg(t2o + group_item(g / PER, (int)(g % PER), G, 0, nt)));
+                cen[j] = make_float4(m[0], m[1], m[2], __int_as_float(part));
+                for (int d = 0; d < 3; ++d) {
+                    mn[d] = fminf(mn[d], m[d]);
+                    mx[d] = fmaxf(mx[d], m[d]);
+                }
+            }
+        }
+        if (PARTS && cen) {
+            // per partition: lanes of one partition together
+            const int32_t p0 = __shfl_sync(0xFFFFFFFFu, part, 0);
+            if (p0 >= 0 && __all_sync(0xFFFFFFFFu, part == p0 || part < 0)) {
+                for (int d = 0; d < 3; ++d) {
+                    float a = part < 0 ? 3.4e38f : m[d], b = part < 0 ? -3.4e38f : m[d];
+                    for (int off = 16; off > 0; off >>= 1) {
+                        a = fminf(a, __shfl_xor_sync(0xFFFFFFFFu, a, off));
+                        b = fmaxf(b, __shfl_xor_sync(0xFFFFFFFFu, b, off));
+                    }
+                    if ((threadIdx.x & 31) == 0) {
+                        atomicMin(bounds + 6 * (int64_t)p0 + d, f2o(a));
+                        atomicMin(bounds + 6 * (int64_t)p0 + 3 + d, ~f2o(b));
+                    }
+                }
+            } else if (part >= 0) {
+                for (int d = 0; d < 3; ++d) {
+                    atomicMin(bounds + 6 * (int64_t)part + d, f2o(m[d]));
+                    atomicMin(bounds + 6 * (int64_t)part + 3 + d, ~f2o(m[d]));
+                }
+            }
+        }
+    }
+    if (PARTS || !cen) return;
+    __shared__ float red[2][3][8];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    for (int d = 0; d < 3; ++d)
+        for (int off = 16; off > 0; off >>= 1) {
+            mn[d] = fminf(mn[d], __shfl_xor_sync(0xFFFFFFFFu, mn[d], off));
+            mx[d] = fmaxf(mx[d], __shfl_xor_sync(0xFFFFFFFFu, mx[d], off));
+        }
+    if (lane == 0)
+        for (int d = 0; d < 3; ++d) {
+            red[0][d][wid] = mn[d];
+            red[1][d][wid] = mx[d];
+        }
+    __syncthreads();
+    if (threadIdx.x < 3) {
+        float a = red[0][threadIdx.x][0], b = red[1][threadIdx.x][0];
+        for (int q = 1; q < 8; ++q) {
+            a = fminf(a, red[0][threadIdx.x][q]);
+            b = fmaxf(b, red[1][threadIdx.x][q]);
+        }
+        if (a <= b) {
+            atomicMin(bounds + threadIdx.x, f2o(a));
+            atomicMin(bounds + 3 + threadIdx.x, ~f2o(b));
         }
     }
 }
 
-// Triangle soup in group leaf order: leaf position j takes group g (its
-// original index, stored by k_soup in the group soup), G triangles each.
-__global__ void __launch_bounds__(256) k_group_soup(const float4* __restrict__ gsoup, int64_t n_groups, int G,
-                                                    const uint32_t* __restrict__ chunk_list,
+// Triangle soup of kept groups, G triangles each: position j holds group
+// list[order[j]] (a hierarchy's leaf order), or list[j] without an order.
+__global__ void __launch_bounds__(256) k_group_soup(const uint32_t* __restrict__ list,
+                                                    const uint32_t* __restrict__ order,
+                                                    const unsigned long long* __restrict__ count, int G,
                                                     const float* __restrict__ verts, const uint32_t* __restrict__ idx,
                                                     const int32_t* __restrict__ t2o, int64_t nt,
                                                     float4* __restrict__ soup) {
     const int per_chunk = 32 / G;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n_groups * G;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t j = i / G;
-        const int64_t g = __float_as_int(__ldg(&gsoup[3 * j + 1].w));
-        const int64_t c = chunk_list[g / per_chunk];
-        const int64_t t = group_item(c, (int)(g % per_chunk), G, (int)(i % G), nt);
-        const float3 a = load_vertex(verts, __ldg(idx + 3 * t));
-        const float3 b = load_vertex(verts, __ldg(idx + 3 * t + 1));
-        const float3 cc = load_vertex(verts, __ldg(idx + 3 * t + 2));
-        soup[3 * i + 0] = make_float4(a.x, a.y, a.z, __int_as_float(__ldg(t2o + t)));
-        soup[3 * i + 1] = make_float4(b.x, b.y, b.z, __int_as_float((int)t));
-        soup[3 * i + 2] = make_float4(cc.x, cc.y, cc.z, 0.0f);
-    }
-}
-
-// The kept groups' triangles in list order (no hierarchy: the walking side of
-// a join by triangle pairs), G per group; the kept count stays on the device.
-__global__ void __launch_bounds__(256) k_unit_soup(const uint32_t* __restrict__ glist,
-                                                   const unsigned long long* __restrict__ count, int G,
-                                                   const uint32_t* __restrict__ chunk_list,
-                                                   const float* __restrict__ verts, const uint32_t* __restrict__ idx,
-                                                   const int32_t* __restrict__ t2o, int64_t nt,
-                                                   float4* __restrict__ soup) {
-    const int per_chunk = 32 / G;
     const int64_t n = (int64_t)*count * G;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t g = __ldg(glist + i / G);
-        const int64_t t = group_item(chunk_list[g / per_chunk], (int)(g % per_chunk), G, (int)(i % G), nt);
+        const int64_t j = i / G;
+        const uint32_t g = __ldg(list + (order ? __ldg(order + j) : (uint32_t)j));
+        const int64_t t = group_item(g / per_chunk, (int)(g % per_chunk), G, (int)(i % G), nt);
         const float3 a = load_vertex(verts, __ldg(idx + 3 * t));
         const float3 b = load_vertex(verts, __ldg(idx + 3 * t + 1));
         const float3 c = load_vertex(verts, __ldg(idx + 3 * t + 2));
         soup[3 * i + 0] = make_float4(a.x, a.y, a.z, __int_as_float(__ldg(t2o + t)));
         soup[3 * i + 1] = make_float4(b.x, b.y, b.z, __int_as_float((int)t));
         soup[3 * i + 2] = make_float4(c.x, c.y, c.z, 0.0f);
+    }
+}
+
+// Leaf wave of a hierarchy over boxes with one box per leaf.
+__global__ void __launch_bounds__(256) k_refit_boxes(const float* __restrict__ gbox, const uint32_t* __restrict__ order,
+                                                     int64_t n, Node* nodes,
+                                                     const unsigned long long* __restrict__ leaf_rec,
+                                                     uint32_t* list_out, unsigned long long* count_out) {
+    for (int64_t base = blockIdx.x * (int64_t)blockDim.x; base < n; base += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t j = base + threadIdx.x;
+        bool done = false;
+        uint32_t node = 0;
+        if (j < n) {
+            const unsigned long long rec = leaf_rec[j];
+            node = (uint32_t)(rec >> 9);
+            const float* b = gbox + 6 * (int64_t)__ldg(order + j);
+            const float lo[3] = {__ldg(b), __ldg(b + 1), __ldg(b + 2)}, hi[3] = {__ldg(b + 3), __ldg(b + 4), __ldg(b + 5)};
+            if ((int64_t)node < n - 1) done = deliver(nodes, node, (int)((rec >> 8) & 1), lo, hi);
+        }
+        block_append(done, node, list_out, count_out);
     }
 }
 
@@ -1001,7 +1358,7 @@ __global__ void k_group_leaves(Node* nodes, int64_t num_nodes, int G) {
 // never read).
 __device__ __forceinline__ void node4_half(const Node* __restrict__ nodes, int64_t n, const float4& bx,
                                            const float4& by, const float4& bz, const int4& c, int side,
-                                           float (&lo)[3][2], float (&hi)[3][2], int (&ch)[2], int (&cnt)[2]) {
+                                           float (&lo)[3][2], float (&hi)[3][2], int (&ch)[2], int (&cnt)[2], int G) {
     const int r = side ? c.y : c.x;
     if (r >= 0 && (int64_t)r >= n) {
         for (int j = 0; j < 2; ++j) {
@@ -1018,8 +1375,8 @@ __device__ __forceinline__ void node4_half(const Node* __restrict__ nodes, int64
         lo[0][0] = side ? bx.z : bx.x; hi[0][0] = side ? bx.w : bx.y;
         lo[1][0] = side ? by.z : by.x; hi[1][0] = side ? by.w : by.y;
         lo[2][0] = side ? bz.z : bz.x; hi[2][0] = side ? bz.w : bz.y;
-        ch[0] = r;
-        cnt[0] = (c.z >> (8 * side)) & 0xFF;
+        ch[0] = ~(~r * G);
+        cnt[0] = ((c.z >> (8 * side)) & 0xFF) * G;
         for (int k = 0; k < 3; ++k) {
             lo[k][1] = 3.4e38f;
             hi[k][1] = -3.4e38f;
@@ -1033,20 +1390,23 @@ __device__ __forceinline__ void node4_half(const Node* __restrict__ nodes, int64
     lo[0][0] = gx.x; hi[0][0] = gx.y; lo[0][1] = gx.z; hi[0][1] = gx.w;
     lo[1][0] = gy.x; hi[1][0] = gy.y; lo[1][1] = gy.z; hi[1][1] = gy.w;
     lo[2][0] = gz.x; hi[2][0] = gz.y; lo[2][1] = gz.z; hi[2][1] = gz.w;
-    ch[0] = gc.x;
-    ch[1] = gc.y;
-    cnt[0] = gc.z & 0xFF;
-    cnt[1] = (gc.z >> 8) & 0xFF;
+    ch[0] = gc.x < 0 ? ~(~gc.x * G) : gc.x;
+    ch[1] = gc.y < 0 ? ~(~gc.y * G) : gc.y;
+    cnt[0] = (gc.z & 0xFF) * G;
+    cnt[1] = ((gc.z >> 8) & 0xFF) * G;
 }
 
-__global__ void __launch_bounds__(256) k_collapse4(const Node* __restrict__ nodes, int64_t n, Node4* __restrict__ out) {
+// G: soup triangles per leaf item (a group hierarchy's leaves become soup
+// ranges of G; 1: the nodes' own leaf ranges).
+__global__ void __launch_bounds__(256) k_collapse4(const Node* __restrict__ nodes, int64_t n, Node4* __restrict__ out,
+                                                   int G) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         const float4 bx = __ldg(&nodes[i].bx), by = __ldg(&nodes[i].by), bz = __ldg(&nodes[i].bz);
         const int4 c = __ldg(&nodes[i].ch);
         float lo0[3][2], hi0[3][2], lo1[3][2], hi1[3][2];
         int ch0[2], ch1[2], n0[2], n1[2];
-        node4_half(nodes, n, bx, by, bz, c, 0, lo0, hi0, ch0, n0);
-        node4_half(nodes, n, bx, by, bz, c, 1, lo1, hi1, ch1, n1);
+        node4_half(nodes, n, bx, by, bz, c, 0, lo0, hi0, ch0, n0, G);
+        node4_half(nodes, n, bx, by, bz, c, 1, lo1, hi1, ch1, n1, G);
         Node4 q;
         q.lox = make_float4(lo0[0][0], lo0[0][1], lo1[0][0], lo1[0][1]);
         q.hix = make_float4(hi0[0][0], hi0[0][1], hi1[0][0], hi1[0][1]);
@@ -1060,39 +1420,11 @@ __global__ void __launch_bounds__(256) k_collapse4(const Node* __restrict__ node
     }
 }
 
-int collapse4(pierce_ctx* ctx, const Node* nodes, int64_t num_nodes, Node4* out) {
+int collapse4(pierce_ctx* ctx, const Node* nodes, int64_t num_nodes, Node4* out, int G) {
     if (num_nodes <= 0) return PIERCE_OK;
-    k_collapse4<<<grid_for(ctx, num_nodes, 256), 256, 0, ctx->stream>>>(nodes, num_nodes, out);
+    k_collapse4<<<grid_for(ctx, num_nodes, 256), 256, 0, ctx->stream>>>(nodes, num_nodes, out, G);
     ctx->launches += 1;
     return check_cuda(cudaGetLastError(), "collapse to four-wide nodes");
-}
-
-// Partitioned datasets: does any group of G triangles of a flagged chunk
-// (every chunk when chunk_flags is null) hold triangles of two partitions?
-// (Then the join builds over triangles.)
-__global__ void __launch_bounds__(256) k_group_mixed(const uint8_t* __restrict__ chunk_flags, int64_t n_chunks,
-                                                     const int32_t* __restrict__ t2o,
-                                                     const int32_t* __restrict__ obj_part, int64_t nt, int G,
-                                                     int32_t* mixed) {
-    const int lane = threadIdx.x & 31;
-    const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-    for (int64_t c = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); c < n_chunks; c += warps) {
-        if (chunk_flags && !chunk_flags[c]) continue;  // warp-uniform
-        const int64_t t = group_item(c, lane / G, G, lane % G, nt);
-        const int32_t o = __ldg(t2o + t);
-        const int32_t p = o >= 0 ? __ldg(obj_part + o) : -1;
-        const int32_t p0 = __shfl_sync(0xFFFFFFFFu, p, lane & ~(G - 1));
-        if (__any_sync(0xFFFFFFFFu, p != p0) && lane == 0) atomicOr(mixed, 1);
-    }
-}
-
-int launch_group_mixed(pierce_ctx* ctx, const uint8_t* chunk_flags, int64_t n_chunks, const int32_t* t2o,
-                       const int32_t* obj_part, int64_t nt, int G, int32_t* mixed) {
-    if (n_chunks <= 0) return PIERCE_OK;
-    k_group_mixed<<<grid_for(ctx, n_chunks * 32, 256), 256, 0, ctx->stream>>>(chunk_flags, n_chunks, t2o, obj_part,
-                                                                             nt, G, mixed);
-    ctx->launches += 1;
-    return check_cuda(cudaGetLastError(), "group partition check");
 }
 
 // Partition roots of a group hierarchy: a root leaf of one group becomes the
@@ -1105,120 +1437,173 @@ __global__ void k_group_roots(int2* roots, int32_t num_parts, int G) {
     }
 }
 
-int build_grouped_lbvh(pierce_ctx* ctx, const float* verts, const uint32_t* idx, const int32_t* t2o, int64_t nt,
-                       const uint32_t* chunk_list, int64_t n_chunks, int G, void* group_scratch, float4* soup,
-                       Node* nodes, BvhShape* shape, const DevDataset* filter, unsigned long long* d_count,
-                       int64_t* kept, const int32_t* obj_part, int32_t num_parts, int2* part_roots) {
-    cudaStream_t st = ctx->stream;
-    const int64_t ng = n_chunks * (32 / G);
-    shape->leaf_size = G;
-    const bool parts = obj_part && num_parts > 0 && part_roots;
-    if (ng == 0) {
-        shape->root_is_leaf = 1;
-        shape->root_leaf_count = 0;
-        shape->num_nodes = 0;
-        if (kept) *kept = 0;
-        if (parts) {
-            k_fill_roots<<<grid_for(ctx, num_parts, 256), 256, 0, st>>>(part_roots, num_parts);
-            ctx->launches += 1;
-        }
-        return check_cuda(cudaGetLastError(), "grouped bvh build");
-    }
-    if (ng * G >= (int64_t(1) << 30))
-        return set_error(PIERCE_ERR_INVALID_ARGUMENT, "bvh build: at most 2^30 - 1 triangles per hierarchy");
-    // group scratch: soup 48, boxes 24, pseudo indices 12, ids 4, filter flags 1
-    // and kept-group list 4 bytes per group
-    char* q = static_cast<char*>(group_scratch);
-    float4* gsoup = reinterpret_cast<float4*>(q);
-    float* gbox = reinterpret_cast<float*>(q + 48 * ng);
-    uint32_t* gidx = reinterpret_cast<uint32_t*>(q + 72 * ng);
-    int32_t* gt2o = reinterpret_cast<int32_t*>(q + 84 * ng);
-    const int64_t warps = n_chunks;
-    k_group_boxes<<<(unsigned)std::max<int64_t>(1, std::min<int64_t>((warps + 7) / 8, (int64_t)ctx->sm_count * 16)),
-                    256, 0, st>>>(verts, idx, t2o, nt, chunk_list, n_chunks, G, gbox, gidx, gt2o);
-    ctx->launches += 1;
-    // optional filter: keep the groups that can meet the other side
-    const uint32_t* list = nullptr;
-    int64_t n = ng;
-    if (filter) {
-        uint8_t* flags = reinterpret_cast<uint8_t*>(q + 88 * ng);
-        char* lq = q + 88 * ng + ng;
-        lq += (256 - ((uintptr_t)lq & 255)) & 255;
-        uint32_t* glist = reinterpret_cast<uint32_t*>(lq);
-        if (int s = launch_group_filter(ctx, gbox, ng, *filter, parts ? gt2o : nullptr, obj_part, flags)) return s;
-        if (int s = select_flagged(ctx, flags, ng, glist, d_count)) return s;
-        if (int s = host_value(ctx, d_count, 8, &n, "kept groups")) return s;
-        list = glist;
-    }
-    if (kept) *kept = n;
-    if (n == 0) {
-        shape->root_is_leaf = 1;
-        shape->root_leaf_count = 0;
-        shape->num_nodes = 0;
-        if (parts) {
-            k_fill_roots<<<grid_for(ctx, num_parts, 256), 256, 0, st>>>(part_roots, num_parts);
-            ctx->launches += 1;
-        }
-        return check_cuda(cudaGetLastError(), "grouped bvh build");
-    }
-    BvhShape gshape;
-    if (int s = build_lbvh(ctx, gbox, gidx, gt2o, list, n, 1, gsoup, nodes, &gshape, nullptr,
-                           parts ? obj_part : nullptr, parts ? num_parts : 0, parts ? part_roots : nullptr))
-        return s;
-    k_group_soup<<<grid_for(ctx, n * G, 256), 256, 0, st>>>(gsoup, n, G, chunk_list, verts, idx, t2o, nt, soup);
-    ctx->launches += 1;
-    if (gshape.root_is_leaf) {
-        shape->root_is_leaf = 1;
-        shape->root_leaf_count = (int)(gshape.root_leaf_count * G);
-        shape->num_nodes = 0;
-    } else {
-        k_group_leaves<<<grid_for(ctx, (int64_t)gshape.num_nodes, 256), 256, 0, st>>>(nodes,
-                                                                                     (int64_t)gshape.num_nodes, G);
-        ctx->launches += 1;
-    }
-    if (parts) {
-        k_group_roots<<<grid_for(ctx, num_parts, 256), 256, 0, st>>>(part_roots, num_parts, G);
-        ctx->launches += 1;
-    }
-    if (!gshape.root_is_leaf) {
-        shape->root_is_leaf = 0;
-        shape->root_leaf_count = 0;
-        shape->num_nodes = gshape.num_nodes;
-    }
-    return check_cuda(cudaGetLastError(), "grouped bvh build");
+// chunk masks, the chunk list, then words cleared together: chunk count, the
+// list pass's ticket and tile status words
+static size_t mask_bytes(int G) { return G >= 4 ? 1 : G == 2 ? 2 : 4; }
+size_t group_cull_bytes(int64_t nt, int G) {
+    const size_t chunks = (size_t)((nt + 31) / 32), tiles = chunks / kListTile + 2;
+    return chunks * (mask_bytes(G) + 4) + 1024 + 8 * tiles;
 }
 
-// The walking side of a join by triangle pairs: the groups of G consecutive
-// triangles of the listed chunks whose box meets a leaf item of `filter`, as
-// a soup in list order with their boxes (gbox[6 g] of group g = glist[j]).
-// The number kept stays in *d_count; group_scratch as build_grouped_lbvh's.
-int build_group_units(pierce_ctx* ctx, const float* verts, const uint32_t* idx, const int32_t* t2o, int64_t nt,
-                      const uint32_t* chunk_list, int64_t n_chunks, int G, void* group_scratch, float4* soup,
-                      const DevDataset& filter, unsigned long long* d_count, const int32_t* obj_part,
-                      GroupUnits* out) {
+#define PG_BY_GROUP(CALL) \
+    do {                  \
+        switch (G) {      \
+            case 1: CALL(1); break;   \
+            case 2: CALL(2); break;   \
+            case 4: CALL(4); break;   \
+            case 8: CALL(8); break;   \
+            default: CALL(16); break; \
+        }                 \
+    } while (0)
+
+int cull_groups(pierce_ctx* ctx, const DevDataset& src, const int32_t* t2o, const uint8_t* active,
+                const DevDataset& other, bool filter, int G, void* mem, uint32_t* list, unsigned long long* d_count,
+                int32_t* d_mixed, uint32_t* bounds, unsigned long long* zero) {
     cudaStream_t st = ctx->stream;
-    const int64_t ng = n_chunks * (32 / G);
-    *out = GroupUnits{};
-    out->bound = ng;
-    if (ng == 0) return check_cuda(cudaMemsetAsync(d_count, 0, 8, st), "group units");
-    char* q = static_cast<char*>(group_scratch);
-    float* gbox = reinterpret_cast<float*>(q + 48 * ng);
-    uint32_t* gidx = reinterpret_cast<uint32_t*>(q + 72 * ng);
-    int32_t* gt2o = reinterpret_cast<int32_t*>(q + 84 * ng);
-    k_group_boxes<<<(unsigned)std::max<int64_t>(1, std::min<int64_t>((n_chunks + 7) / 8, (int64_t)ctx->sm_count * 16)),
-                    256, 0, st>>>(verts, idx, t2o, nt, chunk_list, n_chunks, G, gbox, gidx, gt2o);
-    ctx->launches += 1;
-    uint8_t* flags = reinterpret_cast<uint8_t*>(q + 88 * ng);
-    char* lq = q + 88 * ng + ng;
-    lq += (256 - ((uintptr_t)lq & 255)) & 255;
-    uint32_t* glist = reinterpret_cast<uint32_t*>(lq);
-    if (int s = launch_group_filter(ctx, gbox, ng, filter, obj_part ? gt2o : nullptr, obj_part, flags)) return s;
-    if (int s = select_flagged(ctx, flags, ng, glist, d_count)) return s;
-    k_unit_soup<<<grid_for(ctx, ng * G, 256), 256, 0, st>>>(glist, d_count, G, chunk_list, verts, idx, t2o, nt, soup);
-    ctx->launches += 1;
-    out->gbox = gbox;
-    out->glist = glist;
+    const int64_t nt = src.num_tris, chunks = (nt + 31) / 32, tiles = (chunks + kListTile - 1) / kListTile;
+    if (nt <= 0) return check_cuda(cudaMemsetAsync(d_count, 0, 8, st), "cull groups");
+    char* q = static_cast<char*>(mem) + (size_t)chunks * mask_bytes(G);
+    q += (256 - ((uintptr_t)q & 255)) & 255;
+    uint32_t* chunk_list = reinterpret_cast<uint32_t*>(q);
+    q += 4 * (size_t)chunks;
+    q += (256 - ((uintptr_t)q & 255)) & 255;
+    unsigned long long* chunk_count = reinterpret_cast<unsigned long long*>(q);
+    unsigned int* ticket = reinterpret_cast<unsigned int*>(chunk_count + 1);
+    unsigned long long* status = chunk_count + 2;
+    cudaMemsetAsync(chunk_count, 0, 8 * (size_t)(tiles + 2), st);
+    CullParams P;
+    P.verts = src.verts;
+    P.idx = src.idx;
+    P.t2o = t2o;
+    P.nt = nt;
+    P.chunk_box = src.tri_chunk_box;
+    P.obj_range = src.obj_range;
+    P.active = active;
+    P.obj_part = src.obj_part;
+    P.other = other;
+    P.filter = filter ? 1 : 0;
+    P.wide = other.nodes4 && other.num_tris < (int64_t(1) << 27) ? 1 : 0;
+    P.mask_bytes = (int)mask_bytes(G);
+    P.masks = mem;
+    P.chunk_list = chunk_list;
+    P.chunk_count = chunk_count;
+    P.mixed = d_mixed;
+    P.bounds = bounds;
+    P.zero = zero;
+    const int64_t words = (chunks + 31) / 32;
+    const unsigned blocks = (unsigned)std::max<int64_t>(1, std::min<int64_t>((words + 3) / 4, (int64_t)ctx->sm_count * 32));
+    const unsigned gblocks = (unsigned)std::max<int64_t>(1, std::min<int64_t>((chunks + 4 * G - 1) / (4 * G),
+                                                                            (int64_t)ctx->sm_count * 32));
+    k_cull_chunks<<<blocks, 128, 0, st>>>(P);
+#define PG_CULL(g)                                                                                                  \
+    k_cull_groups<g><<<gblocks, 128, 0, st>>>(P);                                                                   \
+    k_list_groups<g><<<(unsigned)tiles, 256, 0, st>>>(mem, chunks, status, ticket, list, d_count, ctx->d_err)
+    PG_BY_GROUP(PG_CULL);
+#undef PG_CULL
+    ctx->launches += 3;
+    return check_cuda(cudaGetLastError(), "cull groups");
+}
+
+int group_units(pierce_ctx* ctx, const DevDataset& src, const int32_t* t2o, const uint32_t* list,
+                const unsigned long long* d_count, int64_t bound, int G, float* gbox, float4* soup) {
+    if (bound <= 0) return PIERCE_OK;
+    cudaStream_t st = ctx->stream;
+#define PG_PRIMS(g)                                                                                                  \
+    k_group_prims<g, false><<<grid_for(ctx, bound, 256), 256, 0, st>>>(src.verts, src.idx, t2o, src.num_tris, list, \
+                                                                       d_count, nullptr, gbox, nullptr, nullptr)
+    PG_BY_GROUP(PG_PRIMS);
+#undef PG_PRIMS
+    k_group_soup<<<grid_for(ctx, bound * G, 256), 256, 0, st>>>(list, nullptr, d_count, G, src.verts, src.idx, t2o,
+                                                                src.num_tris, soup);
+    ctx->launches += 2;
     return check_cuda(cudaGetLastError(), "group units");
+}
+
+int build_group_lbvh(pierce_ctx* ctx, const DevDataset& src, const int32_t* t2o, const uint32_t* list,
+                     const unsigned long long* d_count, int64_t n, int G, uint32_t* bounds,
+                     unsigned long long* wave_count, void* group_scratch, float4* soup, Node* nodes, BvhShape* shape,
+                     int32_t num_parts, int2* part_roots) {
+    cudaStream_t st = ctx->stream;
+    const bool parts = src.obj_part && num_parts > 0 && part_roots;
+    shape->leaf_size = G;
+    shape->root_is_leaf = 1;
+    shape->root_leaf_count = 0;
+    shape->num_nodes = 0;
+    const int B = 256;
+    if (parts) {
+        k_fill_roots<<<grid_for(ctx, num_parts, B), B, 0, st>>>(part_roots, num_parts);
+        ctx->launches += 1;
+    }
+    if (n <= 0) return check_cuda(cudaGetLastError(), "group hierarchy");
+    if (n * G >= (int64_t(1) << 30))
+        return set_error(PIERCE_ERR_INVALID_ARGUMENT, "bvh build: at most 2^30 - 1 triangles per hierarchy");
+    // scratch: 1 centres, 2 keys (in | out), 3 values (in | out), 4 leaf records, root box, partition bounds
+    void *pc = nullptr, *pk = nullptr, *pv = nullptr, *pm = nullptr;
+    const size_t key_bytes = parts ? sizeof(uint64_t) : sizeof(uint32_t);
+    if (int s = scratch(ctx, 1, sizeof(float4) * (size_t)n, &pc)) return s;
+    if (int s = scratch(ctx, 2, 2 * key_bytes * (size_t)(n + 4), &pk)) return s;
+    if (int s = scratch(ctx, 3, 2 * sizeof(uint32_t) * (size_t)n, &pv)) return s;
+    if (int s = scratch(ctx, 4, 8 * (size_t)n + 64 + (parts ? 24 * (size_t)num_parts : 0), &pm)) return s;
+    float4* cen = static_cast<float4*>(pc);
+    uint32_t *keys = static_cast<uint32_t*>(pk), *vals = static_cast<uint32_t*>(pv);
+    uint64_t* keys64 = static_cast<uint64_t*>(pk);
+    unsigned long long* leaf_rec = static_cast<unsigned long long*>(pm);
+    float* d_root_box = reinterpret_cast<float*>(leaf_rec + n);
+    uint32_t* pbounds = reinterpret_cast<uint32_t*>(d_root_box + 16);
+    float* gbox = static_cast<float*>(group_scratch);
+    if (parts) cudaMemsetAsync(pbounds, 0xFF, 24 * (size_t)num_parts, st);
+#define PG_PRIMS(g)                                                                                                    \
+    if (parts)                                                                                                         \
+        k_group_prims<g, true><<<grid_for(ctx, n, B), B, 0, st>>>(src.verts, src.idx, t2o, src.num_tris, list, d_count, \
+                                                                  src.obj_part, gbox, cen, pbounds);                   \
+    else                                                                                                               \
+        k_group_prims<g, false><<<grid_for(ctx, n, B), B, 0, st>>>(src.verts, src.idx, t2o, src.num_tris, list,        \
+                                                                   d_count, nullptr, gbox, cen, bounds)
+    PG_BY_GROUP(PG_PRIMS);
+#undef PG_PRIMS
+    if (parts) {
+        k_morton_parts<<<grid_for(ctx, n, B), B, 0, st>>>(cen, n, pbounds, keys64, vals, 0xFFFFFFFFu);
+        int bits = 0;
+        while (bits < 32 && (1ll << bits) < (int64_t)num_parts) ++bits;
+        if (int s = sort_u64_pairs(ctx, keys64, keys64 + n, vals, vals + n, n, 30 + bits)) return s;
+    } else {
+        k_morton<<<grid_for(ctx, n, B), B, 0, st>>>(cen, n, bounds, keys, vals, 0xFFFFFFFFu);
+        if (int s = sort_u32_pairs(ctx, keys, keys + n, vals, vals + n, n, 30)) return s;
+    }
+    const uint32_t* order = vals + n;
+    k_group_soup<<<grid_for(ctx, n * G, B), B, 0, st>>>(list, order, d_count, G, src.verts, src.idx, t2o, src.num_tris,
+                                                        soup);
+    ctx->launches += 3;
+    if (n == 1) {
+        if (parts) {
+            k_single_part_root<<<1, 1, 0, st>>>(keys64 + n, part_roots);
+            ctx->launches += 1;
+        }
+        shape->root_leaf_count = G;
+    } else {
+        // one group per leaf: every leaf record is written by its parent
+        if (parts)
+            k_karras<uint64_t><<<grid_for(ctx, n - 1, B), B, 0, st>>>(keys64 + n, n, 1, nodes, leaf_rec, part_roots);
+        else
+            k_karras<uint32_t><<<grid_for(ctx, n - 1, B), B, 0, st>>>(keys + n, n, 1, nodes, leaf_rec, nullptr);
+        k_refit_boxes<<<grid_for(ctx, n, B), B, 0, st>>>(gbox, order, n, nodes, leaf_rec, keys, wave_count);
+        ctx->launches += 2;
+        refit_above(ctx, nodes, n, keys, wave_count, d_root_box);
+        shape->root_is_leaf = 0;
+        shape->num_nodes = (uint64_t)(n - 1);
+    }
+    if (parts) {
+        k_group_roots<<<grid_for(ctx, num_parts, B), B, 0, st>>>(part_roots, num_parts, G);
+        ctx->launches += 1;
+    }
+    return check_cuda(cudaGetLastError(), "group hierarchy");
+}
+
+int group_leaves(pierce_ctx* ctx, Node* nodes, int64_t num_nodes, int G) {
+    if (num_nodes <= 0 || G == 1) return PIERCE_OK;
+    k_group_leaves<<<grid_for(ctx, num_nodes, 256), 256, 0, ctx->stream>>>(nodes, num_nodes, G);
+    ctx->launches += 1;
+    return check_cuda(cudaGetLastError(), "group leaves");
 }
 
 int build_bvh(pierce_ctx* ctx, pierce_dataset* ds, int leaf_size) {

@@ -41,8 +41,7 @@ struct PairParams {
     DevDataset a;                         // soup, nodes4, part_roots of A's per-join hierarchy
     const float4* bsoup;                  // B's kept groups, G triangles each
     const unsigned long long* b_count;    // their number
-    const float* gbox;                    // boxes of B's candidate groups ...
-    const uint32_t* glist;                // ... and the kept ones among them
+    const float* gbox;                    // their boxes
     const int32_t* b_part;                // partition per B object (partitioned joins)
     int G;                                // triangles per group, both sides
     PairSet set;
@@ -369,7 +368,7 @@ __global__ void __launch_bounds__(32 * kPairWarps, DEFER ? 6 : 4) k_tri_pairs(Pa
                 uint2 e = make_uint2((uint32_t)(base + lane), 0);
                 if (P.entries) e = P.entries[base + lane];
                 W.unit[lane] = e.x;
-                const float* gb = P.gbox + 6 * (size_t)__ldg(P.glist + e.x);
+                const float* gb = P.gbox + 6 * (size_t)e.x;
 #pragma unroll
                 for (int k = 0; k < 6; ++k) W.box[k][lane] = __ldg(gb + k);
                 if (P.entries) {
@@ -440,8 +439,7 @@ int launch_tri_pairs(pierce_ctx* ctx, const DevDataset& a, const PairJoin& j, co
     P.a = a;
     P.bsoup = j.bsoup;
     P.b_count = j.b_count;
-    P.gbox = j.units.gbox;
-    P.glist = j.units.glist;
+    P.gbox = j.gbox;
     P.b_part = j.b_part;
     P.G = j.G;
     P.set = set;
@@ -451,8 +449,8 @@ int launch_tri_pairs(pierce_ctx* ctx, const DevDataset& a, const PairJoin& j, co
     P.amb_count = j.work;
     P.amb_cap = j.amb_cap;
     P.a_listed = j.a_listed;
-    if (j.units.bound > 0) {
-        const int64_t blocks = std::min<int64_t>((j.units.bound + kPairWarps - 1) / kPairWarps, (int64_t)ctx->sm_count * 8);
+    if (j.b_bound > 0) {
+        const int64_t blocks = std::min<int64_t>((j.b_bound + kPairWarps - 1) / kPairWarps, (int64_t)ctx->sm_count * 8);
         const unsigned grid = (unsigned)std::max<int64_t>(blocks, 1), threads = 32 * kPairWarps;
         // A group's walk is as long as what it meets (a coarse mesh's group
         // meets thousands of leaves of a fine one): a warp leaves what a
@@ -485,7 +483,7 @@ int launch_tri_pairs(pierce_ctx* ctx, const DevDataset& a, const PairJoin& j, co
         }
     }
     if (int s = check_cuda(cudaGetLastError(), "triangle pairs")) return s;
-    return launch_pair_rays(ctx, a.soup, na, j.a_listed, j.bsoup, j.b_count, j.units.bound, j.G);
+    return launch_pair_rays(ctx, a.soup, na, j.a_listed, j.bsoup, j.b_count, j.b_bound, j.G);
 }
 
 // Pair-count bound for output sizing: B's kept groups are taken in runs of
@@ -517,7 +515,7 @@ __global__ void __launch_bounds__(32 * kPairWarps) k_unit_incidences(PairParams 
         const int64_t g = s * step * run + lane;
         int sp = (int)min((int64_t)run, n - s * step * run), ns = 0;
         if (lane < sp) {
-            const float* gb = P.gbox + 6 * (size_t)__ldg(P.glist + g);
+            const float* gb = P.gbox + 6 * (size_t)g;
 #pragma unroll
             for (int k = 0; k < 6; ++k) boxes[w][k][lane] = __ldg(gb + k);
             objs[w][lane] = __float_as_int(__ldg(&P.bsoup[3 * (size_t)g * G].w));
@@ -597,17 +595,16 @@ __global__ void __launch_bounds__(32 * kPairWarps) k_unit_incidences(PairParams 
 int launch_unit_incidences(pierce_ctx* ctx, const DevDataset& a, const PairJoin& j, int step,
                            unsigned long long* count) {
     cudaMemsetAsync(count, 0, sizeof(unsigned long long), ctx->stream);
-    if (j.units.bound <= 0) return check_cuda(cudaGetLastError(), "unit incidences");
+    if (j.b_bound <= 0) return check_cuda(cudaGetLastError(), "unit incidences");
     PairParams P{};
     P.a = a;
     P.bsoup = j.bsoup;
     P.b_count = j.b_count;
-    P.gbox = j.units.gbox;
-    P.glist = j.units.glist;
+    P.gbox = j.gbox;
     P.G = j.G;
     P.err = ctx->d_err;
     const int min_runs = 4096;
-    const int64_t runs = std::max<int64_t>(min_runs, j.units.bound / ((int64_t)step * kPairUnits) + 1);
+    const int64_t runs = std::max<int64_t>(min_runs, j.b_bound / ((int64_t)step * kPairUnits) + 1);
     const int64_t blocks = std::min<int64_t>((runs + kPairWarps - 1) / kPairWarps, (int64_t)ctx->sm_count * 16);
     k_unit_incidences<<<(unsigned)blocks, 32 * kPairWarps, 0, ctx->stream>>>(P, step, min_runs, count);
     ctx->launches += 1;

@@ -1,0 +1,252 @@
+// Box queries over the hierarchies, shared by the culling and ray kernels.
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include "common.cuh"
+#include "hash.cuh"
+
+namespace pgpu {
+
+// Any-hit box query over a Node4 hierarchy from internal node `node`: true
+// as soon as leaf_hit(first, count) is true for a leaf whose box meets
+// [lo, hi] (and, conservatively, if the stack would overflow).
+template <class LeafHit>
+__device__ __forceinline__ bool any_hit4(const Node4* nodes4, int node, const float3& lo, const float3& hi,
+                                         LeafHit&& leaf_hit) {
+    int stack[kStackSize4];
+    int sp = 0;
+    for (;;) {
+        const Node4* nd = nodes4 + node;
+        const float4 lx = __ldg(&nd->lox), hx = __ldg(&nd->hix), ly = __ldg(&nd->loy), hy = __ldg(&nd->hiy);
+        const float4 lz = __ldg(&nd->loz), hz = __ldg(&nd->hiz);
+        const int4 ch = __ldg(&nd->ch);
+        const int cnt = __ldg(&nd->meta.x);
+        const bool h[4] = {box_overlap(lx.x, hx.x, ly.x, hy.x, lz.x, hz.x, lo, hi),
+                           box_overlap(lx.y, hx.y, ly.y, hy.y, lz.y, hz.y, lo, hi),
+                           box_overlap(lx.z, hx.z, ly.z, hy.z, lz.z, hz.z, lo, hi),
+                           box_overlap(lx.w, hx.w, ly.w, hy.w, lz.w, hz.w, lo, hi)};
+        const int c[4] = {ch.x, ch.y, ch.z, ch.w};
+        int next = -1;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            if (!h[j]) continue;
+            if (c[j] < 0) {
+                if (leaf_hit(~c[j], (cnt >> (8 * j)) & 0xFF)) return true;
+            } else if (next < 0) {
+                next = c[j];
+            } else {
+                if (sp >= kStackSize4) return true;
+                stack[sp++] = c[j];
+            }
+        }
+        if (next >= 0) {
+            node = next;
+        } else {
+            if (sp == 0) return false;
+            node = stack[--sp];
+        }
+    }
+}
+
+// Does item t of `h` meet [lo, hi]?  A soup of boxes (degenerate triangles
+// lo, hi, hi) by the box, a soup of triangles by the triangle's box.
+__device__ __forceinline__ bool item_meets_box(const DevDataset& h, int64_t t, const float3& lo, const float3& hi) {
+    const float4 a4 = __ldg(h.soup + 3 * t), b4 = __ldg(h.soup + 3 * t + 1);
+    if (h.soup_boxes) return box_overlap(a4.x, b4.x, a4.y, b4.y, a4.z, b4.z, lo, hi);
+    const float4 c4 = __ldg(h.soup + 3 * t + 2);
+    return box_overlap(fminf(a4.x, fminf(b4.x, c4.x)), fmaxf(a4.x, fmaxf(b4.x, c4.x)),
+                       fminf(a4.y, fminf(b4.y, c4.y)), fmaxf(a4.y, fmaxf(b4.y, c4.y)),
+                       fminf(a4.z, fminf(b4.z, c4.z)), fmaxf(a4.z, fmaxf(b4.z, c4.z)), lo, hi);
+}
+
+// Does leaf [first, first + count) of `h` meet [lo, hi]?
+__device__ __forceinline__ bool leaf_meets_box(const DevDataset& h, int first, int count, const float3& lo,
+                                               const float3& hi) {
+    for (int k = 0; k < count; ++k)
+        if (item_meets_box(h, (int64_t)first + k, lo, hi)) return true;
+    return false;
+}
+
+// Does [lo, hi] meet an item of `objs` within partition `part`?  Items are
+// the boxes of a box hierarchy (object or chunk boxes as degenerate
+// triangles) or the triangles of a per-join hierarchy (by their boxes).
+static __device__ bool meets_any_object(const DevDataset& objs, int32_t part, const float3& lo, const float3& hi) {
+    auto leaf_hit = [&](int first, int count) { return leaf_meets_box(objs, first, count, lo, hi); };
+    int node;
+    if (objs.part_roots) {
+        const int2 r = __ldg(objs.part_roots + part);
+        if (r.x < 0) return leaf_hit(~r.x, r.y);
+        node = r.x;
+    } else if (objs.root_is_leaf) {
+        return leaf_hit(0, objs.root_leaf_count);
+    } else {
+        node = 0;
+    }
+    if (objs.nodes4) return any_hit4(objs.nodes4, node, lo, hi, leaf_hit);
+    int stack[kStackSize];
+    int sp = 0;
+    for (;;) {
+        const Node* nd = objs.nodes + node;
+        const float4 bx = __ldg(&nd->bx), by = __ldg(&nd->by), bz = __ldg(&nd->bz);
+        const int4 ch = __ldg(&nd->ch);
+        bool h0 = box_overlap(bx.x, bx.y, by.x, by.y, bz.x, bz.y, lo, hi);
+        bool h1 = box_overlap(bx.z, bx.w, by.z, by.w, bz.z, bz.w, lo, hi);
+        if (h0 && ch.x < 0) {
+            if (leaf_hit(~ch.x, ch.z & 0xFF)) return true;
+            h0 = false;
+        }
+        if (h1 && ch.y < 0) {
+            if (leaf_hit(~ch.y, (ch.z >> 8) & 0xFF)) return true;
+            h1 = false;
+        }
+        if (h0 && h1) {
+            if (sp >= kStackSize) return true;  // cannot happen for an LBVH; stay conservative
+            stack[sp++] = ch.y;
+            node = ch.x;
+        } else if (h0) {
+            node = ch.x;
+        } else if (h1) {
+            node = ch.y;
+        } else {
+            if (sp == 0) return false;
+            node = stack[--sp];
+        }
+    }
+}
+
+// ---- walks shared by a warp ------------------------------------------------------
+constexpr int kWarpStack = 512;    // entries per warp
+constexpr int kWarpReserve = 144;  // of them left for a single entry's subtree (48 levels x 3)
+constexpr int kAlone = 12;         // nodes a query visits on its own before its walk is shared
+constexpr int kAloneStack = kWarpStack / 32;
+
+struct WarpBoxes {
+    float box[6][32];            // the queries' boxes
+    uint32_t stack[kWarpStack];  // node << 5 | query
+};
+
+// A four-wide node's children that the box [lo, hi] meets: bit j child j.
+__device__ __forceinline__ unsigned node4_meets(const Node4* nd, const float3& lo, const float3& hi, int4& ch) {
+    const float4 lx = __ldg(&nd->lox), hx = __ldg(&nd->hix), ly = __ldg(&nd->loy), hy = __ldg(&nd->hiy);
+    const float4 lz = __ldg(&nd->loz), hz = __ldg(&nd->hiz);
+    ch = __ldg(&nd->ch);
+    return (box_overlap(lx.x, hx.x, ly.x, hy.x, lz.x, hz.x, lo, hi) ? 1u : 0u) |
+           (box_overlap(lx.y, hx.y, ly.y, hy.y, lz.y, hz.y, lo, hi) ? 2u : 0u) |
+           (box_overlap(lx.z, hx.z, ly.z, hy.z, lz.z, hz.z, lo, hi) ? 4u : 0u) |
+           (box_overlap(lx.w, hx.w, ly.w, hy.w, lz.w, hz.w, lo, hi) ? 8u : 0u);
+}
+
+// Which of the warp's query boxes meet an item of the four-wide hierarchy h
+// (a mask over the lanes; any hit ends a query)?  Each lane brings one query
+// starting at internal node `start` (< 0: none).  First every lane walks its
+// own query depth first, for kAlone nodes at most: most queries that hit are
+// done then (in dense joins nearly all).  What is left of the others goes on
+// one stack in shared memory and all lanes visit its entries, 32 per step, so
+// that no lane waits for the longest walk.  Queries count as hits if the
+// stack would overflow.  (Culling of both sides, everything on the stack from
+// the root against kAlone 12: 2.49 and 2.31 ms on the dense join of 21,008
+// meshes, 0.38 and 0.35 ms on 2 x 50,000 ellipsoids; four lanes per node, a
+// child each, cost more instructions than they saved in L1 passes: 5.2 and
+// 0.56 ms.)
+static __device__ __forceinline__ unsigned warp_any_hit(const DevDataset& h, WarpBoxes& W, int start, const float3& lo,
+                                                        const float3& hi) {
+    const int lane = threadIdx.x & 31;
+    const unsigned below = (1u << lane) - 1u;
+    const unsigned queries = __ballot_sync(0xFFFFFFFFu, start >= 0);
+    bool hit = false;
+    int own = 0;  // entries of this lane: stack[32 d + lane]
+    for (int node = start, n = 0; node >= 0 && n < kAlone; ++n) {
+        int4 ch;
+        const Node4* nd = h.nodes4 + node;
+        const unsigned m = node4_meets(nd, lo, hi, ch);
+        int next = -1;
+        if (m) {
+            const int c[4] = {ch.x, ch.y, ch.z, ch.w};
+            const int cnt = __ldg(&nd->meta.x);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                if (!((m >> j) & 1u)) continue;
+                if (c[j] < 0) {
+                    hit = hit || leaf_meets_box(h, ~c[j], (cnt >> (8 * j)) & 0xFF, lo, hi);
+                } else if (next < 0) {
+                    next = c[j];
+                } else {
+                    W.stack[32 * own + lane] = ((uint32_t)c[j] << 5) | (uint32_t)lane;
+                    ++own;
+                }
+            }
+        }
+        if (hit) {
+            own = 0;
+            break;
+        }
+        if (next >= 0 && (n + 1 == kAlone || own > kAloneStack - 4)) {
+            W.stack[32 * own + lane] = ((uint32_t)next << 5) | (uint32_t)lane;
+            ++own;
+            break;
+        }
+        if (next < 0 && own > 0 && n + 1 < kAlone) next = (int)(W.stack[32 * --own + lane] >> 5);
+        node = next;
+    }
+    unsigned found = __ballot_sync(0xFFFFFFFFu, hit);
+    if (!__any_sync(0xFFFFFFFFu, own > 0)) return found & queries;
+    W.box[0][lane] = lo.x; W.box[1][lane] = lo.y; W.box[2][lane] = lo.z;
+    W.box[3][lane] = hi.x; W.box[4][lane] = hi.y; W.box[5][lane] = hi.z;
+    // the lanes' entries together (each level is read before it is written over)
+    int sp = 0;
+    for (int d = 0;; ++d) {
+        const unsigned mi = __ballot_sync(0xFFFFFFFFu, own > d);
+        if (!mi) break;
+        const uint32_t e = own > d ? W.stack[32 * d + lane] : 0u;
+        __syncwarp();
+        if (own > d) W.stack[sp + __popc(mi & below)] = e;
+        sp += __popc(mi);
+        __syncwarp();
+    }
+    while (sp > 0 && (queries & ~found)) {
+        const int take = min(min(sp, 32), max((kWarpStack - kWarpReserve - sp) / 3, 1));
+        sp -= take;
+        const uint32_t e = lane < take ? W.stack[sp + lane] : 0u;
+        const uint32_t u = e & 31u;
+        const bool in = lane < take && !((found >> u) & 1u);
+        __syncwarp();
+        if (sp + 4 * take > kWarpStack) return queries;  // deeper than any hierarchy this library builds
+        hit = false;
+        unsigned inner = 0;
+        int4 ch = make_int4(0, 0, 0, 0);
+        if (in) {
+            const Node4* nd = h.nodes4 + (e >> 5);
+            const float3 ulo = make_float3(W.box[0][u], W.box[1][u], W.box[2][u]);
+            const float3 uhi = make_float3(W.box[3][u], W.box[4][u], W.box[5][u]);
+            const unsigned m = node4_meets(nd, ulo, uhi, ch);
+            if (m) {
+                const int c[4] = {ch.x, ch.y, ch.z, ch.w};
+                const int cnt = __ldg(&nd->meta.x);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    if (!((m >> j) & 1u)) continue;
+                    if (c[j] >= 0) inner |= 1u << j;
+                    else hit = hit || leaf_meets_box(h, ~c[j], (cnt >> (8 * j)) & 0xFF, ulo, uhi);
+                }
+            }
+        }
+        if (__any_sync(0xFFFFFFFFu, hit)) {
+            found |= __reduce_or_sync(0xFFFFFFFFu, hit ? 1u << u : 0u);
+            if ((found >> u) & 1u) inner = 0;
+        }
+        const int c[4] = {ch.x, ch.y, ch.z, ch.w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const bool push = (inner >> j) & 1u;
+            const unsigned mi = __ballot_sync(0xFFFFFFFFu, push);
+            if (push) W.stack[sp + __popc(mi & below)] = ((uint32_t)c[j] << 5) | u;
+            sp += __popc(mi);
+        }
+        __syncwarp();
+    }
+    __syncwarp();
+    return found & queries;
+}
+
+}  // namespace pgpu
