@@ -218,7 +218,8 @@ typedef struct pierce_stats {
     double ms_total;              /* GPU time of the whole join (CUDA events) */
     double ms_edge_rays[2];       /* A->B, B->A edge-ray kernels (all passes); a join by triangle pairs
                                      tests both directions at once: [0] alone */
-    double ms_parity[2];          /* A->B, B->A parity kernels */
+    double ms_parity[2];          /* A->B, B->A parity kernels; an intersection of datasets with contiguous
+                                     objects casts both directions' rays at once: [0] alone */
     double ms_dedup;              /* scan, sort/unique or compaction */
     uint64_t rays;                /* edge rays traced (per pass); a join by triangle pairs: the segments of
                                      the groups it tests, each group's once (the rays of its triangles) */

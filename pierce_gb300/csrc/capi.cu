@@ -39,15 +39,15 @@ int launch_containment_candidates(pierce_ctx* ctx, const uint64_t* ptable, const
                                   uint8_t* act_a, int64_t na, uint8_t* act_b, int64_t nb);
 int launch_group_incidences(pierce_ctx* ctx, const float4* soup, int64_t n_tris, int G, int step,
                             const DevDataset& tgt, unsigned long long* count);
-int launch_containment_pairs(pierce_ctx* ctx, const uint64_t* ptable, const uint32_t* parity, uint64_t pslots,
+int launch_containment_pairs(pierce_ctx* ctx, const uint64_t* pairs, const unsigned long long* n_pairs,
+                             uint64_t pairs_cap, int64_t bound, uint64_t* big, unsigned long long* n_big,
                              const DevDataset& a, const DevDataset& b, uint64_t* out, unsigned long long* count,
                              uint64_t cap, unsigned long long* fallback);
 int launch_object_pseudo_tris(pierce_ctx* ctx, int32_t n, uint32_t* idx, int32_t* t2o);
 int launch_parity(pierce_ctx* ctx, const DevDataset& src, const DevDataset& tgt, int swap, uint64_t* table,
                   uint32_t* parity, uint64_t slots, int64_t src_lo = 0, int64_t src_hi = -1);
-int launch_parity_objects(pierce_ctx* ctx, const DevDataset& src, const DevDataset& objs, const DevDataset& tgt,
-                          const ColumnGrid* grid, int swap, uint64_t* table, uint32_t* parity, uint64_t slots,
-                          int64_t src_lo = 0, int64_t src_hi = -1);
+int launch_parity_objects(pierce_ctx* ctx, const ParityRays* side0, const ParityRays* side1, const PairSet& set,
+                          uint64_t* out, unsigned long long* out_count, uint64_t out_cap);
 int launch_parity_tracking(pierce_ctx* ctx, const DevDataset& src, const DevDataset& tgt, const ColumnGrid& grid,
                            int32_t k, int32_t* ids, uint32_t* hits, uint32_t* crossed, uint32_t* overflow);
 size_t column_grid_bytes(int32_t n);
@@ -110,6 +110,7 @@ enum : int {
     SLOT_LISTED_A = 36,       // joins by triangle pairs: A's listed groups
     SLOT_MASKS = 41,          // kept groups per chunk of a culling pass
     SLOT_SPILL = 37,          // ... their work words and entries left for the next round
+    SLOT_CONT_WORDS = 42,     // containment: counts of its lists
     SLOT_ENTRY_AB = 38,       // rays from triangles: entry nodes of the listed groups, A->B
     SLOT_ENTRY_BA = 39,
 };
@@ -218,6 +219,21 @@ int host_value(pierce_ctx* ctx, const void* dptr, int bytes, int64_t* out, const
         g->widths.push_back(bytes);
     }
     *out = v;
+    return PIERCE_OK;
+}
+
+// n (at most 4) consecutive 8-byte values in one copy (one by one where a
+// join graph's plan takes them).
+static int host_values(pierce_ctx* ctx, const unsigned long long* dptr, int n, int64_t* out, const char* what) {
+    if (ctx->plan) {
+        for (int i = 0; i < n; ++i)
+            if (int s = host_value(ctx, dptr + i, 8, out + i, what)) return s;
+        return PIERCE_OK;
+    }
+    if (int s = check_cuda(cudaMemcpyAsync(ctx->h_small, dptr, 8 * (size_t)n, cudaMemcpyDeviceToHost, ctx->stream), what))
+        return s;
+    if (int s = check_cuda(cudaStreamSynchronize(ctx->stream), what)) return s;
+    std::memcpy(out, ctx->h_small, 8 * (size_t)n);
     return PIERCE_OK;
 }
 
@@ -1154,9 +1170,10 @@ struct Join {
     }
     bool pairs_pending = false;    // containment: candidate pairs to test before any hierarchy is built
 
-    // Containment from the candidate pairs directly (k_containment_pairs):
-    // the odd parity pairs none of whose triangles meet.  *fallback: some
-    // pair was too large to test this way (nothing is emitted then).
+    // Containment from the candidate pairs directly: the odd parity pairs none
+    // of whose triangles meet.  *fallback: some pair was too large to test
+    // this way (nothing is emitted then).  A list that proved too short is
+    // enlarged and its launches run again.
     int containment_by_pairs(pierce_result** out, bool* fallback) {
         *fallback = false;
         uint64_t cap = 8 * (uint64_t)std::max(B->num_objects, 1) + 16;
@@ -1167,24 +1184,29 @@ struct Join {
             void* p = nullptr;
             if (int s = scratch(ctx, SLOT_BUILD_D, cap * 8, &p)) return s;
             ckeys = static_cast<uint64_t*>(p);
-            void* pc = nullptr;
-            if (int s = scratch(ctx, SLOT_AUX, 64, &pc)) return s;
-            unsigned long long* d_count = static_cast<unsigned long long*>(pc);
-            cudaMemsetAsync(d_count, 0, 16, ctx->stream);
-            if (int s = launch_containment_pairs(ctx, cont_ptable, cont_par, cont_pslots, va, vb, ckeys, d_count, cap,
-                                                 d_count + 1))
+            if (int s = launch_containment_pairs(ctx, cont_ptable, cwords, cont_cap, (int64_t)cont_cap,
+                                                 cont_ptable + cont_cap, cwords + 1, va, vb, ckeys, cwords + 2, cap,
+                                                 cwords + 3))
                 return s;
-            int64_t nf = 0, nv = 0;
-            if (int s = host_value(ctx, d_count + 1, 8, &nf, "containment pairs left over")) return s;
-            if (nf > 0) {
+            // odd pairs, pairs left to blocks, containment pairs, undecided pairs
+            int64_t v[4];
+            if (int s = host_values(ctx, cwords, 4, v, "containment counts")) return s;
+            if ((uint64_t)v[0] > cont_cap) {
+                cont_cap = (uint64_t)v[0];
+                st.retries++;
+                if (int s = odd_pairs()) return s;
+                continue;
+            }
+            cont_pslots = (uint64_t)v[0];
+            if (v[3] > 0) {
                 *fallback = true;
                 return PIERCE_OK;
             }
-            if (int s = host_value(ctx, d_count, 8, &nv, "containment count")) return s;
-            n = (uint64_t)nv;
+            n = (uint64_t)v[2];
             if (n <= cap) break;
             cap = n;
             st.retries++;
+            cudaMemsetAsync(cwords + 1, 0, 24, ctx->stream);
         }
         timer.span(b, timer.record(), &st.ms_edge_rays[1]);
         st.containment_pairs = n;
@@ -1218,9 +1240,51 @@ struct Join {
     uint32_t* cont_par = nullptr;
     uint64_t cont_pslots = 0;
 
-    // Parity of B's first vertices against A into SLOT_CONT_PARITY (a full
-    // table is enlarged and the parity rerun).
+    unsigned long long* cwords = nullptr;  // odd pairs, pairs left to blocks, containment pairs, undecided pairs
+    uint64_t cont_cap = 0;                 // odd pairs SLOT_CONT_PARITY holds (and as many left to blocks)
+
+    // Object pairs: the odd pairs of B's first vertices in A as a list.
+    int odd_pairs() {
+        void *p = nullptr, *w = nullptr;
+        cont_cap = std::max<uint64_t>(cont_cap, 8 * (uint64_t)std::max(B->num_objects, 1) + 16);
+        if (int s = scratch(ctx, SLOT_CONT_PARITY, cont_cap * 16, &p)) return s;
+        if (int s = scratch(ctx, SLOT_CONT_WORDS, 64, &w)) return s;
+        cont_ptable = static_cast<uint64_t*>(p);
+        cont_par = nullptr;
+        cwords = static_cast<unsigned long long*>(w);
+        cudaMemsetAsync(cwords, 0, 32, ctx->stream);
+        const int b = timer.record();
+        const ParityRays rays = parity_rays(1);
+        if (int s = launch_parity_objects(ctx, &rays, nullptr, PairSet{}, cont_ptable, cwords, cont_cap)) return s;
+        timer.span(b, timer.record(), &st.ms_parity[1]);
+        return PIERCE_OK;
+    }
+
+    // Parity rays of direction d: A's objects in B (0), B's in A (1).
+    ParityRays parity_rays(int d) const {
+        ParityRays r;
+        r.src = d ? vb : va;
+        r.tgt = d ? va : vb;
+        r.grid = d ? gridA_ : gridB_;
+        r.lo = shard_lo(r.src.num_objects);
+        r.hi = shard_hi(r.src.num_objects);
+        r.swap = d;
+        return r;
+    }
+
+    // Parity of B's first vertices against A into SLOT_CONT_PARITY: a list of
+    // odd pairs, or a parity table (a full one is enlarged and the parity
+    // rerun).
     int containment_parity() {
+        while (object_parity) {
+            if (int s = odd_pairs()) return s;
+            int64_t n = 0;
+            if (int s = host_value(ctx, cwords, 8, &n, "odd pairs")) return s;
+            cont_pslots = (uint64_t)n;
+            if (cont_pslots <= cont_cap) return PIERCE_OK;
+            cont_cap = cont_pslots;
+            st.retries++;
+        }
         uint64_t pslots = table_slots_for(8 * (uint64_t)std::max(B->num_objects, 1), 0.5);
         for (int attempt = 0;; ++attempt) {
             void* p = nullptr;
@@ -1230,13 +1294,9 @@ struct Join {
             cudaMemsetAsync(ptable, 0xFF, pslots * 8, ctx->stream);
             cudaMemsetAsync(par, 0, pslots * 4, ctx->stream);
             const int b = timer.record();
-            const int64_t lo = shard_lo(B->num_objects), hi = shard_hi(B->num_objects);
-            if (object_parity) {
-                if (int s = launch_parity_objects(ctx, vb, objA_, va, &gridA_, 1, ptable, par, pslots, lo, hi))
-                    return s;
-            } else if (int s = launch_parity(ctx, vb, va, 1, ptable, par, pslots, lo, hi)) {
+            if (int s = launch_parity(ctx, vb, va, 1, ptable, par, pslots, shard_lo(B->num_objects),
+                                      shard_hi(B->num_objects)))
                 return s;
-            }
             timer.span(b, timer.record(), &st.ms_parity[1]);
             uint32_t bits = 0;
             if (int s = read_device_error(ctx, &bits)) return s;
@@ -1423,11 +1483,10 @@ struct Join {
         if (o.predicate == PIERCE_CONTAINMENT && !o.include_overlap_pairs && object_parity) {
             // containment = parity(B in A) \ overlap: the odd-parity pairs
             // are tested directly (containment_by_pairs), which needs only
-            // A's object hierarchy and column grid for the parity; the rest
+            // A's column grid for the parity; the rest
             // is built only if some pair is too large for that
-            if (int s = object_bvh(A, SLOT_OBJ_A, SLOT_NODES4_OBJ_A, &objA_)) return s;
             if (int s = column_grids(true, false)) return s;
-            if (int s = containment_parity()) return s;
+            if (int s = odd_pairs()) return s;
             rays_by_candidates = true;
             pairs_pending = true;
             timer.span(b0, timer.record(), &st.ms_build);
@@ -1443,12 +1502,13 @@ struct Join {
     }
 
     // Containment whose candidate pairs were too large to test directly:
-    // B's object hierarchy, the object flags restricted to the candidates'
+    // the object hierarchies, the object flags restricted to the candidates'
     // objects, then the culling pipeline.
     int containment_fallback() {
         const int b0 = timer.record();
         uint8_t* act_a = active;
         uint8_t* act_b = active + std::max(A->num_objects, 1);
+        if (int s = object_bvh(A, SLOT_OBJ_A, SLOT_NODES4_OBJ_A, &objA_)) return s;
         if (int s = object_bvh(B, SLOT_OBJ_B, SLOT_NODES4_OBJ_B, &objB_)) return s;
         if (int s = launch_object_active(ctx, va, objB_, act_a, vb, objA_, act_b)) return s;
         if (int s = launch_containment_candidates(ctx, cont_ptable, cont_par, cont_pslots, act_a, A->num_objects, act_b,
@@ -2023,6 +2083,13 @@ struct Join {
     // emit odd keys (into out_set, or appended to out_keys).
     int parity(const DevDataset& src, const DevDataset& tgt, int swap, double* ms, const PairSet& out_set,
                uint64_t* out_keys, unsigned long long* out_count, uint64_t out_cap) {
+        if (object_parity) {
+            const int b = timer.record();
+            const ParityRays rays = parity_rays(swap);
+            if (int s = launch_parity_objects(ctx, &rays, nullptr, out_set, out_keys, out_count, out_cap)) return s;
+            timer.span(b, timer.record(), ms);
+            return PIERCE_OK;
+        }
         uint64_t pslots = table_slots_for(8 * (uint64_t)std::max(src.num_objects, 1), 0.5);
         for (int attempt = 0;; ++attempt) {
             void* p = nullptr;
@@ -2033,13 +2100,7 @@ struct Join {
             cudaMemsetAsync(par, 0, pslots * 4, ctx->stream);
             int b = timer.record();
             const int64_t lo = shard_lo(src.num_objects), hi = shard_hi(src.num_objects);
-            if (object_parity) {
-                if (int s = launch_parity_objects(ctx, src, swap ? objA_ : objB_, tgt, swap ? &gridA_ : &gridB_, swap,
-                                                  ptable, par, pslots, lo, hi))
-                    return s;
-            } else if (int s = launch_parity(ctx, src, tgt, swap, ptable, par, pslots, lo, hi)) {
-                return s;
-            }
+            if (int s = launch_parity(ctx, src, tgt, swap, ptable, par, pslots, lo, hi)) return s;
             timer.span(b, timer.record(), ms);
             uint32_t bits = 0;
             if (int s = read_device_error(ctx, &bits)) return s;
@@ -2060,8 +2121,17 @@ struct Join {
     // Parity of both directions into the pair table: both launches, one
     // error check, then both emits.  A full parity table falls back to one
     // direction at a time (each with its own enlarging retries).
+    // Object pairs go straight into the set, both directions in one launch.
     int parity_both(const PairSet& set) {
         const bool need[2] = {ab, ba};
+        if (object_parity) {
+            const int b = timer.record();
+            const ParityRays r0 = parity_rays(0), r1 = parity_rays(1);
+            if (int s = launch_parity_objects(ctx, ab ? &r0 : nullptr, ba ? &r1 : nullptr, set, nullptr, nullptr, 0))
+                return s;
+            timer.span(b, timer.record(), &st.ms_parity[ab ? 0 : 1]);
+            return PIERCE_OK;
+        }
         const int slot_of[2] = {SLOT_BUILD_C, SLOT_BUILD_D};
         uint64_t pslots[2] = {0, 0};
         uint64_t* ptable[2] = {nullptr, nullptr};
@@ -2079,13 +2149,7 @@ struct Join {
             cudaMemsetAsync(par[d], 0, pslots[d] * 4, ctx->stream);
             const int b = timer.record();
             const int64_t lo = shard_lo(src.num_objects), hi = shard_hi(src.num_objects);
-            if (object_parity) {
-                if (int s = launch_parity_objects(ctx, src, d ? objA_ : objB_, tgt, d ? &gridA_ : &gridB_, d,
-                                                  ptable[d], par[d], pslots[d], lo, hi))
-                    return s;
-            } else if (int s = launch_parity(ctx, src, tgt, d, ptable[d], par[d], pslots[d], lo, hi)) {
-                return s;
-            }
+            if (int s = launch_parity(ctx, src, tgt, d, ptable[d], par[d], pslots[d], lo, hi)) return s;
             timer.span(b, timer.record(), &st.ms_parity[d]);
         }
         uint32_t bits = 0;

@@ -166,6 +166,16 @@ struct PairJoin {
     bool defer = true;                           // queue undecided pairs (else exact inline)
 };
 
+// Parity rays of source objects [lo, hi) against the objects of tgt, whose
+// column grid is given; swap: keys are (target, source).
+struct ParityRays {
+    DevDataset src;
+    ColumnGrid grid;
+    DevDataset tgt;
+    int64_t lo = 0, hi = 0;
+    int swap = 0;
+};
+
 struct BvhShape {
     int leaf_size = 1;
     int root_is_leaf = 1;

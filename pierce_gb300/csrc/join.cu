@@ -33,6 +33,7 @@
 #include "hash.cuh"
 #include "predicates.cuh"
 #include "walk.cuh"
+#include "grid.cuh"
 
 namespace pgpu {
 
@@ -772,7 +773,7 @@ __global__ void __launch_bounds__(128) k_parity(ParityParams P) {
     (void)n_cross;
 }
 
-// Odd-parity entries of a parity table.  mode 0: insert into out_table;
+// Odd-parity entries of a parity table (parity null: a list of odd keys).  mode 0: insert into out_table;
 // mode 1 (containment): keep only keys absent from the overlap set (hash
 // table or sorted array) and append them to out_keys.
 __global__ void k_parity_emit(const uint64_t* __restrict__ ptable, const uint32_t* __restrict__ parity, uint64_t pslots,
@@ -780,7 +781,7 @@ __global__ void k_parity_emit(const uint64_t* __restrict__ ptable, const uint32_
                               const uint64_t* lookup_sorted, int64_t lookup_n, PairSet out_set, uint64_t* out_keys, unsigned long long* out_count, uint64_t out_cap, uint32_t* err) {
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < pslots; i += (uint64_t)gridDim.x * blockDim.x) {
         const uint64_t key = ptable[i];
-        if (key == kEmptyKey || !(parity[i] & 1u)) continue;
+        if (key == kEmptyKey || (parity && !(parity[i] & 1u))) continue;
         if (mode == 1) {
             const bool in = lookup_table ? hash_contains(lookup_table, lookup_mask, key)
                                          : sorted_contains(lookup_sorted, lookup_n, key);
@@ -797,7 +798,7 @@ __global__ void k_parity_emit(const uint64_t* __restrict__ ptable, const uint32_
 }
 
 // Containment candidates: the objects of the odd (a, b) entries of a parity
-// table (key a << 32 | b).  Activity flags are 0 or 1; a candidate's flag
+// table (key a << 32 | b; parity null: a list of odd keys).  Activity flags are 0 or 1; a candidate's flag
 // gains bit 1 (only ever OR-ed in, so concurrent stores of one byte agree),
 // then k_keep_candidates keeps the objects that are both active and
 // candidates.
@@ -805,7 +806,7 @@ __global__ void k_mark_candidates(const uint64_t* __restrict__ ptable, const uin
                                   uint64_t pslots, uint8_t* act_a, uint8_t* act_b) {
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < pslots; i += (uint64_t)gridDim.x * blockDim.x) {
         const uint64_t key = ptable[i];
-        if (key == kEmptyKey || !(parity[i] & 1u)) continue;
+        if (key == kEmptyKey || (parity && !(parity[i] & 1u))) continue;
         const uint32_t a = (uint32_t)(key >> 32), b = (uint32_t)key;
         act_a[a] = (uint8_t)(act_a[a] | 2u);
         act_b[b] = (uint8_t)(act_b[b] | 2u);
@@ -815,253 +816,6 @@ __global__ void k_mark_candidates(const uint64_t* __restrict__ ptable, const uin
 __global__ void k_keep_candidates(uint8_t* flags, int64_t n) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         flags[i] = flags[i] == 3u ? 1u : 0u;
-}
-
-// ---- containment by candidate pairs -------------------------------------------
-// Containment is parity(B in A) \ overlap (pierce_containment_main.cpp:
-// 385-550), so only the odd-parity pairs (a, b) need an overlap answer.  A
-// block of kPairThreads takes one such pair, so that one large pair does
-// not hold a lone warp for the whole launch: it lists the triangles of a
-// (those of a's 32-triangle chunks whose boxes meet, read first) whose boxes
-// meet the intersection of the two object boxes (a patch of a's
-// surface; the vertices of up to kPairVerts of them are kept in shared
-// memory), shrinks the box to that patch's box, and streams b's triangles
-// past them, one per thread (a triangle whose 32-triangle chunk box misses
-// the patch is skipped unread), each tested against the listed triangles whose
-// boxes meet its own with the exact closed triangle-triangle predicate (an
-// edge of one meets the other: six segment tests, the edge definition for
-// the edges of triangles).  The pair is a containment pair when none meets;
-// a b deep inside a lists nothing and costs one pass over a's triangles.  A
-// patch larger than kPairList is read from a's range in place.  A pair whose
-// objects hold more than kPairScanMax triangles together, or whose unlisted
-// patch would cost more than kPairStreamMax triangle pairs, is counted in
-// *fallback and the join takes the culling pipeline instead.
-constexpr int kPairThreads = 256;
-constexpr int kPairList = 1024;
-constexpr int kPairVerts = 512;
-constexpr int kPairChunkList = 512;  // listed chunks of the container (more: its whole range)
-constexpr int kPairScanMax = 1 << 16;
-constexpr int64_t kPairStreamMax = 1 << 22;
-
-struct PairParams {
-    const uint64_t* ptable;
-    const uint32_t* parity;
-    uint64_t pslots;
-    DevDataset a, b;  // vertices, indices, object ranges and boxes
-    uint64_t* out;
-    unsigned long long* count;
-    uint64_t cap;
-    unsigned long long* fallback;
-    DevCounters* ctr;
-};
-
-__device__ __forceinline__ float3 tri_vertex(const DevDataset& d, uint32_t tri, int k) {
-    const uint32_t i = __ldg(d.idx + 3 * (size_t)tri + k);
-    return make_float3(__ldg(d.verts + 3 * (size_t)i), __ldg(d.verts + 3 * (size_t)i + 1),
-                       __ldg(d.verts + 3 * (size_t)i + 2));
-}
-
-__device__ __forceinline__ bool tri_box_meets(const float3& p, const float3& q, const float3& r, const float3& lo,
-                                              const float3& hi) {
-    return box_overlap(fminf(p.x, fminf(q.x, r.x)), fmaxf(p.x, fmaxf(q.x, r.x)), fminf(p.y, fminf(q.y, r.y)),
-                       fmaxf(p.y, fmaxf(q.y, r.y)), fminf(p.z, fminf(q.z, r.z)), fmaxf(p.z, fmaxf(q.z, r.z)), lo, hi);
-}
-
-__device__ __forceinline__ float block_min(float v, float* red) {
-    for (int off = 16; off; off >>= 1) v = fminf(v, __shfl_xor_sync(0xFFFFFFFFu, v, off));
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-    __syncthreads();
-    float r = red[0];
-    for (int k = 1; k < kPairThreads / 32; ++k) r = fminf(r, red[k]);
-    __syncthreads();
-    return r;
-}
-__device__ __forceinline__ float block_max(float v, float* red) { return -block_min(-v, red); }
-
-// Position of this thread's flag among the block's set flags, after `base`
-// (warp ballots; per-warp counts in s_warp), and the block's total.
-__device__ __forceinline__ int block_compact(bool flag, int base, int* s_warp) {
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const unsigned m = __ballot_sync(0xFFFFFFFFu, flag);
-    if (lane == 0) s_warp[w] = __popc(m);
-    __syncthreads();
-    int before = base;
-    for (int q = 0; q < w; ++q) before += s_warp[q];
-    return before + __popc(m & ((1u << lane) - 1u));
-}
-__device__ __forceinline__ int block_total(const int* s_warp) {
-    int total = 0;
-    for (int q = 0; q < kPairThreads / 32; ++q) total += s_warp[q];
-    return total;
-}
-
-__global__ void __launch_bounds__(kPairThreads) k_containment_pairs(PairParams P) {
-    __shared__ uint32_t s_list[kPairList];
-    __shared__ uint32_t s_chunk[kPairChunkList];
-    __shared__ float4 s_tri[kPairVerts][3];
-    __shared__ int s_warp[kPairThreads / 32];
-    __shared__ float s_red[kPairThreads / 32];
-    __shared__ uint64_t s_pairs[kPairThreads];
-    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-    PredCounters pc{0, 0};
-    uint32_t tests = 0;
-    // windows of kPairThreads slots of the parity table: every thread reads
-    // one slot, the block compacts the odd pairs, then takes them in turn
-    for (int64_t wbase = (int64_t)blockIdx.x * kPairThreads; wbase < (int64_t)P.pslots;
-         wbase += (int64_t)gridDim.x * kPairThreads) {
-        uint64_t slot_key = kEmptyKey;
-        bool odd = false;
-        if (wbase + tid < (int64_t)P.pslots) {
-            slot_key = P.ptable[wbase + tid];
-            odd = slot_key != kEmptyKey && (P.parity[wbase + tid] & 1u);
-        }
-        const int odd_pos = block_compact(odd, 0, s_warp);
-        const int n_odd = block_total(s_warp);
-        if (odd) s_pairs[odd_pos] = slot_key;
-        __syncthreads();
-        for (int q = 0; q < n_odd; ++q) {
-            const uint64_t key = s_pairs[q];
-            const uint32_t a = (uint32_t)(key >> 32), b = (uint32_t)key;
-            const float* ba = P.a.obj_box + 6 * (size_t)a;
-            const float* bb = P.b.obj_box + 6 * (size_t)b;
-            float3 lo = make_float3(fmaxf(__ldg(ba), __ldg(bb)), fmaxf(__ldg(ba + 1), __ldg(bb + 1)),
-                                    fmaxf(__ldg(ba + 2), __ldg(bb + 2)));
-            float3 hi = make_float3(fminf(__ldg(ba + 3), __ldg(bb + 3)), fminf(__ldg(ba + 4), __ldg(bb + 4)),
-                                    fminf(__ldg(ba + 5), __ldg(bb + 5)));
-            bool meets = false, undecided = false;
-            if (lo.x <= hi.x && lo.y <= hi.y && lo.z <= hi.z) {
-                const int2 ra = __ldg(P.a.obj_range + a), rb = __ldg(P.b.obj_range + b);
-                if ((int64_t)ra.y + rb.y > kPairScanMax) {
-                    undecided = true;
-                } else {
-                    // a's 32-triangle chunks whose boxes meet the common box, then
-                    // the triangles of those chunks that do: the list (block-wide
-                    // compaction) and the patch box
-                    const int c0 = ra.x >> 5, c1 = (ra.x + ra.y - 1) >> 5;
-                    int nmc = 0;
-                    for (int base = c0; base <= c1; base += kPairThreads) {
-                        const int c = base + tid;
-                        bool meet = true;  // no chunk boxes: every chunk
-                        if (c > c1) meet = false;
-                        else if (P.a.tri_chunk_box) {
-                            const float* cb = P.a.tri_chunk_box + 6 * (size_t)c;
-                            meet = box_overlap(__ldg(cb), __ldg(cb + 3), __ldg(cb + 1), __ldg(cb + 4), __ldg(cb + 2),
-                                               __ldg(cb + 5), lo, hi);
-                        }
-                        const int pos = block_compact(meet, nmc, s_warp);
-                        if (meet && pos < kPairChunkList) s_chunk[pos] = (uint32_t)c;
-                        nmc += block_total(s_warp);
-                        __syncthreads();
-                    }
-                    int na = 0;
-                    float3 plo = make_float3(3.4e38f, 3.4e38f, 3.4e38f), phi = make_float3(-3.4e38f, -3.4e38f, -3.4e38f);
-                    const bool by_chunks = nmc <= kPairChunkList;
-                    const int slots = by_chunks ? 32 * nmc : ra.y;
-                    for (int base = 0; base < slots; base += kPairThreads) {
-                        const int k = base + tid;
-                        bool meet = false;
-                        uint32_t t = 0;
-                        if (k < slots) {
-                            const int tt = by_chunks ? (int)(s_chunk[k >> 5] << 5) + (k & 31) : ra.x + k;
-                            if (tt >= ra.x && tt < ra.x + ra.y) {
-                                t = (uint32_t)tt;
-                                const float3 v0 = tri_vertex(P.a, t, 0), v1 = tri_vertex(P.a, t, 1),
-                                             v2 = tri_vertex(P.a, t, 2);
-                                meet = tri_box_meets(v0, v1, v2, lo, hi);
-                                if (meet) {
-                                    plo = make_float3(fminf(plo.x, fminf(v0.x, fminf(v1.x, v2.x))),
-                                                      fminf(plo.y, fminf(v0.y, fminf(v1.y, v2.y))),
-                                                      fminf(plo.z, fminf(v0.z, fminf(v1.z, v2.z))));
-                                    phi = make_float3(fmaxf(phi.x, fmaxf(v0.x, fmaxf(v1.x, v2.x))),
-                                                      fmaxf(phi.y, fmaxf(v0.y, fmaxf(v1.y, v2.y))),
-                                                      fmaxf(phi.z, fmaxf(v0.z, fmaxf(v1.z, v2.z))));
-                                }
-                            }
-                        }
-                        const int pos = block_compact(meet, na, s_warp);
-                        if (meet && pos < kPairList) s_list[pos] = t;
-                        na += block_total(s_warp);
-                        __syncthreads();
-                    }
-                    plo = make_float3(block_min(plo.x, s_red), block_min(plo.y, s_red), block_min(plo.z, s_red));
-                    phi = make_float3(block_max(phi.x, s_red), block_max(phi.y, s_red), block_max(phi.z, s_red));
-                    const bool listed = na <= kPairList;
-                    const bool cached = na <= kPairVerts;
-                    if (cached) {
-                        for (int k = tid; k < na; k += kPairThreads) {
-                            const uint32_t t = s_list[k];
-                            for (int v = 0; v < 3; ++v) {
-                                const float3 x = tri_vertex(P.a, t, v);
-                                s_tri[k][v] = make_float4(x.x, x.y, x.z, 0.0f);
-                            }
-                        }
-                        __syncthreads();
-                    }
-                    if (!listed && (int64_t)ra.y * rb.y > kPairStreamMax) {
-                        undecided = true;
-                    } else if (na > 0) {
-                        lo = make_float3(fmaxf(lo.x, plo.x), fmaxf(lo.y, plo.y), fmaxf(lo.z, plo.z));
-                        hi = make_float3(fminf(hi.x, phi.x), fminf(hi.y, phi.y), fminf(hi.z, phi.z));
-                        const int nj = listed ? na : ra.y;
-                        // b's triangles, one per thread, against the patch
-                        for (int base = 0; base < rb.y && !meets; base += kPairThreads) {
-                            const int k = base + tid;
-                            bool hit = false;
-                            bool near = k < rb.y;
-                            if (near && P.b.tri_chunk_box) {  // the triangle's chunk box first
-                                const float* cb = P.b.tri_chunk_box + 6 * (size_t)((rb.x + k) >> 5);
-                                near = box_overlap(__ldg(cb), __ldg(cb + 3), __ldg(cb + 1), __ldg(cb + 4), __ldg(cb + 2),
-                                                   __ldg(cb + 5), lo, hi);
-                            }
-                            if (near) {
-                                const uint32_t tb = (uint32_t)(rb.x + k);
-                                const float3 b0 = tri_vertex(P.b, tb, 0), b1 = tri_vertex(P.b, tb, 1),
-                                             b2 = tri_vertex(P.b, tb, 2);
-                                const float3 blo = make_float3(fminf(b0.x, fminf(b1.x, b2.x)), fminf(b0.y, fminf(b1.y, b2.y)),
-                                                               fminf(b0.z, fminf(b1.z, b2.z)));
-                                const float3 bhi = make_float3(fmaxf(b0.x, fmaxf(b1.x, b2.x)), fmaxf(b0.y, fmaxf(b1.y, b2.y)),
-                                                               fmaxf(b0.z, fmaxf(b1.z, b2.z)));
-                                if (box_overlap(blo.x, bhi.x, blo.y, bhi.y, blo.z, bhi.z, lo, hi)) {
-                                    for (int j = 0; j < nj && !hit; ++j) {
-                                        float3 a0, a1, a2;
-                                        if (cached) {
-                                            const float4 x0 = s_tri[j][0], x1 = s_tri[j][1], x2 = s_tri[j][2];
-                                            a0 = make_float3(x0.x, x0.y, x0.z);
-                                            a1 = make_float3(x1.x, x1.y, x1.z);
-                                            a2 = make_float3(x2.x, x2.y, x2.z);
-                                        } else {
-                                            const uint32_t ta = listed ? s_list[j] : (uint32_t)(ra.x + j);
-                                            a0 = tri_vertex(P.a, ta, 0);
-                                            a1 = tri_vertex(P.a, ta, 1);
-                                            a2 = tri_vertex(P.a, ta, 2);
-                                        }
-                                        if (!tri_box_meets(a0, a1, a2, blo, bhi)) continue;
-                                        ++tests;
-                                        hit = seg_tri_exact(a0, a1, b0, b1, b2, pc) || seg_tri_exact(a1, a2, b0, b1, b2, pc) ||
-                                              seg_tri_exact(a2, a0, b0, b1, b2, pc) || seg_tri_exact(b0, b1, a0, a1, a2, pc) ||
-                                              seg_tri_exact(b1, b2, a0, a1, a2, pc) || seg_tri_exact(b2, b0, a0, a1, a2, pc);
-                                    }
-                                }
-                            }
-                            meets = __syncthreads_or(hit) != 0;
-                        }
-                    }
-                }
-            }
-            if (tid == 0) {
-                if (undecided) {
-                    atomicAdd(P.fallback, 1ull);
-                } else if (!meets) {
-                    const unsigned long long pos = atomicAdd(P.count, 1ull);
-                    if (pos < P.cap) P.out[pos] = key;
-                }
-            }
-            __syncthreads();
-        }
-    }
-    flush_counter(&P.ctr->tri_tests, tests);
-    flush_counter(&P.ctr->fp32_ambiguous, pc.fp32_ambiguous);
-    flush_counter(&P.ctr->fp64_ambiguous, pc.fp64_ambiguous);
 }
 
 // Occupied slots -> dense key array (warp-aggregated cursor).  The counter
@@ -1880,15 +1634,6 @@ __global__ void k_fill_u32_j(uint32_t* p, uint32_t value, int64_t n) {
 // that is unbounded above.  About one object per cell on average.
 
 
-__device__ __forceinline__ void grid_cell_range(const float* b, int nx, int ny, float lo, float hi, int axis,
-                                                int& c0, int& c1) {
-    const float o = b[axis], e = b[2 + axis] - b[axis];
-    const int n = axis ? ny : nx;
-    const float inv = e > 0.0f ? (float)n / e : 0.0f;
-    c0 = min(max((int)floorf((lo - o) * inv), 0), n - 1);
-    c1 = min(max((int)floorf((hi - o) * inv), 0), n - 1);
-}
-
 __global__ void k_grid_bounds(const float* __restrict__ obj_box, int32_t n, uint32_t* ob) {
     float lo[2] = {3.4e38f, 3.4e38f}, hi[2] = {-3.4e38f, -3.4e38f};
     for (int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; o < n; o += (int64_t)gridDim.x * blockDim.x) {
@@ -1938,202 +1683,6 @@ __global__ void k_grid_fill(const float* __restrict__ obj_box, int32_t n, const 
                 else entries[offsets[c] + atomicAdd(cursor + c, 1)] = (int32_t)o;
             }
     }
-}
-
-// Parity by object pairs: a warp per source object walks the target's
-// object hierarchy with the +Z ray of the object's first vertex (candidate
-// target objects: box contains the point in x, y and reaches above it) and
-// counts, across its lanes, the crossings of every triangle of each
-// candidate (the object's contiguous triangle range).  Odd counts go to the
-// parity table.  Needs no triangle hierarchy, so the per-join hierarchies
-// can drop triangles far from the other side.
-struct ParityObjParams {
-    DevDataset src;   // first vertices, partitions
-    int64_t src_lo, src_hi;  // source objects [src_lo, src_hi) cast rays (a shard)
-    ColumnGrid grid;  // the target's column grid (nx == 0: use the object hierarchy)
-    DevDataset objs;  // the target's object hierarchy
-    DevDataset tgt;   // the target's triangles (verts, idx, obj_range)
-    int swap;
-    uint64_t* table;
-    uint32_t* parity;
-    uint64_t mask;
-    uint32_t* err;
-    DevCounters* ctr;
-    // k_parity_objects<true> (diagnostics) writes, instead of table entries,
-    // per source object s: the targets its ray crosses an odd number of times
-    // with their crossing counts (slots s * track_k ..., in candidate order),
-    // the number of targets it crosses at all, and the odd targets that found
-    // no slot
-    int32_t track_k;
-    int32_t* track_ids;
-    uint32_t* track_hits;
-    uint32_t* track_crossed;
-    uint32_t* track_overflow;
-};
-
-template <bool TRACK>
-__global__ void __launch_bounds__(128) k_parity_objects(ParityObjParams P) {
-    const int lane = threadIdx.x & 31;
-    const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-    uint32_t n_nodes = 0, n_tests = 0, n_rays = 0;
-    PredCounters pc{0, 0};
-    for (int64_t s = P.src_lo + (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); s < P.src_hi;
-         s += warps) {
-        const float4 fv = __ldg(P.src.first_vertex + s);
-        if (fv.w != 0.0f) continue;  // object without triangles (warp-uniform)
-        ++n_rays;
-        const float3 p = make_float3(fv.x, fv.y, fv.z);
-        uint32_t n_crossed = 0, n_odd = 0;  // TRACK: lane 0's tallies of this source
-        auto candidate = [&](int32_t t) {
-            const int2 r = __ldg(P.tgt.obj_range + t);
-            uint32_t crossings = 0;
-            uint32_t ncross = 0;  // TRACK: this lane's crossings
-            auto test = [&](int64_t tri) {
-                const uint32_t i0 = __ldg(P.tgt.idx + 3 * tri), i1 = __ldg(P.tgt.idx + 3 * tri + 1),
-                               i2 = __ldg(P.tgt.idx + 3 * tri + 2);
-                const float3 a = make_float3(__ldg(P.tgt.verts + 3 * (size_t)i0), __ldg(P.tgt.verts + 3 * (size_t)i0 + 1),
-                                             __ldg(P.tgt.verts + 3 * (size_t)i0 + 2));
-                const float3 b = make_float3(__ldg(P.tgt.verts + 3 * (size_t)i1), __ldg(P.tgt.verts + 3 * (size_t)i1 + 1),
-                                             __ldg(P.tgt.verts + 3 * (size_t)i1 + 2));
-                const float3 c = make_float3(__ldg(P.tgt.verts + 3 * (size_t)i2), __ldg(P.tgt.verts + 3 * (size_t)i2 + 1),
-                                             __ldg(P.tgt.verts + 3 * (size_t)i2 + 2));
-                if (fminf(a.x, fminf(b.x, c.x)) > p.x || fmaxf(a.x, fmaxf(b.x, c.x)) < p.x ||
-                    fminf(a.y, fminf(b.y, c.y)) > p.y || fmaxf(a.y, fmaxf(b.y, c.y)) < p.y ||
-                    fmaxf(a.z, fmaxf(b.z, c.z)) < p.z)
-                    return;
-                ++n_tests;
-                if (zray_cross(p, a, b, c, pc)) {
-                    crossings ^= 1u;
-                    if constexpr (TRACK) ++ncross;
-                }
-            };
-            if (P.tgt.tri_chunk_box) {
-                // only the 32-triangle chunks whose box the ray's column meets
-                const int64_t end = (int64_t)r.x + r.y;
-                const int64_t c_first = (int64_t)r.x / 32, c_last = (end - 1) / 32;
-                for (int64_t c0 = c_first; c0 <= c_last; c0 += 32) {
-                    const int64_t c = c0 + lane;
-                    bool hit = false;
-                    if (c <= c_last) {
-                        const float* bb = P.tgt.tri_chunk_box + 6 * c;
-                        hit = __ldg(bb) <= p.x && p.x <= __ldg(bb + 3) && __ldg(bb + 1) <= p.y &&
-                              p.y <= __ldg(bb + 4) && __ldg(bb + 5) >= p.z;
-                    }
-                    unsigned m = __ballot_sync(0xFFFFFFFFu, hit);
-                    while (m) {
-                        const int bit = __ffs(m) - 1;
-                        m &= m - 1;
-                        const int64_t tri = (c0 + bit) * 32 + lane;
-                        if (tri >= r.x && tri < end) test(tri);
-                    }
-                }
-            } else {
-                for (int k = lane; k < r.y; k += 32) test((int64_t)r.x + k);
-            }
-            const unsigned odd = __popc(__ballot_sync(0xFFFFFFFFu, crossings != 0)) & 1u;
-            if constexpr (TRACK) {
-                const uint32_t hits = __reduce_add_sync(0xFFFFFFFFu, ncross);
-                if (hits && lane == 0) {
-                    ++n_crossed;
-                    if (odd) {
-                        if (n_odd < (uint32_t)P.track_k) {
-                            const int64_t at = s * (int64_t)P.track_k + n_odd;
-                            P.track_ids[at] = t;
-                            P.track_hits[at] = hits;
-                        }
-                        ++n_odd;
-                    }
-                }
-            } else if (odd && lane == 0) {
-                const uint64_t key = P.swap ? pack_key(t, (int32_t)s) : pack_key((int32_t)s, t);
-                uint32_t probes = 0;
-                const int64_t slot = hash_insert(P.table, P.mask, key, P.err, probes);
-                if (slot >= 0) P.parity[slot] = 1u;  // one warp owns the keys of its source object
-            }
-        };
-        auto finish = [&]() {
-            if constexpr (TRACK) {
-                if (lane == 0) {
-                    P.track_crossed[s] = n_crossed;
-                    P.track_overflow[s] = n_odd > (uint32_t)P.track_k ? n_odd - (uint32_t)P.track_k : 0u;
-                }
-            }
-        };
-        auto leaf = [&](int first, int count) {
-            for (int k = 0; k < count; ++k) {
-                const float4 a4 = __ldg(P.objs.soup + 3 * (int64_t)(first + k));
-                const float4 b4 = __ldg(P.objs.soup + 3 * (int64_t)(first + k) + 1);
-                if (a4.x <= p.x && p.x <= b4.x && a4.y <= p.y && p.y <= b4.y && b4.z >= p.z)
-                    candidate(__float_as_int(a4.w));
-            }
-        };
-        if (P.grid.nx > 0) {
-            const float* gb = P.grid.bounds;
-            int cx, cx1, cy, cy1;
-            grid_cell_range(gb, P.grid.nx, P.grid.ny, p.x, p.x, 0, cx, cx1);
-            grid_cell_range(gb, P.grid.nx, P.grid.ny, p.y, p.y, 1, cy, cy1);
-            const int c = cy * P.grid.nx + cx;
-            const int32_t e0 = __ldg(P.grid.offsets + c), e1 = __ldg(P.grid.offsets + c + 1);
-            const int32_t part = P.src.obj_part ? __ldg(P.src.obj_part + s) : 0;
-            for (int32_t e = e0; e < e1; ++e) {
-                const int32_t t = __ldg(P.grid.entries + e);
-                if (P.tgt.obj_part && __ldg(P.tgt.obj_part + t) != part) continue;
-                const float* ob = P.tgt.obj_box + 6 * (int64_t)t;
-                if (__ldg(ob) <= p.x && p.x <= __ldg(ob + 3) && __ldg(ob + 1) <= p.y && p.y <= __ldg(ob + 4) &&
-                    __ldg(ob + 5) >= p.z)
-                    candidate(t);
-            }
-            finish();
-            continue;
-        }
-        int first, count;
-        int node = traversal_start(P.src, P.objs, (int32_t)s, first, count);
-        if (node < 0) {
-            leaf(first, count);
-            finish();
-            continue;
-        }
-        int stack[kStackSize];
-        int sp = 0;
-        for (;;) {
-            ++n_nodes;
-            const Node* nd = P.objs.nodes + node;
-            const float4 bx = __ldg(&nd->bx), by = __ldg(&nd->by), bz = __ldg(&nd->bz);
-            const int4 ch = __ldg(&nd->ch);
-            bool h0 = bx.x <= p.x && p.x <= bx.y && by.x <= p.y && p.y <= by.y && bz.y >= p.z;
-            bool h1 = bx.z <= p.x && p.x <= bx.w && by.z <= p.y && p.y <= by.w && bz.w >= p.z;
-            if (h0 && ch.x < 0) {
-                leaf(~ch.x, ch.z & 0xFF);
-                h0 = false;
-            }
-            if (h1 && ch.y < 0) {
-                leaf(~ch.y, (ch.z >> 8) & 0xFF);
-                h1 = false;
-            }
-            if (h0 && h1) {
-                if (sp >= kStackSize) {
-                    if (lane == 0) atomicOr(P.err, ERR_STACK_OVERFLOW);
-                    break;
-                }
-                stack[sp++] = ch.y;
-                node = ch.x;
-            } else if (h0) {
-                node = ch.x;
-            } else if (h1) {
-                node = ch.y;
-            } else {
-                if (sp == 0) break;
-                node = stack[--sp];
-            }
-        }
-        finish();
-    }
-    // per-lane test and ambiguity counts; rays and node visits once per warp
-    flush_counter(&P.ctr->tri_tests, n_tests);
-    flush_counter(&P.ctr->fp32_ambiguous, pc.fp32_ambiguous);
-    flush_counter(&P.ctr->fp64_ambiguous, pc.fp64_ambiguous);
-    flush_counter(&P.ctr->parity_rays, lane == 0 ? n_rays : 0u);
-    flush_counter(&P.ctr->node_visits, lane == 0 ? n_nodes : 0u);
 }
 
 // Column grid of a dataset's object boxes in `mem` (grid_bytes(n) bytes).
@@ -2193,72 +1742,6 @@ int column_grid_fill(pierce_ctx* ctx, const DevDataset& tgt, void* mem, int32_t*
     return check_cuda(cudaGetLastError(), "column grid");
 }
 
-int launch_parity_objects(pierce_ctx* ctx, const DevDataset& src, const DevDataset& objs, const DevDataset& tgt,
-                          const ColumnGrid* grid, int swap, uint64_t* table, uint32_t* parity, uint64_t slots,
-                          int64_t src_lo, int64_t src_hi) {
-    if (src_hi < 0) src_hi = src.num_objects;
-    src_lo = std::max<int64_t>(src_lo, 0);
-    src_hi = std::min<int64_t>(src_hi, src.num_objects);
-    if (src_hi <= src_lo || !tgt.obj_range) return PIERCE_OK;
-    ParityObjParams P;
-    P.src = src;
-    P.src_lo = src_lo;
-    P.src_hi = src_hi;
-    P.grid = grid ? *grid : ColumnGrid{};
-    P.objs = objs;
-    P.tgt = tgt;
-    P.swap = swap;
-    P.table = table;
-    P.parity = parity;
-    P.mask = slots - 1;
-    P.err = ctx->d_err;
-    P.ctr = ctx->d_counters;
-    P.track_k = 0;
-    P.track_ids = nullptr;
-    P.track_hits = nullptr;
-    P.track_crossed = nullptr;
-    P.track_overflow = nullptr;
-    const int64_t warps = src_hi - src_lo;
-    const unsigned blocks = (unsigned)std::max<int64_t>(1, std::min<int64_t>((warps + 3) / 4,
-                                                                             (int64_t)ctx->sm_count * 32));
-    k_parity_objects<false><<<blocks, 128, 0, ctx->stream>>>(P);
-    ctx->launches += 1;
-    return check_cuda(cudaGetLastError(), "parity (object pairs) kernel");
-}
-
-// Parity-ray diagnostics of src's objects against tgt over tgt's column
-// grid: ids[src.num_objects * k] (preset to -1 by the caller), hits (same
-// shape), crossed and overflow (src.num_objects each; entries of objects
-// without triangles are left as they are).
-int launch_parity_tracking(pierce_ctx* ctx, const DevDataset& src, const DevDataset& tgt, const ColumnGrid& grid,
-                           int32_t k, int32_t* ids, uint32_t* hits, uint32_t* crossed, uint32_t* overflow) {
-    if (src.num_objects <= 0 || !tgt.obj_range || grid.nx <= 0) return PIERCE_OK;
-    ParityObjParams P;
-    P.src = src;
-    P.src_lo = 0;
-    P.src_hi = src.num_objects;
-    P.grid = grid;
-    P.objs = DevDataset{};
-    P.tgt = tgt;
-    P.swap = 0;
-    P.table = nullptr;
-    P.parity = nullptr;
-    P.mask = 0;
-    P.err = ctx->d_err;
-    P.ctr = ctx->d_counters;
-    P.track_k = k;
-    P.track_ids = ids;
-    P.track_hits = hits;
-    P.track_crossed = crossed;
-    P.track_overflow = overflow;
-    const int64_t warps = src.num_objects;
-    const unsigned blocks = (unsigned)std::max<int64_t>(1, std::min<int64_t>((warps + 3) / 4,
-                                                                             (int64_t)ctx->sm_count * 32));
-    k_parity_objects<true><<<blocks, 128, 0, ctx->stream>>>(P);
-    ctx->launches += 1;
-    return check_cuda(cudaGetLastError(), "parity tracking kernel");
-}
-
 int compact_table(pierce_ctx* ctx, const uint64_t* table, uint64_t slots, uint64_t* out, uint64_t cap,
                   unsigned long long* d_count) {
     k_compact<<<grid_cap(ctx, (int64_t)slots, 256), 256, 0, ctx->stream>>>(table, slots, out, d_count, cap);
@@ -2298,28 +1781,6 @@ int launch_containment_candidates(pierce_ctx* ctx, const uint64_t* ptable, const
     k_keep_candidates<<<grid_cap(ctx, nb, 256), 256, 0, ctx->stream>>>(act_b, nb);
     ctx->launches += 3;
     return check_cuda(cudaGetLastError(), "containment candidates");
-}
-
-int launch_containment_pairs(pierce_ctx* ctx, const uint64_t* ptable, const uint32_t* parity, uint64_t pslots,
-                             const DevDataset& a, const DevDataset& b, uint64_t* out, unsigned long long* count,
-                             uint64_t cap, unsigned long long* fallback) {
-    if (!a.obj_range || !b.obj_range)
-        return set_error(PIERCE_ERR_INVALID_ARGUMENT, "containment by pairs: objects must be stored contiguously");
-    PairParams P;
-    P.ptable = ptable;
-    P.parity = parity;
-    P.pslots = pslots;
-    P.a = a;
-    P.b = b;
-    P.out = out;
-    P.count = count;
-    P.cap = cap;
-    P.fallback = fallback;
-    P.ctr = ctx->d_counters;
-    const int64_t blocks = std::min<int64_t>(((int64_t)pslots + kPairThreads - 1) / kPairThreads, (int64_t)ctx->sm_count * 8);
-    k_containment_pairs<<<(unsigned)std::max<int64_t>(blocks, 1), kPairThreads, 0, ctx->stream>>>(P);
-    ctx->launches += 1;
-    return check_cuda(cudaGetLastError(), "containment by pairs");
 }
 
 // Grid selectivity estimate per matched cell (estimateSelectivityKernel,

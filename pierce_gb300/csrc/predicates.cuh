@@ -227,6 +227,12 @@ static __device__ __noinline__ int orient3d_fp64_or_exact(float3 a, float3 b, fl
 }
 
 static __device__ __noinline__ int orient2d_fp64_or_exact(float3 a, float3 b, float3 c, int i, int j, PredCounters& pc) {
+    // two points that coincide in the plane make the determinant exactly zero
+    // (a vertex shared by duplicated meshes: every one of the 1,284 expansion
+    // evaluations of the 2 x 50,000 ellipsoid intersection, 250 of B's meshes
+    // duplicates, was such a case)
+    const float ai = fcomp(a, i), aj = fcomp(a, j), bi = fcomp(b, i), bj = fcomp(b, j), ci = fcomp(c, i), cj = fcomp(c, j);
+    if ((ai == bi && aj == bj) || (ai == ci && aj == cj) || (bi == ci && bj == cj)) return 0;
     const double u0 = (double)fcomp(b, i) - fcomp(a, i), u1 = (double)fcomp(b, j) - fcomp(a, j);
     const double v0 = (double)fcomp(c, i) - fcomp(a, i), v1 = (double)fcomp(c, j) - fcomp(a, j);
     const double det = u0 * v1 - u1 * v0;
@@ -414,6 +420,87 @@ __device__ __forceinline__ int seg_tri_fp32_class(float3 p, float3 q, float3 a, 
     if ((s1 > 0 || s2 > 0 || s3 > 0) && (s1 < 0 || s2 < 0 || s3 < 0)) return SEG_MISS;
     if (s1 == 0 || s2 == 0 || s3 == 0) return SEG_AMBIGUOUS;
     return SEG_HIT;
+}
+
+// Closed triangle against closed triangle in float32.  Both plane-side tests
+// with the forward error bound of certain_sign first; when every side is
+// certain and both triangles straddle the other's plane, the two segments in
+// which they cut the planes' common line overlap exactly when two
+// orientations agree (Guigue and Devillers, "Fast and Robust
+// Triangle-Triangle Overlap Test Using Orientation Predicates", 2003).  A
+// vertex of one that is a vertex of the other (duplicated meshes, contacts)
+// is a common point when one of the two certainly has an area.
+// SEG_AMBIGUOUS: some sign is not certain.
+__device__ __forceinline__ int tri_tri_fp32_class(float3 a0, float3 a1, float3 a2, float3 b0, float3 b1, float3 b2) {
+    int s0, s1, s2, t0, t1, t2;
+    bool area;
+    {
+        const float3 u = f3sub(a1, a0), v = f3sub(a2, a0);
+        const float3 n = f3cross(u, v), np = f3cross_perm(u, v);
+        const float3 p = f3sub(b0, a0), q = f3sub(b1, a0), r = f3sub(b2, a0);
+        t0 = certain_sign(f3dot(p, n), f3dot_abs(p, np), 12.0f);
+        t1 = certain_sign(f3dot(q, n), f3dot_abs(q, np), 12.0f);
+        t2 = certain_sign(f3dot(r, n), f3dot_abs(r, np), 12.0f);
+        if (t0 && t0 == t1 && t0 == t2) return SEG_MISS;
+        area = certain_sign(n.x, np.x, 8.0f) || certain_sign(n.y, np.y, 8.0f) || certain_sign(n.z, np.z, 8.0f);
+    }
+    {
+        const float3 u = f3sub(b1, b0), v = f3sub(b2, b0);
+        const float3 n = f3cross(u, v), np = f3cross_perm(u, v);
+        const float3 p = f3sub(a0, b0), q = f3sub(a1, b0), r = f3sub(a2, b0);
+        s0 = certain_sign(f3dot(p, n), f3dot_abs(p, np), 12.0f);
+        s1 = certain_sign(f3dot(q, n), f3dot_abs(q, np), 12.0f);
+        s2 = certain_sign(f3dot(r, n), f3dot_abs(r, np), 12.0f);
+        if (s0 && s0 == s1 && s0 == s2) return SEG_MISS;
+        area = area || certain_sign(n.x, np.x, 8.0f) || certain_sign(n.y, np.y, 8.0f) || certain_sign(n.z, np.z, 8.0f);
+    }
+    if (!s0 || !s1 || !s2 || !t0 || !t1 || !t2) {
+        const bool shared = same_point(a0, b0) || same_point(a0, b1) || same_point(a0, b2) || same_point(a1, b0) ||
+                            same_point(a1, b1) || same_point(a1, b2) || same_point(a2, b0) || same_point(a2, b1) ||
+                            same_point(a2, b2);
+        return shared && area ? SEG_HIT : SEG_AMBIGUOUS;
+    }
+    // a0 and b0: the vertices alone on their side (rotations keep the planes' orientation)
+    if (s0 == s2) { const float3 x = a0; a0 = a1; a1 = a2; a2 = x; s0 = s1; }          // a1 alone
+    else if (s0 == s1) { const float3 x = a0; a0 = a2; a2 = a1; a1 = x; s0 = s2; }     // a2 alone
+    if (t0 == t2) { const float3 x = b0; b0 = b1; b1 = b2; b2 = x; t0 = t1; }
+    else if (t0 == t1) { const float3 x = b0; b0 = b2; b2 = b1; b1 = x; t0 = t2; }
+    // both lone vertices on the positive side of the other plane: a lone
+    // vertex below it turns round when that plane's triangle does
+    if (s0 < 0) { const float3 x = b1; b1 = b2; b2 = x; }
+    if (t0 < 0) { const float3 x = a1; a1 = a2; a2 = x; }
+    // apart when (b1 - a0) . ((a1 - a0) x (b0 - a0)) or (b2 - a0) . ((b0 -
+    // a0) x (a2 - a0)) is positive
+    const float3 p = f3sub(b0, a0), u = f3sub(a1, a0), v = f3sub(b1, a0), w = f3sub(a2, a0), x = f3sub(b2, a0);
+    const float3 c1 = f3cross(u, p), m1 = f3cross_perm(u, p);
+    const int o1 = certain_sign(f3dot(v, c1), f3dot_abs(v, m1), 12.0f);
+    const float3 c2 = f3cross(p, w), m2 = f3cross_perm(p, w);
+    const int o2 = certain_sign(f3dot(x, c2), f3dot_abs(x, m2), 12.0f);
+    if (o1 > 0 || o2 > 0) return SEG_MISS;
+    if (o1 == 0 || o2 == 0) return SEG_AMBIGUOUS;
+    return SEG_HIT;
+}
+
+
+// The edge definition, exact: an edge of one triangle meets the other.
+static __device__ __noinline__ bool tri_tri_exact(float3 a0, float3 a1, float3 a2, float3 b0, float3 b1, float3 b2,
+                                           PredCounters& pc) {
+    bool hit = false;
+#pragma unroll 1
+    for (int side = 0; side < 2 && !hit; ++side) {
+#pragma unroll 1
+        for (int k = 0; k < 3 && !hit; ++k) {
+            hit = seg_tri_exact(b0, b1, a0, a1, a2, pc);
+            const float3 x = b0;
+            b0 = b1;
+            b1 = b2;
+            b2 = x;
+        }
+        const float3 x = a0, y = a1, z = a2;
+        a0 = b0; a1 = b1; a2 = b2;
+        b0 = x; b1 = y; b2 = z;
+    }
+    return hit;
 }
 
 // Plain float32 Moller-Trumbore on the segment p->q (no fallback).
