@@ -110,6 +110,8 @@ enum : int {
     SLOT_LISTED_A = 36,       // joins by triangle pairs: A's listed groups
     SLOT_MASKS = 41,          // kept groups per chunk of a culling pass
     SLOT_SPILL = 37,          // ... their work words and entries left for the next round
+    SLOT_TRI_BOXES_A = 43,    // boxes of the per-join soups' triangles
+    SLOT_TRI_BOXES_B = 44,
     SLOT_CONT_WORDS = 42,     // containment: counts of its lists
     SLOT_ENTRY_AB = 38,       // rays from triangles: entry nodes of the listed groups, A->B
     SLOT_ENTRY_BA = 39,
@@ -1701,6 +1703,16 @@ struct Join {
         return PIERCE_OK;
     }
 
+    // Boxes of a side's n kept triangles.  Short of memory there are none:
+    // the walks read the triangles, and the join traces rays.
+    int tri_boxes(int sd, size_t n, float** out) {
+        void* p = nullptr;
+        const int s = scratch(ctx, sd ? SLOT_TRI_BOXES_B : SLOT_TRI_BOXES_A, 24 * n, &p);
+        if (s && s != PIERCE_ERR_OUT_OF_MEMORY) return s;
+        *out = s ? nullptr : static_cast<float*>(p);
+        return PIERCE_OK;
+    }
+
     // One side's per-join hierarchy over its kept groups.
     int group_hierarchy(int sd) {
         pierce_dataset* ds = sd ? B : A;
@@ -1716,11 +1728,13 @@ struct Join {
         if (int s = scratch(ctx, sd ? SLOT_RED_SOUP_B : SLOT_RED_SOUP_A, 48 * (size_t)G * m, &sp)) return s;
         if (int s = scratch(ctx, sd ? SLOT_RED_NODES_B : SLOT_RED_NODES_A, 64 * m + 8 * (size_t)parts, &np)) return s;
         if (int s = scratch(ctx, SLOT_GROUPS, 24 * m, &gp)) return s;
+        float* tb = nullptr;
+        if (int s = tri_boxes(sd, G * m, &tb)) return s;
         int2* roots = parts ? reinterpret_cast<int2*>((Node*)np + m) : nullptr;
         BvhShape sh;
         if (int s = build_group_lbvh(ctx, ds->view(), ds->d_tri_to_object, group_list[sd], words + 11 + sd, n, G,
                                      reinterpret_cast<uint32_t*>(words + 20 + 8 * sd), words + 16 + 8 * sd, gp,
-                                     (float4*)sp, (Node*)np, &sh, parts, roots))
+                                     (float4*)sp, tb, (Node*)np, &sh, parts, roots))
             return s;
         DevDataset& v = sd ? vb : va;
         v.soup = (const float4*)sp;
@@ -1729,6 +1743,8 @@ struct Join {
         v.root_is_leaf = sh.root_is_leaf;
         v.root_leaf_count = sh.root_leaf_count;
         v.part_roots = roots;
+        v.tri_boxes = tb;
+        v.tri_box_unit = std::min(G, 4);
         // four-wide copy in every traversal mode: it also culls the other
         // side's chunks and filters its groups and rays
         if (int s = wide_nodes(v, sh.num_nodes, sd ? SLOT_NODES4_B : SLOT_NODES4_A, true, G)) return s;
@@ -1743,7 +1759,7 @@ struct Join {
         pairs_route = false;
         const int G = group_size(join_leaf(o, A));
         if (!triangle_pairs_wanted() || G != group_size(join_leaf(o, B)) || va.root_is_leaf || !va.nodes4 ||
-            va.num_tris / G >= (int64_t(1) << 27) || !triangle_edges(0, va.num_tris) ||
+            !va.tri_boxes || va.num_tris / G >= (int64_t(1) << 27) || !triangle_edges(0, va.num_tris) ||
             group_bound[1] * G >= (int64_t(1) << 30))
             return PIERCE_OK;
         if (!triangle_edges(1, group_bound[1] * G)) {
@@ -1760,11 +1776,15 @@ struct Join {
         if (int s = scratch(ctx, SLOT_RED_SOUP_B, 48 * (size_t)G * m, &sp)) return s;
         if (int s = scratch(ctx, SLOT_GROUPS, 24 * m, &gp)) return s;
         if (int s = scratch(ctx, SLOT_LISTED_A, (size_t)(va.num_tris / G) + 64, &fp)) return s;
+        float* tb = nullptr;
+        if (int s = tri_boxes(1, G * m, &tb)) return s;
+        if (!tb) return PIERCE_OK;
         if (int s = group_units(ctx, B->view(), B->d_tri_to_object, group_list[1], words + 12, bound, G, (float*)gp,
-                                (float4*)sp))
+                                (float4*)sp, tb))
             return s;
         pj.bsoup = (const float4*)sp;
         pj.gbox = (const float*)gp;
+        pj.b_tri_boxes = tb;
         pj.b_count = words + 12;
         pj.b_bound = bound;
         pj.b_part = B->d_obj_part;
@@ -1772,9 +1792,9 @@ struct Join {
         pj.a_listed = (uint8_t*)fp;
         // entries left for the next round: up to 512 of each resident warp's
         pj.spill_cap = std::min<uint64_t>((uint64_t)std::max<int64_t>(bound, 32) * 512, 1ull << 22);
-        if (int s = scratch(ctx, SLOT_SPILL, 64 + 2 * 8 * pj.spill_cap, &wp)) return s;
+        if (int s = scratch(ctx, SLOT_SPILL, 128 + 2 * 8 * pj.spill_cap, &wp)) return s;
         pj.work = static_cast<unsigned long long*>(wp);
-        pj.spill = reinterpret_cast<uint2*>(pj.work + 8);
+        pj.spill = reinterpret_cast<uint2*>(pj.work + 16);
         pj.amb_queue = amb_queue;
         pj.amb_cap = amb_cap;
         pairs_route = true;

@@ -96,6 +96,10 @@ struct DevDataset {
     const float* edge_chunk_box;
     int edges_grouped;  // edges stored grouped by source object
     int soup_boxes;     // the soup holds boxes as degenerate triangles (lo, hi, hi), not triangles
+    // optional boxes of the soup's triangles (group hierarchies): per
+    // tri_box_unit = min(G, 4) triangles 6 rows lo.xyz hi.xyz of that many floats
+    const float* tri_boxes;
+    int tri_box_unit;
 };
 
 // Open-addressing set of pair keys (a power of two of slots, empty slot all
@@ -134,7 +138,7 @@ struct RayOpts {
     int entry_group = 1;
 };
 
-constexpr int kScratchSlots = 44;
+constexpr int kScratchSlots = 46;
 constexpr int kPairSetSlot = 40;  // the joins' pair table
 
 // Uniform xy grid over a dataset's object boxes: per cell the objects whose
@@ -153,12 +157,13 @@ struct PairJoin {
     // the walking side: B's kept groups, without a hierarchy
     const float4* bsoup = nullptr;               // their triangles, G each
     const float* gbox = nullptr;                 // their boxes
+    const float* b_tri_boxes = nullptr;          // their triangles' boxes (DevDataset::tri_boxes)
     const unsigned long long* b_count = nullptr; // their number, at most b_bound
     int64_t b_bound = 0;
     const int32_t* b_part = nullptr;             // partition per B object (partitioned joins)
     int G = 4;                                   // triangles per group, both sides
     uint8_t* a_listed = nullptr;                 // a byte per A leaf group
-    unsigned long long* work = nullptr;          // 8 words: deferred-test count, cursors, left-over counts
+    unsigned long long* work = nullptr;          // 16 words: deferred-test count, cursors, left-over counts
     uint2* spill = nullptr;                      // two buffers of entries left for the next round
     uint64_t spill_cap = 0;
     unsigned long long* amb_queue = nullptr;
@@ -292,7 +297,7 @@ struct pierce_dataset {
     int grid_ready = 0;
 
     pgpu::DevDataset view() const {
-        pgpu::DevDataset v;
+        pgpu::DevDataset v{};
         v.soup = d_soup;
         v.nodes = d_nodes;
         v.nodes4 = nullptr;
@@ -382,17 +387,18 @@ size_t group_cull_bytes(int64_t nt, int G);
 int cull_groups(pierce_ctx* ctx, const DevDataset& src, const int32_t* t2o, const uint8_t* active,
                 const DevDataset& other, bool filter, int G, void* mem, uint32_t* list, unsigned long long* d_count,
                 int32_t* d_mixed, uint32_t* bounds, unsigned long long* zero);
-// the listed groups (at most `bound`) as boxes and a soup in list order
+// the listed groups (at most `bound`) as boxes and a soup in list order, with
+// their triangles' boxes (DevDataset::tri_boxes) where tri_boxes is given
 int group_units(pierce_ctx* ctx, const DevDataset& src, const int32_t* t2o, const uint32_t* list,
-                const unsigned long long* d_count, int64_t bound, int G, float* gbox, float4* soup);
+                const unsigned long long* d_count, int64_t bound, int G, float* gbox, float4* soup, float* tri_boxes);
 // hierarchy over the n listed groups, one per leaf (group_scratch: 24 bytes
 // per group); soup in leaf order, G triangles per leaf.  The binary nodes'
 // leaves count groups until group_leaves turns them into soup ranges
 // (collapse4 with G does so for the four-wide copy).
 int build_group_lbvh(pierce_ctx* ctx, const DevDataset& src, const int32_t* t2o, const uint32_t* list,
                      const unsigned long long* d_count, int64_t n, int G, uint32_t* bounds,
-                     unsigned long long* wave_count, void* group_scratch, float4* soup, Node* nodes, BvhShape* shape,
-                     int32_t num_parts, int2* part_roots);
+                     unsigned long long* wave_count, void* group_scratch, float4* soup, float* tri_boxes, Node* nodes,
+                     BvhShape* shape, int32_t num_parts, int2* part_roots);
 int group_leaves(pierce_ctx* ctx, Node* nodes, int64_t num_nodes, int G);
 
 // join.cu, pairs.cu: the pair tests of a join by triangle pairs into a pair

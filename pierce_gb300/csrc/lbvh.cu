@@ -1290,13 +1290,15 @@ __global__ void __launch_bounds__(256) k_group_prims(const float* __restrict__ v
 
 // Triangle soup of kept groups, G triangles each: position j holds group
 // list[order[j]] (a hierarchy's leaf order), or list[j] without an order.
+// tri_boxes: the triangles' boxes by rows of min(G, 4), 24 bytes a triangle
+// beside its 48, for the walks that test a leaf's boxes.
 __global__ void __launch_bounds__(256) k_group_soup(const uint32_t* __restrict__ list,
                                                     const uint32_t* __restrict__ order,
                                                     const unsigned long long* __restrict__ count, int G,
                                                     const float* __restrict__ verts, const uint32_t* __restrict__ idx,
                                                     const int32_t* __restrict__ t2o, int64_t nt,
-                                                    float4* __restrict__ soup) {
-    const int per_chunk = 32 / G;
+                                                    float4* __restrict__ soup, float* __restrict__ tri_boxes) {
+    const int per_chunk = 32 / G, unit = min(G, 4);
     const int64_t n = (int64_t)*count * G;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         const int64_t j = i / G;
@@ -1308,6 +1310,15 @@ __global__ void __launch_bounds__(256) k_group_soup(const uint32_t* __restrict__
         soup[3 * i + 0] = make_float4(a.x, a.y, a.z, __int_as_float(__ldg(t2o + t)));
         soup[3 * i + 1] = make_float4(b.x, b.y, b.z, __int_as_float((int)t));
         soup[3 * i + 2] = make_float4(c.x, c.y, c.z, 0.0f);
+        if (tri_boxes) {
+            float* r = tri_boxes + 6 * (i & ~(int64_t)(unit - 1)) + (i & (unit - 1));
+            r[0] = fminf(a.x, fminf(b.x, c.x));
+            r[unit] = fminf(a.y, fminf(b.y, c.y));
+            r[2 * unit] = fminf(a.z, fminf(b.z, c.z));
+            r[3 * unit] = fmaxf(a.x, fmaxf(b.x, c.x));
+            r[4 * unit] = fmaxf(a.y, fmaxf(b.y, c.y));
+            r[5 * unit] = fmaxf(a.z, fmaxf(b.z, c.z));
+        }
     }
 }
 
@@ -1505,7 +1516,7 @@ int cull_groups(pierce_ctx* ctx, const DevDataset& src, const int32_t* t2o, cons
 }
 
 int group_units(pierce_ctx* ctx, const DevDataset& src, const int32_t* t2o, const uint32_t* list,
-                const unsigned long long* d_count, int64_t bound, int G, float* gbox, float4* soup) {
+                const unsigned long long* d_count, int64_t bound, int G, float* gbox, float4* soup, float* tri_boxes) {
     if (bound <= 0) return PIERCE_OK;
     cudaStream_t st = ctx->stream;
 #define PG_PRIMS(g)                                                                                                  \
@@ -1514,15 +1525,15 @@ int group_units(pierce_ctx* ctx, const DevDataset& src, const int32_t* t2o, cons
     PG_BY_GROUP(PG_PRIMS);
 #undef PG_PRIMS
     k_group_soup<<<grid_for(ctx, bound * G, 256), 256, 0, st>>>(list, nullptr, d_count, G, src.verts, src.idx, t2o,
-                                                                src.num_tris, soup);
+                                                                src.num_tris, soup, tri_boxes);
     ctx->launches += 2;
     return check_cuda(cudaGetLastError(), "group units");
 }
 
 int build_group_lbvh(pierce_ctx* ctx, const DevDataset& src, const int32_t* t2o, const uint32_t* list,
                      const unsigned long long* d_count, int64_t n, int G, uint32_t* bounds,
-                     unsigned long long* wave_count, void* group_scratch, float4* soup, Node* nodes, BvhShape* shape,
-                     int32_t num_parts, int2* part_roots) {
+                     unsigned long long* wave_count, void* group_scratch, float4* soup, float* tri_boxes, Node* nodes,
+                     BvhShape* shape, int32_t num_parts, int2* part_roots) {
     cudaStream_t st = ctx->stream;
     const bool parts = src.obj_part && num_parts > 0 && part_roots;
     shape->leaf_size = G;
@@ -1572,7 +1583,7 @@ int build_group_lbvh(pierce_ctx* ctx, const DevDataset& src, const int32_t* t2o,
     }
     const uint32_t* order = vals + n;
     k_group_soup<<<grid_for(ctx, n * G, B), B, 0, st>>>(list, order, d_count, G, src.verts, src.idx, t2o, src.num_tris,
-                                                        soup);
+                                                        soup, tri_boxes);
     ctx->launches += 3;
     if (n == 1) {
         if (parts) {

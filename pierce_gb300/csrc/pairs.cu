@@ -15,6 +15,7 @@
 #include "common.cuh"
 #include "hash.cuh"
 #include "predicates.cuh"
+#include "walk.cuh"
 
 namespace pgpu {
 
@@ -25,6 +26,8 @@ constexpr int kPairUnits = 32;       // B groups a warp walks together
 constexpr int kPairStack = 512;      // walk entries per warp
 constexpr int kPairReserve = 144;    // of them left for a single entry's subtree (48 levels x 3)
 constexpr int kPairLeafQueue = 160;  // reached (group, leaf) pairs: < 32 left over + 32 x 4
+constexpr int kPairShare = 2;        // fetches per warp at least
+constexpr int kPairSeen = 64;        // keys a warp remembers
 constexpr int kPairTriQueue = 64;    // triangle pairs: < 32 left over + 32
 
 struct WarpWork {
@@ -33,6 +36,7 @@ struct WarpWork {
     uint32_t stack[kPairStack];      // node << 5 | unit
     uint32_t leafq[kPairLeafQueue];  // leaf group << 5 | unit
     uint2 triq[kPairTriQueue];       // (A soup triangle, B soup triangle)
+    unsigned long long seen[kPairSeen];  // keys this warp has added, by their hash
 };
 
 }  // namespace
@@ -42,6 +46,7 @@ struct PairParams {
     const float4* bsoup;                  // B's kept groups, G triangles each
     const unsigned long long* b_count;    // their number
     const float* gbox;                    // their boxes
+    const float* b_tri_boxes;             // their triangles' boxes, as a.tri_boxes
     const int32_t* b_part;                // partition per B object (partitioned joins)
     int G;                                // triangles per group, both sides
     PairSet set;
@@ -54,13 +59,14 @@ struct PairParams {
     uint8_t* a_listed;                    // per A leaf group: meets the box of a kept B triangle
     // rounds: entries (group, node) left by the round before (null: every
     // group from the root), and where a warp leaves what is still on its
-    // stack after `budget` steps (spill null: it carries on)
+    // stack after `budget` steps, or when it finds no groups left to fetch
+    // after another `look` steps (spill null: it carries on)
     const uint2* entries;
     const unsigned long long* n_entries;
     uint2* spill;
     unsigned long long* n_spill;
     uint64_t spill_cap;
-    int budget;
+    int look, budget;
 };
 
 // Each warp takes a few B groups (units) at a time and walks them over A's
@@ -79,8 +85,17 @@ struct PairParams {
 // 12,007 x 9,001 meshes 64.2 -> 8.9 ms (67 M rays and 1.8 G node visits
 // become 3.2 M walks and 123 M visits), 2 x 50,000 ellipsoids 1.13 -> 0.35
 // ms, 400,000 x 100,000 ellipsoids 1.86 -> 0.54 ms, 64 batched joins 28.3 ->
-// 4.2 ms.  6 blocks of 128 per SM (80 registers): 8.86 ms on the dense join
-// against 9.42 with 8 blocks (64 registers, spills) and 9.37 with 5.
+// 4.2 ms.
+//
+// Then bound by L1 (82 %: lanes read different lines) and issue (50 %).  A
+// leaf's triangle boxes are read as stored (12 scattered loads a leaf pair
+// instead of 24, no minima and maxima): dense 8.73 -> 7.70 ms; a warp
+// remembers keys it has added (hits repeat the same pair of meshes some 100
+// times, each a trip to L2): 7.19 ms, batch 4.20 -> 4.03 ms; long walks go on
+// as soon as warps run out of work (launch_tri_pairs): 6.35 and 1.73 ms.  B's
+// boxes in shared memory instead made no difference (7.67 ms).  6 blocks of
+// 128 per SM (80 registers): 7.19 ms against 7.37 with 7 (72, spills) and
+// 7.80 with 8.
 template <int U, bool BIG, bool DEFER>
 __global__ void __launch_bounds__(32 * kPairWarps, DEFER ? 6 : 4) k_tri_pairs(PairParams P) {
     __shared__ WarpWork work[kPairWarps];
@@ -91,18 +106,20 @@ __global__ void __launch_bounds__(32 * kPairWarps, DEFER ? 6 : 4) k_tri_pairs(Pa
     if (!P.entries && blockIdx.x == 0 && threadIdx.x == 0) P.ctr->kept_b = (unsigned long long)n;
     // units per fetch: few when there are few, so that all warps share them
     const int64_t warps = (int64_t)gridDim.x * kPairWarps;
-    const int per = (int)min((int64_t)kPairUnits, max((int64_t)1, n / warps));
+    const int per = (int)min((int64_t)kPairUnits, max((int64_t)1, n / (warps * kPairShare)));
     const int G = BIG ? P.G : U;
     const int side = BIG ? G / U : 1;  // blocks per side of a leaf pair
     PredCounters pc{0, 0};
     uint32_t nodes = 0, tests = 0, hits = 0, probes = 0, ambiguous = 0;
-    int sp = 0, lq = 0, tq = 0, steps = 0;
+    int limit = P.look, sp = 0, lq = 0, tq = 0, steps = 0;
     bool more = true, finish = false;
     // this lane's reached leaf, the block of it in hand and its pairs left:
     // bit U j + i for A triangle ta + j, B triangle tb + i
     int blk = side * side;
     uint32_t leaf_a = 0, leaf_b = 0, mask = 0;
     bool has_leaf = false;
+    for (int i = lane; i < kPairSeen; i += 32) W.seen[i] = kEmptyKey;
+    __syncwarp();
     float ga[6] = {0, 0, 0, 0, 0, 0};
     for (;;) {
         if (tq >= 32 || (tq > 0 && finish)) {
@@ -133,7 +150,14 @@ __global__ void __launch_bounds__(32 * kPairWarps, DEFER ? 6 : 4) k_tri_pairs(Pa
                 }
                 if (hit) {
                     ++hits;
-                    hash_add(P.set, pack_key(__float_as_int(a0.w), __float_as_int(b0.w)), P.err, probes);
+                    const unsigned long long key = pack_key(__float_as_int(a0.w), __float_as_int(b0.w));
+                    volatile unsigned long long* seen = &W.seen[(uint32_t)(fmix64(key) >> 32) & (kPairSeen - 1)];
+                    if (*seen == key) {  // in the set already
+                        ++probes;
+                    } else {
+                        hash_add(P.set, key, P.err, probes);
+                        *seen = key;
+                    }
                 }
             }
             __syncwarp();
@@ -158,25 +182,19 @@ __global__ void __launch_bounds__(32 * kPairWarps, DEFER ? 6 : 4) k_tri_pairs(Pa
             const int bi = BIG ? blk % side : 0, bj = BIG ? blk / side : 0;
             ++blk;
             if (has_leaf) {
-                const float4* bs = P.bsoup + 3 * ((size_t)leaf_b * G + bi * U);
-                const float4* as = P.a.soup + 3 * ((size_t)leaf_a * G + bj * U);
+                const TriBoxes<U> A(P.a.tri_boxes + 6 * U * ((size_t)leaf_a * side + bj));
+                const TriBoxes<U> B(P.b_tri_boxes + 6 * U * ((size_t)leaf_b * side + bi));
                 float3 blo[U], bhi[U];
 #pragma unroll
                 for (int i = 0; i < U; ++i) {
-                    const float4 x = __ldg(bs + 3 * i), y = __ldg(bs + 3 * i + 1), z = __ldg(bs + 3 * i + 2);
-                    blo[i] = make_float3(fminf(x.x, fminf(y.x, z.x)), fminf(x.y, fminf(y.y, z.y)),
-                                         fminf(x.z, fminf(y.z, z.z)));
-                    bhi[i] = make_float3(fmaxf(x.x, fmaxf(y.x, z.x)), fmaxf(x.y, fmaxf(y.y, z.y)),
-                                         fmaxf(x.z, fmaxf(y.z, z.z)));
+                    blo[i] = make_float3(B.v[0][i], B.v[1][i], B.v[2][i]);
+                    bhi[i] = make_float3(B.v[3][i], B.v[4][i], B.v[5][i]);
                 }
                 float3 ulo = make_float3(3.4e38f, 3.4e38f, 3.4e38f), uhi = make_float3(-3.4e38f, -3.4e38f, -3.4e38f);
 #pragma unroll
                 for (int j = 0; j < U; ++j) {
-                    const float4 x = __ldg(as + 3 * j), y = __ldg(as + 3 * j + 1), z = __ldg(as + 3 * j + 2);
-                    const float3 lo = make_float3(fminf(x.x, fminf(y.x, z.x)), fminf(x.y, fminf(y.y, z.y)),
-                                                  fminf(x.z, fminf(y.z, z.z)));
-                    const float3 hi = make_float3(fmaxf(x.x, fmaxf(y.x, z.x)), fmaxf(x.y, fmaxf(y.y, z.y)),
-                                                  fmaxf(x.z, fmaxf(y.z, z.z)));
+                    const float3 lo = make_float3(A.v[0][j], A.v[1][j], A.v[2][j]);
+                    const float3 hi = make_float3(A.v[3][j], A.v[4][j], A.v[5][j]);
 #pragma unroll
                     for (int i = 0; i < U; ++i)
                         if (box_overlap(lo.x, hi.x, lo.y, hi.y, lo.z, hi.z, blo[i], bhi[i])) mask |= 1u << (U * j + i);
@@ -209,10 +227,14 @@ __global__ void __launch_bounds__(32 * kPairWarps, DEFER ? 6 : 4) k_tri_pairs(Pa
                         ga[k] = 3.4e38f;
                         ga[3 + k] = -3.4e38f;
                     }
-                    for (int t = 0; t < 3 * G; ++t) {
-                        const float4 v = __ldg(P.a.soup + 3 * (size_t)leaf_a * G + t);
-                        ga[0] = fminf(ga[0], v.x); ga[1] = fminf(ga[1], v.y); ga[2] = fminf(ga[2], v.z);
-                        ga[3] = fmaxf(ga[3], v.x); ga[4] = fmaxf(ga[4], v.y); ga[5] = fmaxf(ga[5], v.z);
+                    for (int t = 0; t < side; ++t) {
+                        const TriBoxes<U> A(P.a.tri_boxes + 6 * U * ((size_t)leaf_a * side + t));
+#pragma unroll
+                        for (int j = 0; j < U; ++j)
+                            for (int k = 0; k < 3; ++k) {
+                                ga[k] = fminf(ga[k], A.v[k][j]);
+                                ga[3 + k] = fmaxf(ga[3 + k], A.v[3 + k][j]);
+                            }
                     }
                 }
             }
@@ -221,8 +243,17 @@ __global__ void __launch_bounds__(32 * kPairWarps, DEFER ? 6 : 4) k_tri_pairs(Pa
             continue;
         }
         if (sp > 0) {
-            if (P.spill && ++steps > P.budget) {
-                // a long walk: what is left of it goes to the next round
+            bool hand_on = false;
+            if (P.spill && ++steps >= limit) {
+                // a long walk, and nothing left to fetch (or a very long
+                // walk): what is left of it goes to the next round
+                unsigned long long at = 0;
+                if (lane == 0) at = __ldcg(P.cursor);
+                at = __shfl_sync(0xFFFFFFFFu, at, 0);
+                hand_on = steps >= P.budget || (int64_t)at >= n;
+                limit = min(steps + P.look, P.budget);
+            }
+            if (hand_on) {
                 unsigned long long at = 0;
                 if (lane == 0) at = atomicAdd(P.n_spill, (unsigned long long)sp);
                 at = __shfl_sync(0xFFFFFFFFu, at, 0);
@@ -233,6 +264,7 @@ __global__ void __launch_bounds__(32 * kPairWarps, DEFER ? 6 : 4) k_tri_pairs(Pa
                 }
                 sp -= fit;
                 steps = 0;
+                limit = P.look;
                 __syncwarp();
                 if (fit) continue;
             }
@@ -306,6 +338,7 @@ __global__ void __launch_bounds__(32 * kPairWarps, DEFER ? 6 : 4) k_tri_pairs(Pa
             sp = __popc(mn);
             lq = __popc(ml);
             steps = 0;
+            limit = P.look;
             more = base + per < n;
             __syncwarp();
             continue;
@@ -350,8 +383,10 @@ int launch_tri_pairs(pierce_ctx* ctx, const DevDataset& a, const PairJoin& j, co
     cudaStream_t st = ctx->stream;
     const int64_t na = a.num_tris / j.G;
     // words of j.work: [0] deferred tests, then per round [1 + 2 r] cursor, [2 + 2 r] spilled entries
-    constexpr int kRounds = 3;
+    constexpr int kRounds = 4;
     constexpr int kBudget = 192;
+    constexpr int kLook0 = 32, kLook1 = 16;
+    constexpr int64_t kShortWalk = 2048;
     cudaMemsetAsync(j.work, 0, (1 + 2 * kRounds) * sizeof(unsigned long long), st);
     cudaMemsetAsync(j.a_listed, 0, (size_t)na, st);
     PairParams P{};
@@ -359,6 +394,7 @@ int launch_tri_pairs(pierce_ctx* ctx, const DevDataset& a, const PairJoin& j, co
     P.bsoup = j.bsoup;
     P.b_count = j.b_count;
     P.gbox = j.gbox;
+    P.b_tri_boxes = j.b_tri_boxes;
     P.b_part = j.b_part;
     P.G = j.G;
     P.set = set;
@@ -374,15 +410,23 @@ int launch_tri_pairs(pierce_ctx* ctx, const DevDataset& a, const PairJoin& j, co
         // A group's walk is as long as what it meets (a coarse mesh's group
         // meets thousands of leaves of a fine one): a warp leaves what a
         // long walk still has on its stack to the next round, where it is
-        // spread over all warps (64 batched joins of levels 1 to 5: 12.2 ms
-        // in one round, 4.2 ms in three).
-        for (int r = 0; r < kRounds; ++r) {
+        // spread over all warps -- after kBudget steps, or when it looks (every
+        // kLook steps) and the groups have run out, so that other warps are
+        // idle.  64 batched joins of levels 1 to 5: 12.2 ms in one round, 4.0
+        // ms in three by budgets of 192 steps alone (3.0 ms by 96, 3.7 by 48),
+        // 1.73 ms by both rules in four rounds; looking every 16 steps in the
+        // first round too 1.65 ms, but 400,000 x 100,000 ellipsoids 0.50
+        // instead of 0.48 ms.  Where A has so few groups that one walk over
+        // all of them is short, one round does.
+        const int rounds = na <= kShortWalk ? 1 : kRounds;
+        for (int r = 0; r < rounds; ++r) {
             P.cursor = j.work + 1 + 2 * r;
-            P.entries = r ? j.spill + (r - 1) * j.spill_cap : nullptr;
+            P.entries = r ? j.spill + ((r - 1) & 1) * j.spill_cap : nullptr;
             P.n_entries = r ? j.work + 2 * r : nullptr;
-            P.spill = r + 1 < kRounds ? j.spill + r * j.spill_cap : nullptr;
+            P.spill = r + 1 < rounds ? j.spill + (r & 1) * j.spill_cap : nullptr;
             P.n_spill = j.work + 2 + 2 * r;
             P.spill_cap = j.spill_cap;
+            P.look = r ? kLook1 : kLook0;
             P.budget = kBudget;
 #define PG_PAIRS(U, BIG)                                                                \
     do {                                                                                \

@@ -49,6 +49,26 @@ __device__ __forceinline__ bool any_hit4(const Node4* nodes4, int node, const fl
     }
 }
 
+// Boxes of U consecutive soup triangles: rows lo.xyz hi.xyz.
+template <int U>
+struct TriBoxes {
+    float v[6][U];
+    __device__ __forceinline__ explicit TriBoxes(const float* rec) {
+#pragma unroll
+        for (int d = 0; d < 6; ++d) {
+            if constexpr (U == 4) {
+                const float4 x = __ldg(reinterpret_cast<const float4*>(rec) + d);
+                v[d][0] = x.x; v[d][1] = x.y; v[d][2] = x.z; v[d][3] = x.w;
+            } else if constexpr (U == 2) {
+                const float2 x = __ldg(reinterpret_cast<const float2*>(rec) + d);
+                v[d][0] = x.x; v[d][1] = x.y;
+            } else {
+                v[d][0] = __ldg(rec + d);
+            }
+        }
+    }
+};
+
 // Does item t of `h` meet [lo, hi]?  A soup of boxes (degenerate triangles
 // lo, hi, hi) by the box, a soup of triangles by the triangle's box.
 __device__ __forceinline__ bool item_meets_box(const DevDataset& h, int64_t t, const float3& lo, const float3& hi) {
@@ -63,6 +83,26 @@ __device__ __forceinline__ bool item_meets_box(const DevDataset& h, int64_t t, c
 // Does leaf [first, first + count) of `h` meet [lo, hi]?
 __device__ __forceinline__ bool leaf_meets_box(const DevDataset& h, int first, int count, const float3& lo,
                                                const float3& hi) {
+    if (h.tri_boxes) {
+        const int U = h.tri_box_unit;
+        bool hit = false;
+        if (U == 4) {
+            for (int t = first; t < first + count; t += 4) {
+                const TriBoxes<4> b(h.tri_boxes + 6 * (int64_t)t);
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    hit |= box_overlap(b.v[0][k], b.v[3][k], b.v[1][k], b.v[4][k], b.v[2][k], b.v[5][k], lo, hi);
+                if (hit) return true;
+            }
+            return false;
+        }
+        for (int t = first; t < first + count; ++t) {
+            const float* r = h.tri_boxes + 6 * (int64_t)(t & ~(U - 1)) + (t & (U - 1));
+            hit |= box_overlap(__ldg(r), __ldg(r + 3 * U), __ldg(r + U), __ldg(r + 4 * U), __ldg(r + 2 * U),
+                               __ldg(r + 5 * U), lo, hi);
+        }
+        return hit;
+    }
     for (int k = 0; k < count; ++k)
         if (item_meets_box(h, (int64_t)first + k, lo, hi)) return true;
     return false;
