@@ -375,8 +375,7 @@ int build_lbvh(pierce_ctx* ctx, const float* verts, const uint32_t* idx, const i
 // Node4 copy of a binary hierarchy with num_nodes internal nodes (G soup
 // triangles per leaf item)
 int collapse4(pierce_ctx* ctx, const Node* nodes, int64_t num_nodes, Node4* out, int G = 1);
-int prepare_objects(pierce_ctx* ctx, pierce_dataset* ds, cudaEvent_t edges_ready = nullptr,
-                    const int32_t* grouped_flag = nullptr);
+int prepare_objects(pierce_ctx* ctx, pierce_dataset* ds, bool edges_later = false);
 // Groups of G consecutive triangles (G divides 32; each in one of the
 // dataset's 32-triangle chunks) that can meet the other side: list[k] =
 // chunk * (32 / G) + group in order, *d_count their number.  mem:
