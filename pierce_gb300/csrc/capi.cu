@@ -1731,7 +1731,7 @@ struct Join {
         group_filter[sd] = other.nodes4 != nullptr;
         if (int s = cull_groups(ctx, ds->view(), ds->d_tri_to_object, active_flags, other, group_filter[sd], G, mem,
                                 group_list[sd], words + 11 + sd, reinterpret_cast<int32_t*>(words + 13),
-                                reinterpret_cast<uint32_t*>(words + 20 + 8 * sd), words + 16 + 8 * sd))
+                                reinterpret_cast<uint32_t*>(words + 20 + 8 * sd)))
             return s;
         group_count[sd] = -1;
         // A's hierarchy is sized by its count; B's groups are sized by it
@@ -1778,7 +1778,7 @@ struct Join {
         int2* roots = parts ? reinterpret_cast<int2*>((Node*)np + m) : nullptr;
         BvhShape sh;
         if (int s = build_group_lbvh(ctx, ds->view(), ds->d_tri_to_object, group_list[sd], words + 11 + sd, n, G,
-                                     reinterpret_cast<uint32_t*>(words + 20 + 8 * sd), words + 16 + 8 * sd, gp,
+                                     reinterpret_cast<uint32_t*>(words + 20 + 8 * sd), gp,
                                      (float4*)sp, tb, (Node*)np, &sh, parts, roots))
             return s;
         DevDataset& v = sd ? vb : va;

@@ -381,11 +381,11 @@ int prepare_objects(pierce_ctx* ctx, pierce_dataset* ds, bool edges_later = fals
 // chunk * (32 / G) + group in order, *d_count their number.  mem:
 // group_cull_bytes; with `filter` groups are tested too (other.nodes4);
 // *d_mixed |= a group of a kept chunk spans two partitions.  bounds (6
-// words) and zero (4 words) are prepared for build_group_lbvh.
+// words) are prepared for build_group_lbvh.
 size_t group_cull_bytes(int64_t nt, int G);
 int cull_groups(pierce_ctx* ctx, const DevDataset& src, const int32_t* t2o, const uint8_t* active,
                 const DevDataset& other, bool filter, int G, void* mem, uint32_t* list, unsigned long long* d_count,
-                int32_t* d_mixed, uint32_t* bounds, unsigned long long* zero);
+                int32_t* d_mixed, uint32_t* bounds);
 // the listed groups (at most `bound`) as boxes and a soup in list order, with
 // their triangles' boxes (DevDataset::tri_boxes) where tri_boxes is given
 int group_units(pierce_ctx* ctx, const DevDataset& src, const int32_t* t2o, const uint32_t* list,
@@ -396,7 +396,7 @@ int group_units(pierce_ctx* ctx, const DevDataset& src, const int32_t* t2o, cons
 // (collapse4 with G does so for the four-wide copy).
 int build_group_lbvh(pierce_ctx* ctx, const DevDataset& src, const int32_t* t2o, const uint32_t* list,
                      const unsigned long long* d_count, int64_t n, int G, uint32_t* bounds,
-                     unsigned long long* wave_count, void* group_scratch, float4* soup, float* tri_boxes, Node* nodes,
+                     void* group_scratch, float4* soup, float* tri_boxes, Node* nodes,
                      BvhShape* shape, int32_t num_parts, int2* part_roots);
 int group_leaves(pierce_ctx* ctx, Node* nodes, int64_t num_nodes, int G);
 
