@@ -1731,7 +1731,7 @@ struct Join {
         group_filter[sd] = other.nodes4 != nullptr;
         if (int s = cull_groups(ctx, ds->view(), ds->d_tri_to_object, active_flags, other, group_filter[sd], G, mem,
                                 group_list[sd], words + 11 + sd, reinterpret_cast<int32_t*>(words + 13),
-                                reinterpret_cast<uint32_t*>(words + 20 + 8 * sd)))
+                                reinterpret_cast<uint32_t*>(words + 20 + 8 * sd), ctx->d_counters->active_tris + sd))
             return s;
         group_count[sd] = -1;
         // A's hierarchy is sized by its count; B's groups are sized by it

@@ -38,6 +38,7 @@ struct DevCounters {
     unsigned long long hash_accesses;
     unsigned long long hash_contentions;
     unsigned long long kept_b;  // joins by triangle pairs: B's kept groups
+    unsigned long long active_tris[2];  // triangles of active objects, A and B (culling)
 };
 
 // Binary BVH node holding the boxes of its two children (64 bytes, four
@@ -381,11 +382,13 @@ int prepare_objects(pierce_ctx* ctx, pierce_dataset* ds, bool edges_later = fals
 // chunk * (32 / G) + group in order, *d_count their number.  mem:
 // group_cull_bytes; with `filter` groups are tested too (other.nodes4);
 // *d_mixed |= a group of a kept chunk spans two partitions.  bounds (6
-// words) are prepared for build_group_lbvh.
+// words) are prepared for build_group_lbvh.  active_tris (device): triangles
+// of src's active objects.
 size_t group_cull_bytes(int64_t nt, int G);
 int cull_groups(pierce_ctx* ctx, const DevDataset& src, const int32_t* t2o, const uint8_t* active,
                 const DevDataset& other, bool filter, int G, void* mem, uint32_t* list, unsigned long long* d_count,
-                int32_t* d_mixed, uint32_t* bounds);
+                int32_t* d_mixed, uint32_t* bounds,
+                const unsigned long long* active_tris);
 // the listed groups (at most `bound`) as boxes and a soup in list order, with
 // their triangles' boxes (DevDataset::tri_boxes) where tri_boxes is given
 int group_units(pierce_ctx* ctx, const DevDataset& src, const int32_t* t2o, const uint32_t* list,

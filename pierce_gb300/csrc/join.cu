@@ -551,7 +551,8 @@ struct ActiveSide {
     DevDataset src, tgt;
     uint8_t* active;
 };
-__global__ void __launch_bounds__(128) k_object_active(ActiveSide side0, ActiveSide side1, unsigned blocks0) {
+__global__ void __launch_bounds__(128) k_object_active(ActiveSide side0, ActiveSide side1, unsigned blocks0,
+                                                       unsigned long long* active_tris) {
     __shared__ int sstack[kShortStack][128];
     int lstack[kStackSize - kShortStack];
     const int tid = threadIdx.x;
@@ -560,11 +561,11 @@ __global__ void __launch_bounds__(128) k_object_active(ActiveSide side0, ActiveS
     const DevDataset& tgt = second ? side1.tgt : side0.tgt;
     uint8_t* active = second ? side1.active : side0.active;
     const int64_t o = (blockIdx.x - (second ? blocks0 : 0u)) * (int64_t)blockDim.x + tid;
-    if (o >= src.num_objects) return;
-    const float* b = src.obj_box + 6 * o;
+    const bool in = o < src.num_objects;
+    const float* b = src.obj_box + 6 * (in ? o : 0);
     const float3 lo = make_float3(b[0], b[1], b[2]), hi = make_float3(b[3], b[4], b[5]);
     bool found = false;
-    if (lo.x <= hi.x && tgt.num_tris > 0) {
+    if (in && lo.x <= hi.x && tgt.num_tris > 0) {
         auto leaf = [&](int first, int count) {
             for (int k = 0; k < count && !found; ++k) {
                 const int64_t t = (int64_t)first + k;
@@ -622,7 +623,11 @@ __global__ void __launch_bounds__(128) k_object_active(ActiveSide side0, ActiveS
             }
         }
     }
-    active[o] = found ? 1 : 0;
+    if (in) active[o] = found ? 1 : 0;
+    if (src.obj_range) {
+        const unsigned c = __reduce_add_sync(0xFFFFFFFFu, found ? (unsigned)__ldg(&src.obj_range[o].y) : 0u);
+        if ((tid & 31) == 0 && c) atomicAdd(active_tris + (second ? 1 : 0), (unsigned long long)c);
+    }
 }
 
 // Block-aggregated stream compaction: each thread takes ITEMS consecutive
@@ -973,7 +978,8 @@ int launch_object_active(pierce_ctx* ctx, const DevDataset& a, const DevDataset&
     const unsigned n0 = (unsigned)((std::max(a.num_objects, 0) + 127) / 128);
     const unsigned n1 = (unsigned)((std::max(b.num_objects, 0) + 127) / 128);
     if (n0 + n1 == 0) return PIERCE_OK;
-    k_object_active<<<n0 + n1, 128, 0, ctx->stream>>>(ActiveSide{a, tgt_a, active_a}, ActiveSide{b, tgt_b, active_b}, n0);
+    k_object_active<<<n0 + n1, 128, 0, ctx->stream>>>(ActiveSide{a, tgt_a, active_a}, ActiveSide{b, tgt_b, active_b}, n0,
+                                                      ctx->d_counters->active_tris);
     ctx->launches += 1;
     return check_cuda(cudaGetLastError(), "object activity");
 }

@@ -101,14 +101,16 @@ __device__ __forceinline__ uint32_t expand_bits10(uint32_t v) {
 
 // 2. Morton codes
 // (inverted: all ones when the bounds' maxima are stored inverted, else 0)
-__global__ void k_morton(const float4* __restrict__ cen, int64_t nt, const uint32_t* __restrict__ bounds,
-                         uint32_t* __restrict__ keys, uint32_t* __restrict__ vals, uint32_t inverted) {
-    const float lo[3] = {o2f(bounds[0]), o2f(bounds[1]), o2f(bounds[2])};
-    const float hi[3] = {o2f(bounds[3] ^ inverted), o2f(bounds[4] ^ inverted), o2f(bounds[5] ^ inverted)};
-    float inv[3];
-    for (int k = 0; k < 3; ++k) inv[k] = hi[k] > lo[k] ? 1.0f / (hi[k] - lo[k]) : 0.0f;
-    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < nt; t += (int64_t)gridDim.x * blockDim.x) {
-        const float4 c = cen[t];
+struct CodeFrame {
+    float lo[3], inv[3];
+    __device__ __forceinline__ CodeFrame(const uint32_t* bounds, uint32_t inverted) {
+        for (int k = 0; k < 3; ++k) {
+            lo[k] = o2f(bounds[k]);
+            const float hi = o2f(bounds[3 + k] ^ inverted);
+            inv[k] = hi > lo[k] ? 1.0f / (hi - lo[k]) : 0.0f;
+        }
+    }
+    __device__ __forceinline__ uint32_t code(const float4& c) const {
         const float cc[3] = {c.x, c.y, c.z};
         uint32_t q[3];
         for (int k = 0; k < 3; ++k) {
@@ -116,9 +118,111 @@ __global__ void k_morton(const float4* __restrict__ cen, int64_t nt, const uint3
             u = fminf(fmaxf(u, 0.0f), 1.0f);
             q[k] = min((uint32_t)(u * 1024.0f), 1023u);
         }
-        keys[t] = (expand_bits10(q[0]) << 2) | (expand_bits10(q[1]) << 1) | expand_bits10(q[2]);
+        return (expand_bits10(q[0]) << 2) | (expand_bits10(q[1]) << 1) | expand_bits10(q[2]);
+    }
+};
+
+__global__ void k_morton(const float4* __restrict__ cen, int64_t nt, const uint32_t* __restrict__ bounds,
+                         uint32_t* __restrict__ keys, uint32_t* __restrict__ vals, uint32_t inverted) {
+    const CodeFrame f(bounds, inverted);
+    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < nt; t += (int64_t)gridDim.x * blockDim.x) {
+        keys[t] = f.code(cen[t]);
         vals[t] = (uint32_t)t;
     }
+}
+
+// 3'. few primitives: codes sorted a tile of 1,024 per block (bitonic, by code
+// and position, so equal codes keep their order), then every code placed at
+// its rank: its place in its own tile and a binary search in each other tile,
+// four lanes sharing a code's tiles.  A radix sort of so few codes is four
+// passes that a handful of blocks each run, eleven launches and fills with the
+// codes: 7,700 codes 41 us of kernels and 86 from first to last, so 15 and 17.
+// The searches grow with the square of n: 92,000 codes 96 us here, 42 (75
+// from first to last) by radix sort, so kSmallSort lies below that.
+constexpr int kSortTile = 1024;
+constexpr int64_t kSmallSort = 1 << 16;
+__global__ void __launch_bounds__(kSortTile) k_code_tiles(const float4* __restrict__ cen, int n,
+                                                          const uint32_t* __restrict__ bounds, uint32_t inverted,
+                                                          uint32_t* __restrict__ keys, uint32_t* __restrict__ vals) {
+    __shared__ unsigned long long s_v[kSortTile];
+    const int tid = threadIdx.x, i = blockIdx.x * kSortTile + tid;
+    unsigned long long v = ~0ull;
+    if (i < n) v = ((unsigned long long)CodeFrame(bounds, inverted).code(cen[i]) << 32) | (uint32_t)i;
+#pragma unroll 1
+    for (int k = 2; k <= kSortTile; k <<= 1)
+#pragma unroll 1
+        for (int j = k >> 1; j > 0; j >>= 1) {
+            unsigned long long o;
+            if (j >= 32) {
+                __syncthreads();
+                s_v[tid] = v;
+                __syncthreads();
+                o = s_v[tid ^ j];
+            } else {
+                o = __shfl_xor_sync(0xFFFFFFFFu, v, j);
+            }
+            const bool low = ((tid & j) == 0) == ((tid & k) == 0);
+            v = low == (o < v) ? o : v;
+        }
+    if (i < n) {
+        keys[i] = (uint32_t)(v >> 32);
+        vals[i] = (uint32_t)v;
+    }
+}
+
+__global__ void __launch_bounds__(256) k_merge_tiles(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ vals,
+                                                     int n, uint32_t* __restrict__ keys_out,
+                                                     uint32_t* __restrict__ vals_out) {
+    constexpr int kAt = 4;  // searches in flight
+    const int e = (blockIdx.x * 256 + threadIdx.x) >> 2, sub = threadIdx.x & 3;
+    const int tiles = (n + kSortTile - 1) / kSortTile;
+    const uint32_t key = e < n ? __ldg(keys + e) : 0u;
+    const int mine = e / kSortTile;
+    int rank = sub == 0 ? e - mine * kSortTile : 0;
+    for (int t0 = sub; t0 < tiles && e < n; t0 += 4 * kAt) {
+        int pos[kAt];
+#pragma unroll
+        for (int a = 0; a < kAt; ++a) pos[a] = 0;
+#pragma unroll
+        for (int step = kSortTile; step > 0; step >>= 1)
+#pragma unroll
+            for (int a = 0; a < kAt; ++a) {
+                const int t = t0 + 4 * a;
+                const int p = pos[a] + step;
+                if (t == mine || p > min(kSortTile, n - t * kSortTile)) continue;
+                const uint32_t other = __ldg(keys + t * kSortTile + p - 1);
+                // equal codes: those of earlier tiles come first
+                if (other < key || (other == key && t < mine)) pos[a] = p;
+            }
+#pragma unroll
+        for (int a = 0; a < kAt; ++a) rank += pos[a];
+    }
+    rank += __shfl_xor_sync(0xFFFFFFFFu, rank, 1);
+    rank += __shfl_xor_sync(0xFFFFFFFFu, rank, 2);
+    if (sub == 0 && e < n) {
+        keys_out[rank] = key;
+        vals_out[rank] = __ldg(vals + e);
+    }
+}
+
+// Morton codes of n centres and their order: keys + n, vals + n.
+static int sorted_codes(pierce_ctx* ctx, const float4* cen, int64_t n, const uint32_t* bounds, uint32_t inverted,
+                        uint32_t* keys, uint32_t* vals) {
+    cudaStream_t st = ctx->stream;
+    if (n <= kSmallSort) {
+        const bool one = n <= kSortTile;
+        k_code_tiles<<<(unsigned)((n + kSortTile - 1) / kSortTile), kSortTile, 0, st>>>(
+            cen, (int)n, bounds, inverted, one ? keys + n : keys, one ? vals + n : vals);
+        ctx->launches += 1;
+        if (one) return check_cuda(cudaGetLastError(), "sort codes");
+        k_merge_tiles<<<(unsigned)((4 * n + 255) / 256), 256, 0, st>>>(keys, vals, (int)n, keys + n, vals + n);
+        ctx->launches += 1;
+        return check_cuda(cudaGetLastError(), "sort codes");
+    }
+    k_morton<<<(unsigned)std::min<int64_t>((n + 255) / 256, (int64_t)ctx->sm_count * 16), 256, 0, st>>>(
+        cen, n, bounds, keys, vals, inverted);
+    ctx->launches += 1;
+    return sort_u32_pairs(ctx, keys, keys + n, vals, vals + n, n, 30);
 }
 
 // 1'/2'. partitioned hierarchy: centroid bounds per partition (warps whose
@@ -882,9 +986,8 @@ int build_lbvh(pierce_ctx* ctx, const float* verts, const uint32_t* idx, const i
         k_fill_u32<<<1, 32, 0, st>>>(bounds, 0xFFFFFFFFu, 3);  // ordered +max
         k_fill_u32<<<1, 32, 0, st>>>(bounds + 3, 0u, 3);       // ordered -max
         k_centroids<<<std::min(grid_for(ctx, n, B), ctx->sm_count * 4), B, 0, st>>>(verts, idx, list, n, cen, bounds);
-        k_morton<<<grid_for(ctx, n, B), B, 0, st>>>(cen, n, bounds, keys, vals, 0u);
-        ctx->launches += 4;
-        if (int s = sort_u32_pairs(ctx, keys, keys + n, vals, vals + n, n, 30)) return s;
+        ctx->launches += 3;
+        if (int s = sorted_codes(ctx, cen, n, bounds, 0u, keys, vals)) return s;
     }
     const uint32_t* skeys = keys + n;
     const uint64_t* skeys64 = keys64 + n;
@@ -963,6 +1066,14 @@ struct GroupMask<2> { using type = uint16_t; };
 template <>
 struct GroupMask<1> { using type = uint32_t; };
 
+// Where the active objects have few triangles k_cull_chunks lists all of
+// their chunks: the groups' walks fill the chip once anyway, and the chunks'
+// walks before them only add their length (60 x 60 spheres 57 -> 31 us for
+// both sides, 2000 x 2000 66 -> 42, 6,000 x 5,003 ellipsoids with some 0.8 M
+// triangles a side 77 -> 65); with more the chunks' walks save most of the
+// groups' (7,013 x 4,999 spheres 129 us, 147 without, tubes 150 and 455, 2 x
+// 50,000 ellipsoids 340 and 703).  The line lies at 2^20 triangles.
+constexpr int64_t kGroupsOnly = 1 << 20;
 struct CullParams {
     const float* verts;
     const uint32_t* idx;
@@ -973,6 +1084,7 @@ struct CullParams {
     const uint8_t* active;       // per object
     const int32_t* obj_part;     // partitioned datasets
     DevDataset other;            // the other side's object boxes or kept triangles
+    const unsigned long long* active_tris;  // triangles of active objects (null: unknown)
     int filter;                  // groups too are tested (the hierarchy has four-wide nodes)
     int wide;                    // node ids fit the shared walk's stack
     int mask_bytes;
@@ -1006,6 +1118,7 @@ __global__ void __launch_bounds__(128) k_cull_chunks(CullParams P) {
     const int64_t n_chunks = (P.nt + 31) / 32, n_words = (n_chunks + 31) / 32;
     const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
     if (blockIdx.x == 0 && threadIdx.x < 6) P.bounds[threadIdx.x] = 0xFFFFFFFFu;
+    const bool walk = !P.active_tris || *P.active_tris > (unsigned long long)kGroupsOnly;
     for (int64_t w = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); w < n_words; w += warps) {
         const int64_t c = w * 32 + lane;
         const bool in = c < n_chunks;
@@ -1062,7 +1175,7 @@ __global__ void __launch_bounds__(128) k_cull_chunks(CullParams P) {
                 live = !act;
             }
         }
-        act = cull_query(P, W, live, part, lo, hi) || act;
+        act = (walk ? cull_query(P, W, live, part, lo, hi) : live) || act;
         const unsigned m = __ballot_sync(0xFFFFFFFFu, act);
         if (!m) continue;
         unsigned long long at = 0;
@@ -1484,7 +1597,8 @@ size_t group_cull_bytes(int64_t nt, int G) {
 
 int cull_groups(pierce_ctx* ctx, const DevDataset& src, const int32_t* t2o, const uint8_t* active,
                 const DevDataset& other, bool filter, int G, void* mem, uint32_t* list, unsigned long long* d_count,
-                int32_t* d_mixed, uint32_t* bounds) {
+                int32_t* d_mixed, uint32_t* bounds,
+                const unsigned long long* active_tris) {
     cudaStream_t st = ctx->stream;
     const int64_t nt = src.num_tris, chunks = (nt + 31) / 32, tiles = (chunks + kListTile - 1) / kListTile;
     if (nt <= 0) return check_cuda(cudaMemsetAsync(d_count, 0, 8, st), "cull groups");
@@ -1508,6 +1622,7 @@ int cull_groups(pierce_ctx* ctx, const DevDataset& src, const int32_t* t2o, cons
     P.obj_part = src.obj_part;
     P.other = other;
     P.filter = filter ? 1 : 0;
+    P.active_tris = filter && src.obj_range ? active_tris : nullptr;
     P.wide = other.nodes4 && other.num_tris < (int64_t(1) << 27) ? 1 : 0;
     P.mask_bytes = (int)mask_bytes(G);
     P.masks = mem;
@@ -1591,13 +1706,12 @@ int build_group_lbvh(pierce_ctx* ctx, const DevDataset& src, const int32_t* t2o,
         while (bits < 32 && (1ll << bits) < (int64_t)num_parts) ++bits;
         if (int s = sort_u64_pairs(ctx, keys64, keys64 + n, vals, vals + n, n, 30 + bits)) return s;
     } else {
-        k_morton<<<grid_for(ctx, n, B), B, 0, st>>>(cen, n, bounds, keys, vals, 0xFFFFFFFFu);
-        if (int s = sort_u32_pairs(ctx, keys, keys + n, vals, vals + n, n, 30)) return s;
+        if (int s = sorted_codes(ctx, cen, n, bounds, 0xFFFFFFFFu, keys, vals)) return s;
     }
     const uint32_t* order = vals + n;
     k_group_soup<<<grid_for(ctx, n * G, B), B, 0, st>>>(list, order, d_count, G, src.verts, src.idx, t2o, src.num_tris,
                                                         soup, tri_boxes);
-    ctx->launches += 3;
+    ctx->launches += parts ? 3 : 2;
     if (n == 1) {
         if (parts) {
             k_single_part_root<<<1, 1, 0, st>>>(keys64 + n, part_roots);

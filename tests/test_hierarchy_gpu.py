@@ -25,7 +25,8 @@ def triangles(n, kind, seed, per_object=4, size=0.2):
 
 
 @pytest.mark.parametrize("kind", ["spread", "one place", "sheet"])
-@pytest.mark.parametrize("n,leaf", [(2, 1), (511, 1), (512, 4), (513, 1), (514, 8), (1025, 3), (5000, 16), (40000, 1)])
+@pytest.mark.parametrize("n,leaf", [(2, 1), (511, 1), (512, 4), (513, 1), (514, 8), (1024, 1), (1025, 3), (5000, 16),
+                                    (65536, 1), (65537, 1)])
 def test_own_hierarchies_find_the_oracles_pairs(ctx, n, leaf, kind):
     A, B = triangles(n, kind, 1, size=0.3), triangles(60, "spread", 2, size=6.0)
     t = J.default_tuning(leaf_size=leaf)
