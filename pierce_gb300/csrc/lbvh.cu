@@ -322,19 +322,6 @@ __global__ void k_soup(const float* __restrict__ verts, const uint32_t* __restri
 }
 
 // longest common prefix of sorted keys i and j (index tie-break), -1 outside
-__device__ __forceinline__ int lcp(const uint32_t* keys, int64_t n, int64_t i, int64_t j) {
-    if (j < 0 || j >= n) return -1;
-    const uint32_t ki = keys[i], kj = keys[j];
-    if (ki == kj) return 32 + __clzll((unsigned long long)(i ^ j)) - 32;  // 32 + clz over 32-bit index
-    return __clz(ki ^ kj);
-}
-__device__ __forceinline__ int lcp(const uint64_t* keys, int64_t n, int64_t i, int64_t j) {
-    if (j < 0 || j >= n) return -1;
-    const uint64_t ki = keys[i], kj = keys[j];
-    if (ki == kj) return 64 + __clzll((unsigned long long)(i ^ j));
-    return __clzll(ki ^ kj);
-}
-
 // partition of sorted key k (32-bit keys carry none)
 __device__ __forceinline__ uint32_t key_part(const uint32_t*, int64_t) { return 0u; }
 __device__ __forceinline__ uint32_t key_part(const uint64_t* keys, int64_t k) { return (uint32_t)(keys[k] >> 30); }
@@ -358,7 +345,8 @@ __device__ __forceinline__ uint32_t key_part(const uint64_t* keys, int64_t k) { 
 // This takes the place of linking everything through memory and refitting
 // upwards in list waves and chains, an atomic with fences and two more trips to
 // L2 per level of the tree: hierarchies of 463 groups 31 -> 17 us, 7,700 39 ->
-// 28, 6.8 M 1,022 -> 630; those of 169,000 and 73,000 together 119 -> 75.
+// 25, 6.8 M 1,022 -> 555 (630 with the search in 64-bit indices); those of
+// 169,000 and 73,000 together 119 -> 68.
 //
 // Partitioned keys: a range is collapsed into a leaf only when it lies in
 // one partition, and every range that is exactly one whole partition
@@ -367,16 +355,15 @@ __device__ __forceinline__ uint32_t key_part(const uint64_t* keys, int64_t k) { 
 // subtree of the radix tree.
 constexpr int kLocal = 512;
 
-// Box of a leaf at sorted position j: one prepared box each, or the boxes of
-// the soup's triangles.
+// Box of a leaf at sorted position j: a prepared box, or that of the soup's
+// triangles.
 struct LeafBoxes {
     const float* gbox;
-    const uint32_t* order;
     const float4* soup;
 };
 __device__ __forceinline__ void leaf_box(const LeafBoxes& L, int64_t j, int count, float lo[3], float hi[3]) {
     if (L.gbox) {
-        const float* b = L.gbox + 6 * (int64_t)__ldg(L.order + j);
+        const float* b = L.gbox + 6 * j;
         for (int k = 0; k < 3; ++k) {
             lo[k] = __ldg(b + k);
             hi[k] = __ldg(b + 3 + k);
@@ -438,46 +425,57 @@ __global__ void __launch_bounds__(kLocal / 2) k_build_local(const K* __restrict_
 #pragma unroll
     for (int q = 0; q < 2; ++q) {
         const int k = q * (kLocal / 2) + tid;
-        const int64_t i = b0 + k;
-        if (i >= n - 1) continue;
-        const int d = (lcp(keys, n, i, i + 1) - lcp(keys, n, i, i - 1)) >= 0 ? 1 : -1;
-        const int dmin = lcp(keys, n, i, i - d);
-        int64_t lmax = 2;
-        while (lcp(keys, n, i, i + lmax * d) > dmin) lmax <<= 1;
-        int64_t l = 0;
-        for (int64_t t = lmax >> 1; t >= 1; t >>= 1)
-            if (lcp(keys, n, i, i + (l + t) * d) > dmin) l += t;
-        const int64_t j = i + l * d;
-        const int64_t first = i < j ? i : j, last = i < j ? j : i;
+        if (b0 + k >= n - 1) continue;
+        const int i = (int)(b0 + k), count_n = (int)n;
+        const K own = __ldg(keys + i);
+        // common leading bits of the keys at i and j, equal keys told apart by
+        // position; -1 outside [0, n)
+        auto common = [&](int j) {
+            if ((unsigned)j >= (unsigned)count_n) return -1;
+            const K other = __ldg(keys + j);
+            if (other == own) return 8 * (int)sizeof(K) + __clz(i ^ j);
+            return sizeof(K) == 8 ? __clzll((long long)(other ^ own)) : __clz((int)(other ^ own));
+        };
+        const int next = common(i + 1), before = common(i - 1);
+        const int d = next >= before ? 1 : -1;
+        const int dmin = min(next, before);
+        int lmax = 2;
+        while (common(i + lmax * d) > dmin) lmax <<= 1;
+        int l = 0;
+        for (int t = lmax >> 1; t >= 1; t >>= 1)
+            if (common(i + (l + t) * d) > dmin) l += t;
+        const int j = i + l * d;
+        const int first = min(i, j), last = max(i, j);
         if (i != 0 && last - first + 1 <= leaf_size && key_part(keys, first) == key_part(keys, last))
             continue;  // inside a collapsed leaf
-        if (part_roots && whole_part(first, last)) part_roots[key_part(keys, first)] = make_int2((int)i, 0);
-        const int dnode = lcp(keys, n, i, j);
-        int64_t s = 0, t = l;
+        if (part_roots && whole_part(first, last)) part_roots[key_part(keys, first)] = make_int2(i, 0);
+        const int dnode = common(j);
+        int s = 0, t = l;
         do {
             t = (t + 1) >> 1;
-            if (lcp(keys, n, i, i + (s + t) * d) > dnode) s += t;
+            if (common(i + (s + t) * d) > dnode) s += t;
         } while (t > 1);
-        const int64_t gamma = i + s * d + (d < 0 ? -1 : 0);
+        const int gamma = i + s * d + (d < 0 ? -1 : 0);
         local[q] = first >= b0 && last < b1;
         int child[2];
         int count[2] = {0, 0};
-        const int64_t cfirst[2] = {first, gamma + 1}, clast[2] = {gamma, last};
-        const int64_t cidx[2] = {gamma, gamma + 1};
+        const int cfirst[2] = {first, gamma + 1}, clast[2] = {gamma, last};
+        const int cidx[2] = {gamma, gamma + 1};
+#pragma unroll
         for (int side = 0; side < 2; ++side) {
-            const int64_t size = clast[side] - cfirst[side] + 1;
+            const int size = clast[side] - cfirst[side] + 1;
             if (size <= leaf_size && key_part(keys, cfirst[side]) == key_part(keys, clast[side])) {
-                child[side] = ~(int)cfirst[side];
-                count[side] = (int)size;
+                child[side] = ~cfirst[side];
+                count[side] = size;
                 if (local[q]) {
                     const int f = (int)(cfirst[side] - b0);
-                    s_leaf[f] = (((k << 1) | side) << 5) | (int)size;
-                    for (int m = 1; m < (int)size; ++m) s_leaf[f + m] = kInside;
+                    s_leaf[f] = (((k << 1) | side) << 5) | size;
+                    for (int m = 1; m < size; ++m) s_leaf[f + m] = kInside;
                 }
                 if (part_roots && whole_part(cfirst[side], clast[side]))
-                    part_roots[key_part(keys, cfirst[side])] = make_int2(~(int)cfirst[side], (int)size);
+                    part_roots[key_part(keys, cfirst[side])] = make_int2(~cfirst[side], size);
             } else {
-                child[side] = (int)cidx[side];
+                child[side] = cidx[side];
                 if (local[q]) s_par[cidx[side] - b0] = (k << 1) | side;
             }
         }
@@ -486,7 +484,7 @@ __global__ void __launch_bounds__(kLocal / 2) k_build_local(const K* __restrict_
             nodes[i].ch = ch[q];
             const int at = atomicAdd(&s_nodes, 1);
             if (at < kTileItems)
-                T.nodes[(int64_t)blockIdx.x * kTileItems + at] = make_int4((int)i, (int)first, (int)last, (int)gamma);
+                T.nodes[(int64_t)blockIdx.x * kTileItems + at] = make_int4(i, first, last, gamma);
         }
     }
     __syncthreads();
@@ -1007,7 +1005,7 @@ int build_lbvh(pierce_ctx* ctx, const float* verts, const uint32_t* idx, const i
         shape->root_leaf_count = (int)n;
         shape->num_nodes = 0;
     } else {
-        const LeafBoxes L{nullptr, nullptr, soup};
+        const LeafBoxes L{nullptr, soup};
         if (parts) build_nodes(ctx, skeys64, n, leaf_size, nodes, part_roots, L, pm, d_root_box);
         else build_nodes(ctx, skeys, n, leaf_size, nodes, nullptr, L, pm, d_root_box);
         shape->num_nodes = (uint64_t)(n - 1);
@@ -1342,25 +1340,48 @@ __global__ void __launch_bounds__(256) k_list_groups(const void* __restrict__ ma
         for (uint32_t b = mask[k]; b; b &= b - 1) list[pos++] = (uint32_t)((c0 + k) * PER + __ffs(b) - 1);
 }
 
-// Kept groups -> boxes, box centres (w: partition) and the centres' bounds
+// Kept groups -> box centres (w: partition) and the centres' bounds
 // (ordered integers; the maxima stored inverted, so that all six start as all
-// ones).  One thread per group.
+// ones).  One thread per group.  Partitioned: a warp takes a contiguous range
+// and keeps the bounds of the partition it is in, which goes to memory when
+// the partition changes (a set of atomics per 32 groups on the few words of 64
+// joins' bounds: 411 us for 6.3 M groups, so 185).
 template <int G, bool PARTS>
 __global__ void __launch_bounds__(256) k_group_prims(const float* __restrict__ verts, const uint32_t* __restrict__ idx,
                                                      const int32_t* __restrict__ t2o, int64_t nt,
                                                      const uint32_t* __restrict__ list,
                                                      const unsigned long long* __restrict__ count,
-                                                     const int32_t* __restrict__ obj_part, float* __restrict__ gbox,
+                                                     const int32_t* __restrict__ obj_part,
                                                      float4* __restrict__ cen, uint32_t* __restrict__ bounds) {
     constexpr int PER = 32 / G;
     const int64_t n = (int64_t)*count;
     float mn[3] = {3.4e38f, 3.4e38f, 3.4e38f}, mx[3] = {-3.4e38f, -3.4e38f, -3.4e38f};
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t base = blockIdx.x * (int64_t)blockDim.x; base < n; base += stride) {
-        const int64_t j = base + threadIdx.x;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    int64_t j0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x - lane, j1 = n, stride = (int64_t)gridDim.x * blockDim.x;
+    if (PARTS) {
+        const int64_t runs = (n + 31) / 32, warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+        const int64_t w = (int64_t)blockIdx.x * (blockDim.x >> 5) + wid;
+        j0 = 32 * (runs * w / warps);
+        j1 = min(n, 32 * (runs * (w + 1) / warps));
+        stride = 32;
+    }
+    int32_t cur = -1;  // the partition mn, mx belong to
+    auto flush = [&]() {
+        for (int d = 0; cur >= 0 && d < 3; ++d) {
+            const float a = warp_min(mn[d]), b = warp_max(mx[d]);
+            if (lane == 0 && a <= b) {
+                atomicMin(bounds + 6 * (int64_t)cur + d, f2o(a));
+                atomicMin(bounds + 6 * (int64_t)cur + 3 + d, ~f2o(b));
+            }
+            mn[d] = 3.4e38f;
+            mx[d] = -3.4e38f;
+        }
+    };
+    for (int64_t base = j0; base < j1; base += stride) {
+        const int64_t j = base + lane;
         int32_t part = -1;
         float m[3] = {0.0f, 0.0f, 0.0f};
-        if (j < n) {
+        if (j < j1) {
             const uint32_t g = __ldg(list + j);
             float lo[3] = {3.4e38f, 3.4e38f, 3.4e38f}, hi[3] = {-3.4e38f, -3.4e38f, -3.4e38f};
 #pragma unroll
@@ -1373,50 +1394,39 @@ __global__ void __launch_bounds__(256) k_group_prims(const float* __restrict__ v
                     hi[0] = fmaxf(hi[0], p.x); hi[1] = fmaxf(hi[1], p.y); hi[2] = fmaxf(hi[2], p.z);
                 }
             }
-            float* b = gbox + 6 * j;
-            b[0] = lo[0]; b[1] = lo[1]; b[2] = lo[2];
-            b[3] = hi[0]; b[4] = hi[1]; b[5] = hi[2];
-            if (cen) {
-                for (int d = 0; d < 3; ++d) m[d] = 0.5f * lo[d] + 0.5f * hi[d];
-                if (PARTS) part = __ldg(obj_part + __ldg(t2o + group_item(g / PER, (int)(g % PER), G, 0, nt)));
-                cen[j] = make_float4(m[0], m[1], m[2], __int_as_float(part));
-                for (int d = 0; d < 3; ++d) {
-                    mn[d] = fminf(mn[d], m[d]);
-                    mx[d] = fmaxf(mx[d], m[d]);
-                }
-            }
+            for (int d = 0; d < 3; ++d) m[d] = 0.5f * lo[d] + 0.5f * hi[d];
+            if (PARTS) part = __ldg(obj_part + __ldg(t2o + group_item(g / PER, (int)(g % PER), G, 0, nt)));
+            cen[j] = make_float4(m[0], m[1], m[2], __int_as_float(part));
         }
-        if (PARTS && cen) {
-            // per partition: lanes of one partition together
+        if (PARTS) {
             const int32_t p0 = __shfl_sync(0xFFFFFFFFu, part, 0);
-            if (p0 >= 0 && __all_sync(0xFFFFFFFFu, part == p0 || part < 0)) {
-                for (int d = 0; d < 3; ++d) {
-                    float a = part < 0 ? 3.4e38f : m[d], b = part < 0 ? -3.4e38f : m[d];
-                    for (int off = 16; off > 0; off >>= 1) {
-                        a = fminf(a, __shfl_xor_sync(0xFFFFFFFFu, a, off));
-                        b = fmaxf(b, __shfl_xor_sync(0xFFFFFFFFu, b, off));
-                    }
-                    if ((threadIdx.x & 31) == 0) {
-                        atomicMin(bounds + 6 * (int64_t)p0 + d, f2o(a));
-                        atomicMin(bounds + 6 * (int64_t)p0 + 3 + d, ~f2o(b));
-                    }
-                }
-            } else if (part >= 0) {
+            const bool one = p0 >= 0 && __all_sync(0xFFFFFFFFu, part == p0 || part < 0);
+            if (!one || p0 != cur) flush();
+            cur = one ? p0 : -1;
+            if (!one && part >= 0) {
                 for (int d = 0; d < 3; ++d) {
                     atomicMin(bounds + 6 * (int64_t)part + d, f2o(m[d]));
                     atomicMin(bounds + 6 * (int64_t)part + 3 + d, ~f2o(m[d]));
                 }
             }
+            if (!one || part < 0) continue;
+        } else if (j >= j1) {
+            continue;
+        }
+        for (int d = 0; d < 3; ++d) {
+            mn[d] = fminf(mn[d], m[d]);
+            mx[d] = fmaxf(mx[d], m[d]);
         }
     }
-    if (PARTS || !cen) return;
+    if (PARTS) {
+        flush();
+        return;
+    }
     __shared__ float red[2][3][8];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    for (int d = 0; d < 3; ++d)
-        for (int off = 16; off > 0; off >>= 1) {
-            mn[d] = fminf(mn[d], __shfl_xor_sync(0xFFFFFFFFu, mn[d], off));
-            mx[d] = fmaxf(mx[d], __shfl_xor_sync(0xFFFFFFFFu, mx[d], off));
-        }
+    for (int d = 0; d < 3; ++d) {
+        mn[d] = warp_min(mn[d]);
+        mx[d] = warp_max(mx[d]);
+    }
     if (lane == 0)
         for (int d = 0; d < 3; ++d) {
             red[0][d][wid] = mn[d];
@@ -1437,35 +1447,59 @@ __global__ void __launch_bounds__(256) k_group_prims(const float* __restrict__ v
 }
 
 // Triangle soup of kept groups, G triangles each: position j holds group
-// list[order[j]] (a hierarchy's leaf order), or list[j] without an order.
-// tri_boxes: the triangles' boxes by rows of min(G, 4), 24 bytes a triangle
-// beside its 48, for the walks that test a leaf's boxes.
+// list[order[j]] (a hierarchy's leaf order), or list[j] without an order; gbox:
+// the groups' boxes in the same order (read there in order by the build: a
+// gather through `order` instead cost that 25 us of 580 at 6.8 M groups, and a
+// launch of its own for the groups without a hierarchy 5 us a join).  tri_boxes: the triangles'
+// boxes by rows of min(G, 4), 24 bytes a triangle beside its 48, for the walks
+// that test a leaf's boxes.  Bound by memory (40 M triangles of the dense join
+// 0.8 ms, 4.9 TB/s).
+template <int G>
 __global__ void __launch_bounds__(256) k_group_soup(const uint32_t* __restrict__ list,
                                                     const uint32_t* __restrict__ order,
-                                                    const unsigned long long* __restrict__ count, int G,
+                                                    const unsigned long long* __restrict__ count,
                                                     const float* __restrict__ verts, const uint32_t* __restrict__ idx,
                                                     const int32_t* __restrict__ t2o, int64_t nt,
-                                                    float4* __restrict__ soup, float* __restrict__ tri_boxes) {
-    const int per_chunk = 32 / G, unit = min(G, 4);
+                                                    float4* __restrict__ soup, float* __restrict__ gbox,
+                                                    float* __restrict__ tri_boxes) {
+    constexpr int PER = 32 / G, UNIT = G < 4 ? G : 4;
     const int64_t n = (int64_t)*count * G;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t j = i / G;
-        const uint32_t g = __ldg(list + (order ? __ldg(order + j) : (uint32_t)j));
-        const int64_t t = group_item(g / per_chunk, (int)(g % per_chunk), G, (int)(i % G), nt);
-        const float3 a = load_vertex(verts, __ldg(idx + 3 * t));
-        const float3 b = load_vertex(verts, __ldg(idx + 3 * t + 1));
-        const float3 c = load_vertex(verts, __ldg(idx + 3 * t + 2));
-        soup[3 * i + 0] = make_float4(a.x, a.y, a.z, __int_as_float(__ldg(t2o + t)));
-        soup[3 * i + 1] = make_float4(b.x, b.y, b.z, __int_as_float((int)t));
-        soup[3 * i + 2] = make_float4(c.x, c.y, c.z, 0.0f);
-        if (tri_boxes) {
-            float* r = tri_boxes + 6 * (i & ~(int64_t)(unit - 1)) + (i & (unit - 1));
-            r[0] = fminf(a.x, fminf(b.x, c.x));
-            r[unit] = fminf(a.y, fminf(b.y, c.y));
-            r[2 * unit] = fminf(a.z, fminf(b.z, c.z));
-            r[3 * unit] = fmaxf(a.x, fmaxf(b.x, c.x));
-            r[4 * unit] = fmaxf(a.y, fmaxf(b.y, c.y));
-            r[5 * unit] = fmaxf(a.z, fmaxf(b.z, c.z));
+    for (int64_t base = blockIdx.x * (int64_t)blockDim.x; base < n; base += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t i = base + threadIdx.x, j = i / G;
+        const bool in = i < n;
+        float v[6] = {3.4e38f, 3.4e38f, 3.4e38f, -3.4e38f, -3.4e38f, -3.4e38f};
+        if (in) {
+            const uint32_t g = __ldg(list + (order ? __ldg(order + j) : (uint32_t)j));
+            const int64_t t = group_item(g / PER, (int)(g % PER), G, (int)(i % G), nt);
+            const float3 a = load_vertex(verts, __ldg(idx + 3 * t));
+            const float3 b = load_vertex(verts, __ldg(idx + 3 * t + 1));
+            const float3 c = load_vertex(verts, __ldg(idx + 3 * t + 2));
+            soup[3 * i + 0] = make_float4(a.x, a.y, a.z, __int_as_float(__ldg(t2o + t)));
+            soup[3 * i + 1] = make_float4(b.x, b.y, b.z, __int_as_float((int)t));
+            soup[3 * i + 2] = make_float4(c.x, c.y, c.z, 0.0f);
+            v[0] = fminf(a.x, fminf(b.x, c.x));
+            v[1] = fminf(a.y, fminf(b.y, c.y));
+            v[2] = fminf(a.z, fminf(b.z, c.z));
+            v[3] = fmaxf(a.x, fmaxf(b.x, c.x));
+            v[4] = fmaxf(a.y, fmaxf(b.y, c.y));
+            v[5] = fmaxf(a.z, fmaxf(b.z, c.z));
+            if (tri_boxes) {
+                float* r = tri_boxes + 6 * (i & ~(int64_t)(UNIT - 1)) + (i & (UNIT - 1));
+#pragma unroll
+                for (int e = 0; e < 6; ++e) r[e * UNIT] = v[e];
+            }
+        }
+        // the group's box: its lanes' extremes, written by all of them
+        const float empty[6] = {3.4e38f, 3.4e38f, 3.4e38f, -3.4e38f, -3.4e38f, -3.4e38f};
+#pragma unroll
+        for (int e = 0; e < 6; ++e) {
+            v[e] = e < 3 ? fminf(empty[e], v[e]) : fmaxf(empty[e], v[e]);
+#pragma unroll
+            for (int off = 1; off < G; off <<= 1) {
+                const float o = __shfl_xor_sync(0xFFFFFFFFu, v[e], off);
+                v[e] = e < 3 ? fminf(v[e], o) : fmaxf(v[e], o);
+            }
+            if (in && e % G == (int)(i % G)) gbox[6 * j + e] = v[e];
         }
     }
 }
@@ -1648,14 +1682,12 @@ int group_units(pierce_ctx* ctx, const DevDataset& src, const int32_t* t2o, cons
                 const unsigned long long* d_count, int64_t bound, int G, float* gbox, float4* soup, float* tri_boxes) {
     if (bound <= 0) return PIERCE_OK;
     cudaStream_t st = ctx->stream;
-#define PG_PRIMS(g)                                                                                                  \
-    k_group_prims<g, false><<<grid_for(ctx, bound, 256), 256, 0, st>>>(src.verts, src.idx, t2o, src.num_tris, list, \
-                                                                       d_count, nullptr, gbox, nullptr, nullptr)
-    PG_BY_GROUP(PG_PRIMS);
-#undef PG_PRIMS
-    k_group_soup<<<grid_for(ctx, bound * G, 256), 256, 0, st>>>(list, nullptr, d_count, G, src.verts, src.idx, t2o,
-                                                                src.num_tris, soup, tri_boxes);
-    ctx->launches += 2;
+#define PG_SOUP(g)                                                                                               \
+    k_group_soup<g><<<grid_for(ctx, bound * G, 256), 256, 0, st>>>(list, nullptr, d_count, src.verts, src.idx, t2o, \
+                                                                   src.num_tris, soup, gbox, tri_boxes)
+    PG_BY_GROUP(PG_SOUP);
+#undef PG_SOUP
+    ctx->launches += 1;
     return check_cuda(cudaGetLastError(), "group units");
 }
 
@@ -1694,10 +1726,10 @@ int build_group_lbvh(pierce_ctx* ctx, const DevDataset& src, const int32_t* t2o,
 #define PG_PRIMS(g)                                                                                                    \
     if (parts)                                                                                                         \
         k_group_prims<g, true><<<grid_for(ctx, n, B), B, 0, st>>>(src.verts, src.idx, t2o, src.num_tris, list, d_count, \
-                                                                  src.obj_part, gbox, cen, pbounds);                   \
+                                                                  src.obj_part, cen, pbounds);                         \
     else                                                                                                               \
         k_group_prims<g, false><<<grid_for(ctx, n, B), B, 0, st>>>(src.verts, src.idx, t2o, src.num_tris, list,        \
-                                                                   d_count, nullptr, gbox, cen, bounds)
+                                                                   d_count, nullptr, cen, bounds)
     PG_BY_GROUP(PG_PRIMS);
 #undef PG_PRIMS
     if (parts) {
@@ -1709,8 +1741,11 @@ int build_group_lbvh(pierce_ctx* ctx, const DevDataset& src, const int32_t* t2o,
         if (int s = sorted_codes(ctx, cen, n, bounds, 0xFFFFFFFFu, keys, vals)) return s;
     }
     const uint32_t* order = vals + n;
-    k_group_soup<<<grid_for(ctx, n * G, B), B, 0, st>>>(list, order, d_count, G, src.verts, src.idx, t2o, src.num_tris,
-                                                        soup, tri_boxes);
+#define PG_SOUP(g)                                                                                                    \
+    k_group_soup<g><<<grid_for(ctx, n * G, B), B, 0, st>>>(list, order, d_count, src.verts, src.idx, t2o, src.num_tris, \
+                                                           soup, gbox, tri_boxes)
+    PG_BY_GROUP(PG_SOUP);
+#undef PG_SOUP
     ctx->launches += parts ? 3 : 2;
     if (n == 1) {
         if (parts) {
@@ -1720,7 +1755,7 @@ int build_group_lbvh(pierce_ctx* ctx, const DevDataset& src, const int32_t* t2o,
         shape->root_leaf_count = G;
     } else {
         // one group per leaf
-        const LeafBoxes L{gbox, order, nullptr};
+        const LeafBoxes L{gbox, nullptr};
         if (parts) build_nodes(ctx, keys64 + n, n, 1, nodes, part_roots, L, pm, d_root_box);
         else build_nodes(ctx, keys + n, n, 1, nodes, nullptr, L, pm, d_root_box);
         shape->root_is_leaf = 0;
