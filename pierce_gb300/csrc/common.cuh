@@ -144,11 +144,19 @@ constexpr int kPairSetSlot = 40;  // the joins' pair table
 
 // Uniform xy grid over a dataset's object boxes: per cell the objects whose
 // box covers the cell in x and y (parity candidates).
+// An object in a grid cell, with what a ray needs to pass it over.
+struct __align__(16) GridEntry {
+    float4 xy;             // box: lo.x, hi.x, lo.y, hi.y
+    float hi_z;
+    int32_t object;
+    int32_t first, count;  // its triangles
+};
+
 struct ColumnGrid {
     int nx = 0, ny = 0;
     const float* bounds = nullptr;   // lo.x, lo.y, hi.x, hi.y (device)
     const int32_t* offsets = nullptr; // nx*ny + 1
-    const int32_t* entries = nullptr;
+    const GridEntry* entries = nullptr;
 };
 
 constexpr int kSizingScratchSlot = 21;  // 21 and 22: learned sizing (sizing.cu)
@@ -293,7 +301,7 @@ struct pierce_dataset {
     // xy column grid over the object boxes (parity candidates when this
     // dataset is the target), kept the same way
     void* d_grid = nullptr;          // bounds, counts and offsets
-    void* d_grid_entries = nullptr;  // object ids per cell
+    void* d_grid_entries = nullptr;  // objects per cell
     pgpu::ColumnGrid grid{};
     int grid_ready = 0;
 
@@ -413,6 +421,7 @@ int launch_tri_pairs(pierce_ctx* ctx, const DevDataset& a, const PairJoin& j, co
 // n different pair keys (any order) -> pairs sorted by (a, b); object ids
 // below num_a, num_b
 int sort_pairs(pierce_ctx* ctx, const uint64_t* keys, int64_t n, int32_t num_a, int32_t num_b, pierce_pair* out);
+int launch_add_keys(pierce_ctx* ctx, const uint64_t* keys, int64_t n, const PairSet& set);
 int launch_clear_set(pierce_ctx* ctx, const PairSet& set, int64_t n);
 
 // sortscan.cu (CUB library calls)

@@ -20,10 +20,12 @@ namespace pgpu {
 // goes straight to where it is wanted -- the join's pair set, or a list --
 // and no parity table (12 MB per direction at 50,000 objects) is filled,
 // scanned and read back.  Both directions in one launch.  Bound by the chain
-// of dependent loads per source (cell, entries, boxes, chunk boxes, indices,
-// vertices; 17 % of issue slots used): with the candidates found lane by lane
-// and kAhead chunks' loads in flight 2 x 50,000 rays take 0.38 ms instead of
-// 0.60 (10 blocks of 128 per SM, 48 registers; 8 blocks 0.40, 6 0.47, 12 0.37).
+// of dependent loads per source (cell, entries, chunk boxes, indices,
+// vertices; 17 % of issue slots used).  2 x 50,000 rays took 0.60 ms; with the
+// candidates found lane by lane and four chunks' loads in flight 0.38 (10
+// blocks of 128 per SM, 48 registers; 8 blocks 0.40, 6 0.47, 12 0.37), with the
+// objects' boxes and ranges in the grid's entries 0.355, with 64 chunks' boxes
+// and kAhead chunks' triangles in flight 0.335.
 struct ParitySide {
     DevDataset src;      // first vertices, partitions
     ColumnGrid grid;     // the target's column grid
@@ -66,7 +68,7 @@ __device__ __noinline__ bool zray_cross_call(float3 p, float3 a, float3 b, float
     return zray_cross(p, a, b, c, pc);
 }
 
-constexpr int kAhead = 4;
+constexpr int kAhead = 6;
 template <bool TRACK>
 __global__ void __launch_bounds__(128, 10) k_parity_objects(ParityObjParams P) {
     const int lane = threadIdx.x & 31;
@@ -89,28 +91,36 @@ __global__ void __launch_bounds__(128, 10) k_parity_objects(ParityObjParams P) {
         const int32_t e0 = __ldg(S.grid.offsets + cell), e1 = __ldg(S.grid.offsets + cell + 1);
         const int32_t part = T.obj_part ? __ldg(S.src.obj_part + s) : 0;
         for (int32_t base = e0; base < e1; base += 32) {
-            int32_t cand = -1;
+            int4 cand = make_int4(0, -1, 0, 0);  // (hi.z bits), object, first triangle, count
             if (base + lane < e1) {
-                const int32_t t = __ldg(S.grid.entries + base + lane);
-                const float* ob = T.obj_box + 6 * (int64_t)t;
-                if (__ldg(ob) <= p.x && p.x <= __ldg(ob + 3) && __ldg(ob + 1) <= p.y && p.y <= __ldg(ob + 4) &&
-                    __ldg(ob + 5) >= p.z && (!T.obj_part || __ldg(T.obj_part + t) == part))
-                    cand = t;
+                const float4* e = reinterpret_cast<const float4*>(S.grid.entries + base + lane);
+                const float4 xy = __ldg(e);
+                cand = __ldg(reinterpret_cast<const int4*>(e + 1));
+                if (!(xy.x <= p.x && p.x <= xy.y && xy.z <= p.y && p.y <= xy.w && __int_as_float(cand.x) >= p.z &&
+                      (!T.obj_part || __ldg(T.obj_part + cand.y) == part)))
+                    cand.y = -1;
             }
-            for (unsigned left = __ballot_sync(0xFFFFFFFFu, cand >= 0); left; left &= left - 1) {
-                const int32_t t = __shfl_sync(0xFFFFFFFFu, cand, __ffs(left) - 1);
-                const int2 r = __ldg(T.obj_range + t);
+            for (unsigned left = __ballot_sync(0xFFFFFFFFu, cand.y >= 0); left; left &= left - 1) {
+                const int from = __ffs(left) - 1;
+                const int32_t t = __shfl_sync(0xFFFFFFFFu, cand.y, from);
+                const int2 r = make_int2(__shfl_sync(0xFFFFFFFFu, cand.z, from), __shfl_sync(0xFFFFFFFFu, cand.w, from));
                 const int64_t end = (int64_t)r.x + r.y, c_last = (end - 1) / 32;
                 uint32_t crossings = 0;  // this lane's
-                for (int64_t c0 = (int64_t)r.x / 32; c0 <= c_last; c0 += 32) {
-                    const int64_t c = c0 + lane;
-                    bool hit = false;
-                    if (c <= c_last) {
-                        const float* bb = T.tri_chunk_box + 6 * c;
-                        hit = __ldg(bb) <= p.x && p.x <= __ldg(bb + 3) && __ldg(bb + 1) <= p.y &&
-                              p.y <= __ldg(bb + 4) && __ldg(bb + 5) >= p.z;
+                for (int64_t c0 = (int64_t)r.x / 32; c0 <= c_last; c0 += 64) {
+                    // 64 chunks' boxes in flight together
+                    bool hit[2];
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const int64_t c = c0 + 32 * h + lane;
+                        hit[h] = false;
+                        if (c <= c_last) {
+                            const float* bb = T.tri_chunk_box + 6 * c;
+                            hit[h] = __ldg(bb) <= p.x && p.x <= __ldg(bb + 3) && __ldg(bb + 1) <= p.y &&
+                                     p.y <= __ldg(bb + 4) && __ldg(bb + 5) >= p.z;
+                        }
                     }
-                    for (unsigned m = __ballot_sync(0xFFFFFFFFu, hit); m;) {
+                    const unsigned m_hi = __ballot_sync(0xFFFFFFFFu, hit[1]);
+                    for (unsigned long long m = ((unsigned long long)m_hi << 32) | __ballot_sync(0xFFFFFFFFu, hit[0]); m;) {
                         // the triangles of up to kAhead chunks, their loads in
                         // flight together; those whose box the ray meets (one
                         // or two lanes per chunk) are tested after, together
@@ -119,7 +129,7 @@ __global__ void __launch_bounds__(128, 10) k_parity_objects(ParityObjParams P) {
                         unsigned pass = 0;
 #pragma unroll
                         for (int q = 0; q < kAhead; ++q) {
-                            tri[q] = m ? (c0 + __ffs(m) - 1) * 32 + lane : -1;
+                            tri[q] = m ? (c0 + __ffsll((long long)m) - 1) * 32 + lane : -1;
                             m &= m - 1;
                             if (tri[q] < r.x || tri[q] >= end) tri[q] = -1;
                         }

@@ -1671,22 +1671,28 @@ __global__ void k_grid_decode(const uint32_t* ob, float* b) {
     }
 }
 
-// MODE 0: count covered cells per cell; MODE 1: write object ids.
+// MODE 0: count covered cells per cell; MODE 1: write the cells' objects.
 template <int MODE>
-__global__ void k_grid_fill(const float* __restrict__ obj_box, int32_t n, const float* __restrict__ b, int nx, int ny,
-                            int32_t* __restrict__ counts, const int32_t* __restrict__ offsets,
-                            int32_t* __restrict__ cursor, int32_t* __restrict__ entries) {
+__global__ void k_grid_fill(const float* __restrict__ obj_box, const int2* __restrict__ obj_range, int32_t n,
+                            const float* __restrict__ b, int nx, int ny, int32_t* __restrict__ counts,
+                            const int32_t* __restrict__ offsets, int32_t* __restrict__ cursor,
+                            GridEntry* __restrict__ entries) {
     for (int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; o < n; o += (int64_t)gridDim.x * blockDim.x) {
         const float* ob = obj_box + 6 * o;
         if (!(ob[0] <= ob[3])) continue;
         int x0, x1, y0, y1;
         grid_cell_range(b, nx, ny, ob[0], ob[3], 0, x0, x1);
         grid_cell_range(b, nx, ny, ob[1], ob[4], 1, y0, y1);
+        GridEntry e;
+        if (MODE == 1) {
+            const int2 r = obj_range ? __ldg(obj_range + o) : make_int2(0, 0);
+            e = GridEntry{make_float4(ob[0], ob[3], ob[1], ob[4]), ob[5], (int32_t)o, r.x, r.y};
+        }
         for (int y = y0; y <= y1; ++y)
             for (int x = x0; x <= x1; ++x) {
                 const int c = y * nx + x;
                 if (MODE == 0) atomicAdd(counts + c, 1);
-                else entries[offsets[c] + atomicAdd(cursor + c, 1)] = (int32_t)o;
+                else entries[offsets[c] + atomicAdd(cursor + c, 1)] = e;
             }
     }
 }
@@ -1717,7 +1723,7 @@ int column_grid_count(pierce_ctx* ctx, const DevDataset& tgt, void* mem, const i
     if (n > 0) k_grid_bounds<<<grid_cap(ctx, n, 256), 256, 0, st>>>(tgt.obj_box, n, ob);
     k_grid_decode<<<1, 32, 0, st>>>(ob, b);
     if (n > 0)
-        k_grid_fill<0><<<grid_cap(ctx, n, 256), 256, 0, st>>>(tgt.obj_box, n, b, side, side, counts, nullptr, nullptr,
+        k_grid_fill<0><<<grid_cap(ctx, n, 256), 256, 0, st>>>(tgt.obj_box, nullptr, n, b, side, side, counts, nullptr, nullptr,
                                                                nullptr);
     ctx->launches += 5;
     if (int s = exclusive_scan_i32(ctx, counts, offsets, cells + 1)) return s;
@@ -1725,8 +1731,8 @@ int column_grid_count(pierce_ctx* ctx, const DevDataset& tgt, void* mem, const i
     return PIERCE_OK;
 }
 
-// Second phase: the object ids of every cell into `entries` (n_entries).
-int column_grid_fill(pierce_ctx* ctx, const DevDataset& tgt, void* mem, int32_t* entries, ColumnGrid* g) {
+// Second phase: the objects of every cell into `entries` (n_entries).
+int column_grid_fill(pierce_ctx* ctx, const DevDataset& tgt, void* mem, GridEntry* entries, ColumnGrid* g) {
     const int32_t n = tgt.num_objects;
     const int side = std::max(1, (int)std::ceil(std::sqrt((double)std::max(n, 1))));
     const int cells = side * side;
@@ -1736,7 +1742,7 @@ int column_grid_fill(pierce_ctx* ctx, const DevDataset& tgt, void* mem, int32_t*
     int32_t* offsets = counts + cells + 1;
     int32_t* cursor = offsets + cells + 1;
     if (n > 0) {
-        k_grid_fill<1><<<grid_cap(ctx, n, 256), 256, 0, ctx->stream>>>(tgt.obj_box, n, b, side, side, nullptr,
+        k_grid_fill<1><<<grid_cap(ctx, n, 256), 256, 0, ctx->stream>>>(tgt.obj_box, tgt.obj_range, n, b, side, side, nullptr,
                                                                        offsets, cursor, entries);
         ctx->launches += 1;
     }

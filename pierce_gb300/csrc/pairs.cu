@@ -576,6 +576,21 @@ int launch_unit_incidences(pierce_ctx* ctx, const DevDataset& a, const PairJoin&
 
 // ---- pair output ---------------------------------------------------------------
 
+// Keys, repeats among them, into a set.
+__global__ void __launch_bounds__(256) k_add_keys(const uint64_t* __restrict__ keys, int64_t n, PairSet set,
+                                                  uint32_t* err) {
+    uint32_t probes = 0;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+        hash_add(set, keys[i], err, probes);
+}
+
+int launch_add_keys(pierce_ctx* ctx, const uint64_t* keys, int64_t n, const PairSet& set) {
+    k_add_keys<<<(unsigned)std::min<int64_t>((n + 255) / 256, (int64_t)ctx->sm_count * 16), 256, 0, ctx->stream>>>(
+        keys, n, set, ctx->d_err);
+    ctx->launches += 1;
+    return check_cuda(cudaGetLastError(), "add keys");
+}
+
 // The listed slots of a set back to empty.
 __global__ void __launch_bounds__(256) k_clear_set(PairSet set, int64_t n) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
