@@ -150,17 +150,33 @@ def edge_ray_bytes(src, tgt, raw_hits):
     return 28 * E + 16 * F + 12 * V + 32 * (2 * F - 1) + 8 * raw_hits
 
 
-# DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) per traced
-# segment of the two edge-ray launches of one join, from one full-size ncu
-# capture of this build (one pass per launch): the tube join's 3.896 GB over
-# 67,917,789 segments, the ellipsoid intersection join's 250.3 MB over
-# 4,148,442 segments.
+# DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) per segment of a
+# join's ray stage, from ncu captures (one pass per launch).  Rays
+# (k_edge_rays, both launches): the tube join's 3.896 GB over 67,917,789
+# segments, the ellipsoid intersection join's 250.3 MB over 4,148,442.
+# Triangle pairs (k_tri_pairs, which stand for those segments): PAIRBYTES
 EDGE_RAY_DRAM_BYTES_PER_RAY = {"tubes": 57.37, "ellipsoids": 60.34}
+TRI_PAIR_DRAM_BYTES_PER_RAY = {"tubes": None, "ellipsoids": None}
 
 
-def traffic_estimate(rays, workload="tubes"):
-    per = EDGE_RAY_DRAM_BYTES_PER_RAY.get(workload)
+def triangle_pairs_ran(stats):
+    """Joins by triangle pairs report their one walk in the first direction."""
+    return stats["ms_edge_rays"][0] > 0 and stats["ms_edge_rays"][1] == 0
+
+
+def traffic_estimate(rays, workload="tubes", table=EDGE_RAY_DRAM_BYTES_PER_RAY):
+    per = table.get(workload)
     return None if per is None else per * rays
+
+
+def ray_traffic(stats, workload):
+    return traffic_estimate(stats["rays"], workload,
+                            TRI_PAIR_DRAM_BYTES_PER_RAY if triangle_pairs_ran(stats) else EDGE_RAY_DRAM_BYTES_PER_RAY)
+
+
+def ray_kernel(stats):
+    return ("k_tri_pairs: the triangle pairs that stand for both directions' edge rays" if triangle_pairs_ran(stats)
+            else "k_edge_rays, both directions")
 
 
 def traced_edge_ray_bytes(rays, raw_hits, targets):
@@ -837,8 +853,8 @@ def main_tubes(args):
                                               "fp64_ambiguous", "predicted_pairs", "sizing_overflow", "hash_slots",
                                               "active_triangles", "launches")},
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
-                     "frac": achieved / peak if peak else None, "traffic": traffic_estimate(st["rays"], "tubes"),
-                     "kernel": "k_edge_rays, both directions of the tube join", "peak_kind": peak_kind,
+                     "frac": achieved / peak if peak else None, "traffic": ray_traffic(st, "tubes"),
+                     "kernel": ray_kernel(st) + " of the tube join", "peak_kind": peak_kind,
                      "algorithmic_bytes": traced_bytes, "kernel_ms": edge_ms},
         "plain": {"value": 1000.0 / plain_ms, "unit": UNIT, "ms_per_step": plain_ms,
                   "form": "dataset BVH builds + fp32 Moller-Trumbore two-pass join, no culling",
@@ -1188,8 +1204,8 @@ def main_ellipsoids(args):
         "active_triangles": list(ri.stats["active_triangles"]),
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak if peak else None,
-                     "traffic": traffic_estimate(ri.stats["rays"], "ellipsoids"),
-                     "kernel": "k_edge_rays (exact, hash mode), both directions of the intersection join",
+                     "traffic": ray_traffic(ri.stats, "ellipsoids"),
+                     "kernel": ray_kernel(ri.stats) + " of the intersection join",
                      "peak_kind": peak_kind, "algorithmic_bytes": traced_bytes,
                      "unculled_equivalent_gbs": unculled_bytes / (edge_ms / 1000.0) / 1e9 if edge_ms > 0 else None},
         "plain": plain, "cpu_baseline": cpu, "reference_semantics_diff": ref_sem, "e2e": e2e,
