@@ -48,8 +48,7 @@ struct __align__(16) Node {
     float4 bx;   // c0.lo.x, c0.hi.x, c1.lo.x, c1.hi.x
     float4 by;   // c0.lo.y, c0.hi.y, c1.lo.y, c1.hi.y
     float4 bz;   // c0.lo.z, c0.hi.z, c1.lo.z, c1.hi.z
-    int4 ch;     // child0, child1, leaf counts (count0 | count1 << 8),
-                 // build link (parent << 2 | side << 1 | arrival toggle)
+    int4 ch;     // child0, child1, leaf counts (count0 | count1 << 8), 0
 };
 
 // Four-wide node collapsed from a binary hierarchy: Node4[n] holds the

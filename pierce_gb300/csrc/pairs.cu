@@ -107,6 +107,8 @@ __global__ void __launch_bounds__(32 * kPairWarps, DEFER ? 6 : 4) k_tri_pairs(Pa
     // units per fetch: few when there are few, so that all warps share them
     const int64_t warps = (int64_t)gridDim.x * kPairWarps;
     const int per = (int)min((int64_t)kPairUnits, max((int64_t)1, n / (warps * kPairShare)));
+    const int64_t dealt = warps * per;
+    int64_t first_share = ((int64_t)blockIdx.x * kPairWarps + (threadIdx.x >> 5)) * per;
     const int G = BIG ? P.G : U;
     const int side = BIG ? G / U : 1;  // blocks per side of a leaf pair
     PredCounters pc{0, 0};
@@ -250,7 +252,7 @@ __global__ void __launch_bounds__(32 * kPairWarps, DEFER ? 6 : 4) k_tri_pairs(Pa
                 unsigned long long at = 0;
                 if (lane == 0) at = __ldcg(P.cursor);
                 at = __shfl_sync(0xFFFFFFFFu, at, 0);
-                hand_on = steps >= P.budget || (int64_t)at >= n;
+                hand_on = steps >= P.budget || dealt + (int64_t)at >= n;
                 limit = min(steps + P.look, P.budget);
             }
             if (hand_on) {
@@ -309,9 +311,15 @@ __global__ void __launch_bounds__(32 * kPairWarps, DEFER ? 6 : 4) k_tri_pairs(Pa
             continue;
         }
         if (more) {
-            unsigned long long b = 0;
-            if (lane == 0) b = atomicAdd(P.cursor, (unsigned long long)per);
-            const int64_t base = (int64_t)__shfl_sync(0xFFFFFFFFu, b, 0);
+            // every warp's first share lies at its own place, the rest is
+            // taken in turn (4,864 warps asking one word for their first share
+            // took 3.4 of an empty round's 6.3 us, and as much of a small join)
+            int64_t base = first_share;
+            if (base < 0) {
+                unsigned long long b = 0;
+                if (lane == 0) b = atomicAdd(P.cursor, (unsigned long long)per);
+                base = dealt + (int64_t)__shfl_sync(0xFFFFFFFFu, b, 0);
+            }
             const bool item = lane < per && base + lane < n;
             bool node = item, leaf = false;
             uint32_t entry = (uint32_t)lane;  // node 0
@@ -339,7 +347,8 @@ __global__ void __launch_bounds__(32 * kPairWarps, DEFER ? 6 : 4) k_tri_pairs(Pa
             lq = __popc(ml);
             steps = 0;
             limit = P.look;
-            more = base + per < n;
+            more = first_share >= 0 ? dealt < n : base + per < n;
+            first_share = -1;
             __syncwarp();
             continue;
         }
@@ -405,7 +414,10 @@ int launch_tri_pairs(pierce_ctx* ctx, const DevDataset& a, const PairJoin& j, co
     P.amb_cap = j.amb_cap;
     P.a_listed = j.a_listed;
     if (j.b_bound > 0) {
-        const int64_t blocks = std::min<int64_t>((j.b_bound + kPairWarps - 1) / kPairWarps, (int64_t)ctx->sm_count * 8);
+        // the blocks that are resident together (launch bounds): a block that
+        // starts late would hold its first share back
+        const int64_t resident = (int64_t)ctx->sm_count * (j.defer ? 6 : 4);
+        const int64_t blocks = std::min<int64_t>((j.b_bound + kPairWarps - 1) / kPairWarps, resident);
         const unsigned grid = (unsigned)std::max<int64_t>(blocks, 1), threads = 32 * kPairWarps;
         // A group's walk is as long as what it meets (a coarse mesh's group
         // meets thousands of leaves of a fine one): a warp leaves what a
